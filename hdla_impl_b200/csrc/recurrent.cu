@@ -5,16 +5,9 @@
 //     S_t   = exp(g_t) (.) S_{t-1} + sum_r b_r sa_r^T + k_t v_t^T
 //     o_t   = (scale q_t)^T S_t
 //
-// The kernel is bound by HBM traffic: with one token per call the fp32 state [K,V] of every
-// (sequence, head) is read once and written once.  Layout of the work:
-//   * one CTA per (sequence, head); one warp per 32 state columns;
-//   * a lane owns rows k = (lane/8) + 4 s, s = 0..KT-1, of 4 adjacent columns, so every state
-//     access is a 128-bit load/store and 8 lanes cover one full 128-byte line of a row;
-//   * the two K-reductions per token (a^T S and q^T S) are register sums over the lane's rows
-//     followed by two warp shuffles (xor 8, 16) -- no shared-memory reduction, no block barrier
-//     on the reduction path;
-//   * the per-token K-vectors (q, k, exp(g), a_r, b_r) and v are staged once per CTA in shared
-//     memory (double buffered, one barrier per token) and broadcast from there.
+// Two kernels: up to kBulkTokens tokens per call the state tile passes through shared memory by bulk copies
+// (recurrent_bulk_kernel: bound by HBM, the fp32 state is read and written once); longer sequences keep it in
+// registers (recurrent_reg_kernel: bound by fp32 arithmetic or by the dependent steps of the recurrence).
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -35,126 +28,326 @@ struct RecParams {
     int T, H, K, V, dt, gdt, reverse;
 };
 
-template <int KT, int R>
-__global__ void __launch_bounds__(256) recurrent_fwd_kernel(RecParams p) {
-    const int nh = blockIdx.x;
+// ---- packed fp32 pairs (two rows of the state per register pair: one FFMA2 instead of two FFMA)
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 f2_dup(float x) { f2 r; asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x)); return r; }
+__device__ __forceinline__ f2 f2_pack(float x, float y) { f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y)); return r; }
+__device__ __forceinline__ void f2_unpack(f2 a, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a)); }
+__device__ __forceinline__ float f2_sum(f2 a) { float x, y; f2_unpack(a, x, y); return x + y; }
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) { f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sm100::smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// Sum N values over the eight row lanes of a warp (lane bits 2..4), N = 1, 2, 4 or 8: each step halves the values a lane
+// still carries, so N = 8 costs 7 shuffles instead of 24.  Lane r ends with the sums of N/8 (at least one) values,
+// the first of them number scatter_index<N>(r).
+template <int N>
+__device__ __forceinline__ void reduce_scatter(float* v, int lane) {
+    int n = N;
+#pragma unroll
+    for (int m = 4; m <= 16; m <<= 1) {
+        if (n > 1) {
+            const bool up = (lane & m) != 0;
+            n >>= 1;
+#pragma unroll
+            for (int i = 0; i < N / 2; ++i)
+                if (i < n) {
+                    const float give = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+                }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], m);
+        }
+    }
+}
+// ... and with every lane holding all N sums (three dependent steps instead of the six of scatter and gather)
+template <int N>
+__device__ __forceinline__ void all_reduce(float* v) {
+#pragma unroll
+    for (int m = 4; m <= 16; m <<= 1)
+#pragma unroll
+        for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], m);
+}
+template <int N>
+__device__ __forceinline__ int scatter_index(int lane) {
+    int n = N, at = 0;
+#pragma unroll
+    for (int m = 4; m <= 16; m <<= 1)
+        if (n > 1) { n >>= 1; at += (lane & m) ? n : 0; }
+    return at;
+}
+
+// CPT adjacent columns (from c0, a multiple of CPT) of row k of a state tile; V is a multiple of 4, so a group of up to
+// four columns exists as a whole or not at all.  Rows and columns outside the tile read as zero.
+template <int CPT>
+__device__ __forceinline__ void ld_cols(float* x, const float* base, int nh, int k, int c0, int K, int V) {
+#pragma unroll
+    for (int q = 0; q < CPT; ++q) x[q] = 0.f;
+    if (!base || k >= K) return;
+    const float* src = base + ((size_t)nh * K + k) * V + c0;
+    if constexpr (CPT == 2) {
+        if (c0 < V) { const float2 t = __ldcs(reinterpret_cast<const float2*>(src)); x[0] = t.x; x[1] = t.y; }
+    } else {
+#pragma unroll
+        for (int q = 0; q < CPT; q += 4)
+            if (c0 + q < V) {
+                const float4 t = __ldcs(reinterpret_cast<const float4*>(src + q));
+                x[q] = t.x; x[q + 1] = t.y; x[q + 2] = t.z; x[q + 3] = t.w;
+            }
+    }
+}
+template <int CPT>
+__device__ __forceinline__ void st_cols(const float* x, float* base, int nh, int k, int c0, int K, int V) {
+    if (k >= K) return;
+    float* dst = base + ((size_t)nh * K + k) * V + c0;
+    if constexpr (CPT == 2) {
+        if (c0 < V) __stcs(reinterpret_cast<float2*>(dst), make_float2(x[0], x[1]));
+    } else {
+#pragma unroll
+        for (int q = 0; q < CPT; q += 4)
+            if (c0 + q < V) __stcs(reinterpret_cast<float4*>(dst + q), make_float4(x[q], x[q + 1], x[q + 2], x[q + 3]));
+    }
+}
+
+// Register-state kernel: more than kBulkTokens tokens per call.
+//   * A column of the state depends on the other columns through nothing, so the columns are spread over warps (and,
+//     while there are fewer warps than the chip runs, over CTAs): a warp owns 4 CPT columns, lane (r, c) of it the
+//     rows 4 r + 32 j + {0..3} of CPT adjacent columns, in registers, as packed row pairs.
+//   * Tokens are staged kRecBlock at a time: the raw K- and V-vectors of the next block arrive by asynchronous copies
+//     while the current one is worked on; at the block boundary they are turned into fp32 (q scaled, decay
+//     exponentiated) in shared memory once for the whole CTA.  Between two boundaries there is no CTA barrier.
+//   * One pass over the state per token: the update of token t, its output q^T S, and a^T S for token t + 1.  A
+//     128-bit shared load of a vector (four rows) feeds 4 CPT state elements.
+// What bounds it: instruction issue with many sequences (0.55 of the issue slots, 0.31 of the fp32 pipe: 224 packed FMAs
+// of 578 instructions per warp and token at K = 128; shared loads, shuffles and the block conversion are the rest),
+// with few the dependent pass + shuffle sums, 0.66 us per token.  Before, every token's vectors were fetched from
+// global memory between two CTA barriers: 413 tokens in 16 sequences x 16 heads of 128 took 262 us, now 66; one
+// sequence of 128 tokens x 4 heads 540 us, now 85.
+constexpr int kRecBlock = 8;
+// Up to two tokens the bulk-copied tile is the faster form (256 x 32 heads: 176 / 267 us for 1 / 2 tokens against 328 /
+// 284), from three on the registers are (4 tokens: 366 against 456 us; 8 heads, 4 tokens: 7.4 against 15.5).
+constexpr int kBulkTokens = 2;
+
+template <int KR, int CPT, int R>
+__global__ void __launch_bounds__(128, KR * CPT <= 32 ? 4 : KR * CPT <= 64 ? 3 : 2) recurrent_reg_kernel(RecParams p, int col_blocks, int async_ok) {
+    constexpr int KP = 8 * KR, NV = 3 + 2 * R;               // padded rows; K-vectors per token: e k q a.. b..
+    extern __shared__ __align__(16) float sm[];
+    const int nh = blockIdx.x / col_blocks, cb = blockIdx.x % col_blocks;
     const int n = nh / p.H, h = nh % p.H;
     const int K = p.K, V = p.V, H = p.H;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = lane >> 3;
-    const int c4 = (warp * 8 + (lane & 7)) * 4;
-    const bool col_ok = c4 < V;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int r = lane >> 2, c = lane & 3;
+    const int cta_cols = (blockDim.x >> 5) * 4 * CPT;
+    const int cta_c0 = cb * cta_cols;                        // first column of this CTA
+    const int wc = warp * 4 * CPT + c * CPT;                 // this lane's first column within the CTA
+    const int c0 = cta_c0 + wc;
+    const int ncol = min(cta_cols, V - cta_c0);              // columns of this CTA that exist
+    const int tok_floats = NV * KP + cta_cols;
+    unsigned char* raw = reinterpret_cast<unsigned char*>(sm + kRecBlock * tok_floats);
+    const int es = p.dt == HDLA_F32 ? 4 : 2, gs = p.gdt == HDLA_F32 ? 4 : 2;
+    const int tok_raw = ((2 + 2 * R) * K + ncol) * es + K * gs;
 
     long long bos, len;
     if (p.cu) { bos = p.cu[n]; len = p.cu[n + 1] - bos; }
     else      { bos = (long long)n * p.T; len = p.T; }
 
-    extern __shared__ float sm[];
-    const int vec_floats = (3 + 2 * R) * K + V;       // q k eg a[R] b[R] v
-
-    float S[KT][4];
+    const long long stride = p.reverse ? -1 : 1, first = p.reverse ? bos + len - 1 : bos;     // token s is first + s * stride
+    // Request the raw vectors of tokens [s0, s0 + kRecBlock): a thread keeps its 16-byte piece for all tokens of the block.
+    auto request = [&](long long s0) {
+        const int cnt = (int)min((long long)kRecBlock, len - s0);
+        const int nq = K * es / 16, ng = K * gs / 16, nv = ncol * es / 16;
+        const int per = nq * (2 + 2 * R) + ng + nv;
+        for (int w = tid; w < per; w += blockDim.x) {
+            const char* src;
+            size_t step;                                          // bytes between tokens
+            const size_t t0 = (size_t)(first + s0 * stride);
+            if (w < ng) {
+                src = static_cast<const char*>(p.gk) + (t0 * H + h) * K * gs + (size_t)w * 16;
+                step = (size_t)H * K * gs;
+            } else if (w < ng + nv) {
+                src = static_cast<const char*>(p.v) + ((t0 * H + h) * V + cta_c0) * es + (size_t)(w - ng) * 16;
+                step = (size_t)H * V * es;
+            } else {
+                const int vec = (w - ng - nv) / nq, at = (w - ng - nv) % nq;      // 0 k, 1 q, 2.. a, 2 + R.. b
+                const char* base = static_cast<const char*>(vec == 0 ? p.k : vec == 1 ? p.q : vec < 2 + R ? p.a : p.b);
+                const size_t row = vec < 2 ? t0 * H + h : (t0 * R + (vec < 2 + R ? vec - 2 : vec - 2 - R)) * H + h;
+                src = base + row * K * es + (size_t)at * 16;
+                step = (size_t)H * K * es * (vec < 2 ? 1 : R);
+            }
+            unsigned char* dst = raw + (size_t)w * 16;
+            if (p.reverse) step = (size_t)0 - step;
+            for (int tk = 0; tk < cnt; ++tk, src += step, dst += tok_raw) cp_async16(dst, src);
+        }
+        cp_async_commit();
+    };
+    // Turn them into fp32, four elements at a time: a thread keeps its place for all tokens of the block, so the
+    // eight tokens' loads are in flight together.
+    auto convert = [&](long long s0) {
+        const int cnt = (int)min((long long)kRecBlock, len - s0);
+        for (int i = tid; i < NV * (KP / 4) + cta_cols / 4; i += blockDim.x) {
+            const int vec = i / (KP / 4);                         // 0 e, 1 k, 2 q, 3.. a, 3 + R.. b, NV: v
+            const bool is_v = i >= NV * (KP / 4);
+            const int kk = is_v ? (i - NV * (KP / 4)) * 4 : (i % (KP / 4)) * 4;
+            const int lim = is_v ? ncol : K;
+            float4* dst = reinterpret_cast<float4*>(sm + (is_v ? NV * KP : vec * KP) + kk);
+            const int dt = vec == 0 ? p.gdt : p.dt;
+            if (async_ok) {
+                const unsigned char* rw = raw + (is_v ? K * gs : vec == 0 ? 0 : K * gs + ncol * es + (vec - 1) * K * es)
+                                          + kk * (dt == HDLA_F32 ? 4 : 2);
+                float4 x[kRecBlock];
 #pragma unroll
-    for (int s = 0; s < KT; ++s) {
-        const int kk = r + 4 * s;
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (p.h0 && col_ok && kk < K)
-            x = __ldcs(reinterpret_cast<const float4*>(p.h0 + ((size_t)nh * K + kk) * V + c4));
-        S[s][0] = x.x; S[s][1] = x.y; S[s][2] = x.z; S[s][3] = x.w;
-    }
-
-    for (long long step = 0; step < len; ++step) {
-        const long long t = p.reverse ? (bos + len - 1 - step) : (bos + step);
-        float* buf = sm + (step & 1) * vec_floats;
-        float* s_q = buf;
-        float* s_k = buf + K;
-        float* s_e = buf + 2 * K;
-        float* s_a = buf + 3 * K;
-        float* s_b = buf + (3 + R) * K;
-        float* s_v = buf + (3 + 2 * R) * K;
-        const size_t tk = ((size_t)t * H + h) * K;
-        for (int i = threadIdx.x; i < K; i += blockDim.x) {
-            s_q[i] = ld_elem(p.q, tk + i, p.dt) * p.scale;
-            s_k[i] = ld_elem(p.k, tk + i, p.dt);
-            s_e[i] = __expf(ld_elem(p.gk, tk + i, p.gdt));
+                for (int tk = 0; tk < kRecBlock; ++tk) {
+                    x[tk] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (tk < cnt && kk < lim) {
+                        if (dt == HDLA_F32) {
+                            x[tk] = *reinterpret_cast<const float4*>(rw + (size_t)tk * tok_raw);
+                        } else {
+                            const uint2 u = *reinterpret_cast<const uint2*>(rw + (size_t)tk * tok_raw);
+                            x[tk] = make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u),
+                                                __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+                        }
+                        if (vec == 0) { x[tk].x = __expf(x[tk].x); x[tk].y = __expf(x[tk].y); x[tk].z = __expf(x[tk].z); x[tk].w = __expf(x[tk].w); }
+                        if (vec == 2) { x[tk].x *= p.scale; x[tk].y *= p.scale; x[tk].z *= p.scale; x[tk].w *= p.scale; }
+                    }
+                }
 #pragma unroll
-            for (int rr = 0; rr < R; ++rr) {
-                const size_t ta = (((size_t)t * R + rr) * H + h) * K;
-                s_a[rr * K + i] = ld_elem(p.a, ta + i, p.dt);
-                s_b[rr * K + i] = ld_elem(p.b, ta + i, p.dt);
+                for (int tk = 0; tk < kRecBlock; ++tk) dst[tk * (tok_floats / 4)] = x[tk];
+            } else {                                              // rows that asynchronous copies cannot take: element by element
+                const void* base = is_v ? p.v : vec == 0 ? p.gk : vec == 1 ? p.k : vec == 2 ? p.q : vec < 3 + R ? p.a : p.b;
+                for (int tk = 0; tk < cnt; ++tk) {
+                    const size_t t = (size_t)(first + (s0 + tk) * stride);
+                    const size_t at = is_v ? (t * H + h) * V + cta_c0
+                                           : (vec < 3 ? t * H + h : (t * R + (vec < 3 + R ? vec - 3 : vec - 3 - R)) * H + h) * K;
+                    float e[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        e[j] = kk + j < lim ? ld_elem(base, at + kk + j, dt) : 0.f;
+                        if (vec == 0 && kk + j < lim) e[j] = __expf(e[j]);
+                        if (vec == 2) e[j] *= p.scale;
+                    }
+                    dst[tk * (tok_floats / 4)] = make_float4(e[0], e[1], e[2], e[3]);
+                }
             }
         }
-        for (int i = threadIdx.x; i < V; i += blockDim.x)
-            s_v[i] = ld_elem(p.v, ((size_t)t * H + h) * V + i, p.dt);
-        __syncthreads();
+    };
 
-        float sa[R][4];
+    if (async_ok && len > 0) request(0);
+    f2 S[KR / 2][CPT];                                       // S[2 j + u][c]: rows 4 r + 32 j + 2 u + {0, 1}
 #pragma unroll
-        for (int rr = 0; rr < R; ++rr) { sa[rr][0] = sa[rr][1] = sa[rr][2] = sa[rr][3] = 0.f; }
+    for (int j = 0; j < KR / 4; ++j)
 #pragma unroll
-        for (int s = 0; s < KT; ++s) {
-            const int kk = r + 4 * s;
-            if (kk < K) {
+        for (int u = 0; u < 2; ++u) {
+            const int k0 = 32 * j + 4 * r + 2 * u;
+            float x[CPT], y[CPT];
+            ld_cols<CPT>(x, p.h0, nh, k0, c0, K, V);
+            ld_cols<CPT>(y, p.h0, nh, k0 + 1, c0, K, V);
+#pragma unroll
+            for (int q = 0; q < CPT; ++q) S[2 * j + u][q] = f2_pack(x[q], y[q]);
+        }
+
+    for (long long s0 = 0; s0 < len; s0 += kRecBlock) {
+        const int cnt = (int)min((long long)kRecBlock, len - s0);
+        if (async_ok) cp_async_wait_all();
+        __syncthreads();                                     // the raw block is here and the fp32 block has been read
+        convert(s0);
+        __syncthreads();
+        if (async_ok && s0 + kRecBlock < len) request(s0 + kRecBlock);
+        // a^T S for the block's first token
+        float sa[R][CPT];
+        {
+            f2 acc[R][CPT];
+#pragma unroll
+            for (int rr = 0; rr < R; ++rr)
+#pragma unroll
+                for (int q = 0; q < CPT; ++q) acc[rr][q] = 0ull;
+#pragma unroll
+            for (int j = 0; j < KR / 4; ++j)
 #pragma unroll
                 for (int rr = 0; rr < R; ++rr) {
-                    const float av = s_a[rr * K + kk];
+                    const ulonglong2 av = *reinterpret_cast<const ulonglong2*>(sm + (3 + rr) * KP + 32 * j + 4 * r);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) sa[rr][j] = fmaf(av, S[s][j], sa[rr][j]);
+                    for (int q = 0; q < CPT; ++q) {
+                        acc[rr][q] = f2_fma(av.x, S[2 * j][q], acc[rr][q]);
+                        acc[rr][q] = f2_fma(av.y, S[2 * j + 1][q], acc[rr][q]);
+                    }
+                }
+#pragma unroll
+            for (int rr = 0; rr < R; ++rr) {
+#pragma unroll
+                for (int q = 0; q < CPT; ++q) sa[rr][q] = f2_sum(acc[rr][q]);
+                all_reduce<CPT>(sa[rr]);
+            }
+        }
+        for (int tk = 0; tk < cnt; ++tk) {
+            const float* tok = sm + tk * tok_floats;
+            const float* nxt = tk + 1 < cnt ? tok + tok_floats : tok;     // (the last token's a^T S is not used)
+            f2 v2[CPT], s2[R][CPT], oa[CPT], na[R][CPT];
+#pragma unroll
+            for (int q = 0; q < CPT; ++q) {
+                v2[q] = f2_dup(tok[NV * KP + wc + q]);
+#pragma unroll
+                for (int rr = 0; rr < R; ++rr) s2[rr][q] = f2_dup(sa[rr][q]);
+            }
+#pragma unroll
+            for (int j = 0; j < KR / 4; ++j) {
+                const int at = 32 * j + 4 * r;
+                auto vec = [&](const float* base, int i) { return *reinterpret_cast<const ulonglong2*>(base + i * KP + at); };
+                const ulonglong2 e = vec(tok, 0), kv = vec(tok, 1), qv = vec(tok, 2);
+                ulonglong2 bv[R], av[R];
+#pragma unroll
+                for (int rr = 0; rr < R; ++rr) { bv[rr] = vec(tok, 3 + R + rr); av[rr] = vec(nxt, 3 + rr); }
+#pragma unroll
+                for (int q = 0; q < CPT; ++q) {
+                    f2 x = f2_fma(kv.x, v2[q], f2_mul(e.x, S[2 * j][q]));
+                    f2 y = f2_fma(kv.y, v2[q], f2_mul(e.y, S[2 * j + 1][q]));
+#pragma unroll
+                    for (int rr = 0; rr < R; ++rr) { x = f2_fma(bv[rr].x, s2[rr][q], x); y = f2_fma(bv[rr].y, s2[rr][q], y); }
+                    S[2 * j][q] = x; S[2 * j + 1][q] = y;
+                    oa[q] = f2_fma(qv.y, y, j == 0 ? f2_mul(qv.x, x) : f2_fma(qv.x, x, oa[q]));
+#pragma unroll
+                    for (int rr = 0; rr < R; ++rr)
+                        na[rr][q] = f2_fma(av[rr].y, y, j == 0 ? f2_mul(av[rr].x, x) : f2_fma(av[rr].x, x, na[rr][q]));
                 }
             }
-        }
+            if (tk + 1 < cnt) {
 #pragma unroll
-        for (int rr = 0; rr < R; ++rr)
+                for (int rr = 0; rr < R; ++rr) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                sa[rr][j] += __shfl_xor_sync(0xffffffffu, sa[rr][j], 8);
-                sa[rr][j] += __shfl_xor_sync(0xffffffffu, sa[rr][j], 16);
-            }
-        float vv[4] = {0.f, 0.f, 0.f, 0.f};
-        if (col_ok) { vv[0] = s_v[c4]; vv[1] = s_v[c4 + 1]; vv[2] = s_v[c4 + 2]; vv[3] = s_v[c4 + 3]; }
-        float oa[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int s = 0; s < KT; ++s) {
-            const int kk = r + 4 * s;
-            if (kk < K) {
-                const float e = s_e[kk], kv = s_k[kk], qv = s_q[kk];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    float x = fmaf(kv, vv[j], e * S[s][j]);
-#pragma unroll
-                    for (int rr = 0; rr < R; ++rr) x = fmaf(s_b[rr * K + kk], sa[rr][j], x);
-                    S[s][j] = x;
-                    oa[j] = fmaf(qv, x, oa[j]);
+                    for (int q = 0; q < CPT; ++q) sa[rr][q] = f2_sum(na[rr][q]);
+                    all_reduce<CPT>(sa[rr]);
                 }
             }
-        }
+            float o[CPT];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            oa[j] += __shfl_xor_sync(0xffffffffu, oa[j], 8);
-            oa[j] += __shfl_xor_sync(0xffffffffu, oa[j], 16);
-        }
-        if (r == 0 && col_ok) {
-            const size_t to = ((size_t)t * H + h) * V + c4;
-            if (p.dt == HDLA_F32) {
-                *reinterpret_cast<float4*>(static_cast<float*>(p.o) + to) = make_float4(oa[0], oa[1], oa[2], oa[3]);
-            } else {
-                __nv_bfloat162 lo = __floats2bfloat162_rn(oa[0], oa[1]);
-                __nv_bfloat162 hi = __floats2bfloat162_rn(oa[2], oa[3]);
-                uint2 pk;
-                pk.x = *reinterpret_cast<uint32_t*>(&lo);
-                pk.y = *reinterpret_cast<uint32_t*>(&hi);
-                *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.o) + to) = pk;
+            for (int q = 0; q < CPT; ++q) o[q] = f2_sum(oa[q]);
+            reduce_scatter<CPT>(o, lane);
+            // with fewer values than row lanes several lanes hold the same sum: one of them stores it
+            const int col = c0 + scatter_index<CPT>(lane);
+            const bool mine = CPT >= 8 || (CPT == 4 ? (r & 4) == 0 : (r & 6) == 0);
+            if (mine && col < V) {
+                const long long t = first + (s0 + tk) * stride;
+                st_elem(p.o, ((size_t)t * H + h) * V + col, p.dt, o[0]);
             }
         }
     }
 
-    if (p.ht && col_ok) {
+    if (p.ht) {
 #pragma unroll
-        for (int s = 0; s < KT; ++s) {
-            const int kk = r + 4 * s;
-            if (kk < K)
-                __stcs(reinterpret_cast<float4*>(p.ht + ((size_t)nh * K + kk) * V + c4),
-                       make_float4(S[s][0], S[s][1], S[s][2], S[s][3]));
-        }
+        for (int j = 0; j < KR / 4; ++j)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int k0 = 32 * j + 4 * r + 2 * u;
+                float x[CPT], y[CPT];
+#pragma unroll
+                for (int q = 0; q < CPT; ++q) f2_unpack(S[2 * j + u][q], x[q], y[q]);
+                st_cols<CPT>(x, p.ht, nh, k0, c0, K, V);
+                st_cols<CPT>(y, p.ht, nh, k0 + 1, c0, K, V);
+            }
     }
 }
 
@@ -303,16 +496,39 @@ __global__ void __launch_bounds__(256) recurrent_bulk_kernel(RecParams p) {
     }
 }
 
-template <int KT>
-int launch_r(const RecParams& p, int R, int blocks, int threads, size_t smem, cudaStream_t st) {
+template <int KR, int CPT, int R>
+int launch_reg(const RecParams& p, int NH, cudaStream_t st) {
+    // up to four warps (4 CPT columns each) of one head per CTA share its staged vectors
+    const int warps = (p.V + 4 * CPT - 1) / (4 * CPT);
+    const int per_cta = warps < 4 ? warps : 4;
+    const int col_blocks = (warps + per_cta - 1) / per_cta;
+    const int cols = per_cta * 4 * CPT;
+    const int es = p.dt == HDLA_F32 ? 4 : 2, gs = p.gdt == HDLA_F32 ? 4 : 2;
+    bool async_ok = p.K * es % 16 == 0 && p.K * gs % 16 == 0 && p.V * es % 16 == 0;
+    for (const void* q : {p.q, p.k, p.v, p.a, p.b, p.gk}) async_ok = async_ok && reinterpret_cast<uintptr_t>(q) % 16 == 0;
+    const size_t smem = (size_t)kRecBlock * (((3 + 2 * R) * 8 * KR + cols) * sizeof(float)
+                                             + (async_ok ? ((2 + 2 * R) * p.K + cols) * es + p.K * gs : 0));
+    static thread_local int attr_dev = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (attr_dev != dev) {
+        cudaError_t e = cudaFuncSetAttribute(recurrent_reg_kernel<KR, CPT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (e != cudaSuccess) return fail(HDLA_ERR_CUDA, "recurrent: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+        attr_dev = dev;
+    }
+    recurrent_reg_kernel<KR, CPT, R><<<NH * col_blocks, per_cta * 32, smem, st>>>(p, col_blocks, async_ok ? 1 : 0);
+    return HDLA_OK;
+}
+
+template <int KR, int CPT>
+int launch_rank(const RecParams& p, int NH, int R, cudaStream_t st) {
     switch (R) {
-        case 1: recurrent_fwd_kernel<KT, 1><<<blocks, threads, smem, st>>>(p); break;
-        case 2: recurrent_fwd_kernel<KT, 2><<<blocks, threads, smem, st>>>(p); break;
-        case 3: recurrent_fwd_kernel<KT, 3><<<blocks, threads, smem, st>>>(p); break;
-        case 4: recurrent_fwd_kernel<KT, 4><<<blocks, threads, smem, st>>>(p); break;
+        case 1: return launch_reg<KR, CPT, 1>(p, NH, st);
+        case 2: return launch_reg<KR, CPT, 2>(p, NH, st);
+        case 3: return launch_reg<KR, CPT, 3>(p, NH, st);
+        case 4: return launch_reg<KR, CPT, 4>(p, NH, st);
         default: return fail(HDLA_ERR_UNSUPPORTED, "recurrent: rank R=%d not in 1..4", R);
     }
-    return HDLA_OK;
 }
 
 }  // namespace
@@ -339,8 +555,7 @@ int recurrent_fwd_launch(const HdlaDims& d, const void* q, const void* k, const 
     const int threads = 32 * ((d.V + 31) / 32);
     // few tokens per call: the bulk-copy staged kernel (state tile must fit in shared memory)
     const size_t tile = (size_t)d.K * d.V * 4;
-    const long long tokens = cu_seqlens ? (long long)d.T : (long long)d.T;
-    if (tokens <= 8 && tile <= 65536 && tile % 16 == 0 && d.R <= 4) {
+    if (d.T <= kBulkTokens && tile <= 65536 && tile % 16 == 0 && d.R <= 4) {
         const size_t smem_b = tile + sizeof(float) * ((3 + 2 * d.R) * (size_t)d.K + d.V);
         static thread_local int attr_dev = -1;
         int dev = 0;
@@ -362,14 +577,20 @@ int recurrent_fwd_launch(const HdlaDims& d, const void* q, const void* k, const 
         HDLA_CHECK_LAUNCH("recurrent_bulk_kernel");
         return HDLA_OK;
     }
-    const size_t smem = 2 * sizeof(float) * ((3 + 2 * d.R) * (size_t)d.K + d.V);
     int rc;
-    if (d.K <= 32)       rc = launch_r<8>(p, d.R, blocks, threads, smem, st);
-    else if (d.K <= 64)  rc = launch_r<16>(p, d.R, blocks, threads, smem, st);
-    else if (d.K <= 128) rc = launch_r<32>(p, d.R, blocks, threads, smem, st);
-    else                 rc = launch_r<64>(p, d.R, blocks, threads, smem, st);
+    const int NH = N * d.H;
+    // Two columns per lane instead of four while that leaves no more than two warps to a scheduler (148 SMs x 4): the pass
+    // over the state is then what a token waits for, and it is half as long.  (With more warps the wider tile wins,
+    // since a shared load feeds twice the arithmetic.)
+    const bool narrow = d.R == 2 && (long long)NH * ((d.V + 15) / 16) <= 148 * 4;
+    if (narrow && d.K <= 64)       rc = launch_reg<8, 2, 2>(p, NH, st);
+    else if (narrow && d.K <= 128) rc = launch_reg<16, 2, 2>(p, NH, st);
+    else if (d.K <= 32)  rc = launch_rank<4, 4>(p, NH, d.R, st);
+    else if (d.K <= 64)  rc = launch_rank<8, 4>(p, NH, d.R, st);
+    else if (d.K <= 128) rc = launch_rank<16, 4>(p, NH, d.R, st);
+    else                 rc = launch_rank<32, 4>(p, NH, d.R, st);
     if (rc != HDLA_OK) return rc;
-    HDLA_CHECK_LAUNCH("recurrent_fwd_kernel");
+    HDLA_CHECK_LAUNCH("recurrent_reg_kernel");
     return HDLA_OK;
 }
 

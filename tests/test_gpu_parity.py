@@ -202,6 +202,31 @@ def test_recurrent_random_shapes_against_oracle(dev, seed):
     check_recurrent_status(dev)
 
 
+@pytest.mark.parametrize("B,T,H,K,V,rank,cu", [
+    (1, 3, 2, 128, 128, 2, None), (1, 8, 1, 64, 64, 2, None), (1, 9, 1, 64, 36, 1, None), (40, 17, 2, 128, 128, 2, None),
+    (80, 16, 2, 32, 128, 2, None), (1, 12, 1, 256, 256, 4, None), (1, 11, 2, 33, 20, 3, None), (1, 10, 1, 100, 132, 2, None),
+    (1, 40, 3, 128, 24, 2, [0, 13, 13, 14, 40])])
+@pytest.mark.parametrize("dtype,reverse", [(torch.float32, False), (torch.bfloat16, True)])
+def test_recurrent_register_kernel_edges(dev, B, T, H, K, V, rank, cu, dtype, reverse):
+    """The register-state kernel at the edges of its token blocks (8), row quads and column groups, with both lane tiles
+    (few and many warps), rows that asynchronous copies can and cannot take, ranks 1..4, packed sequences."""
+    import hdla_impl_b200 as Hm
+    reverse = reverse and cu is None
+    x = make_inputs(B, T, H, K, V, rank, seed=T + K, dtype=dtype, gk_div=2.0)
+    n = B if cu is None else len(cu) - 1
+    h0 = torch.randn(n, H, K, V, generator=torch.Generator().manual_seed(7)) * 0.3
+    args = [x[m].to(dev) for m in ("q", "k", "v", "a", "b", "gk")]
+    o, ht = Hm.fused_recurrent_dplr_delta_rule(*args, rank, None, h0.to(dev), True, reverse,
+                                               None if cu is None else torch.tensor(cu, device=dev))
+    f = lambda m: x[m].double()
+    ro, rh = orc.recurrent_ref(f("q"), f("k"), f("v"), f("a"), f("b"), f("gk"), rank, None, h0,
+                               **(dict(reverse=reverse) if cu is None else dict(cu_seqlens=cu)))
+    # fp32 throughout: T dependent steps of K-term sums, sqrt(K T) 2^-24 ~ 4e-6 of the largest value; a bf16 output is
+    # rounded once, 2^-9 of it
+    assert orc.rel_err(ht, rh) < 2e-5
+    assert orc.rel_err(o, ro) < (2e-5 if dtype == torch.float32 else 4e-3)
+
+
 def test_recurrent_inplace_state(dev):
     import hdla_impl_b200 as H
     x = make_inputs(4, 1, 2, 64, 64, R, seed=10, h0_std=0.5)
