@@ -2,10 +2,13 @@
 
 There is no fallback: if the library is missing it is built with nvcc once; if that is not
 possible, or a call fails, a ``RuntimeError`` carrying ``hdla_last_error()`` is raised.
+
+``native()`` is the compiled host path of the entry points (csrc/binding.cpp), bound to the same library.
 """
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 import threading
 from typing import Optional
@@ -113,6 +116,33 @@ def load() -> C.CDLL:
                                            vp, C.c_int32, C.c_int32, vp]
         _lib = lib
         return lib
+
+
+_native = None
+
+
+def _on_overflow() -> None:
+    from . import hrdplr
+    hrdplr.warn_fallback()
+
+
+def native():
+    """The compiled host path (module ``_binding``): one call from Python per operator call."""
+    global _native
+    if _native is None:
+        lib = load()
+        with _lock:
+            if _native is None:
+                from . import build as _build
+                path = _build.BINDING
+                if not os.path.exists(path):
+                    _build.build_binding()
+                spec = importlib.util.spec_from_file_location("hdla_impl_b200._binding", path)
+                mod = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(mod)
+                mod.bind(lib._handle, _on_overflow)
+                _native = mod
+    return _native
 
 
 def kernel_launches() -> int:

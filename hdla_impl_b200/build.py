@@ -1,9 +1,9 @@
-"""Build libhdla.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
+"""Build libhdla.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a, and _binding.so (the host path between
+PyTorch and that library) with g++.
 
     python -m hdla_impl_b200.build [--force] [--verbose]
 
-The library lands next to this file as ``libhdla.so``; it is rebuilt only when a source or
-header is newer than it.
+Both land next to this file; each is rebuilt only when a source or header of it is newer.
 """
 from __future__ import annotations
 
@@ -12,10 +12,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libhdla.so")
+BINDING = os.path.join(HERE, "_binding.so")
+BINDING_SRC = os.path.join(CSRC, "binding.cpp")
 ROOT = os.path.dirname(HERE)
 
 NVCC_FLAGS = [
@@ -43,7 +46,32 @@ def _stale() -> bool:
     return any(os.path.getmtime(f) > t for f in deps)
 
 
+def _binding_stale() -> bool:
+    deps = [BINDING_SRC, os.path.join(ROOT, "include", "hdla.h")]
+    return not os.path.exists(BINDING) or any(os.path.getmtime(f) > os.path.getmtime(BINDING) for f in deps)
+
+
+def build_binding(force: bool = False) -> str:
+    """Compile csrc/binding.cpp against the installed PyTorch (its headers and libraries)."""
+    if not force and not _binding_stale():
+        return BINDING
+    import torch
+    top = os.path.dirname(os.path.abspath(torch.__file__))
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    inc = [os.path.join(top, "include"), os.path.join(top, "include", "torch", "csrc", "api", "include"),
+           os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{d}" for d in inc], BINDING_SRC,
+           "-o", BINDING, "-L" + os.path.join(top, "lib"), "-L" + os.path.join(cuda, "lib64"), "-ltorch", "-ltorch_cpu",
+           "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda", "-lcudart"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on {BINDING_SRC}:\n{r.stdout}")
+    return BINDING
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    build_binding(force)
     if not force and not _stale():
         return LIB
     objdir = os.path.join(HERE, "build")

@@ -99,105 +99,53 @@ def workspace_bytes(dims: _lib.HdlaDims, with_backward: bool) -> int:
 
 
 # ---- device status words ----------------------------------------------------------------------
-# The bf16 tensor-core kernels report in the first bytes of the workspace (see include/hdla.h):
-# word 0 a device-side wait that ran out, word 1 a chunk whose total log decay is beyond what the
-# pipeline represents, word 2 the largest chunk decay of the call.  After every launch the words are
-# copied to pinned host memory without blocking and inspected the next time this module is entered on
-# that device, so a problem never stays silent and the hot path never waits.
-#
-# A decay overflow is different from the other conditions: the call's results are wrong but the fp32
-# pipeline would have computed them correctly (the reference layer feeds undivided logsigmoid decays,
-# HRDPLR/hdla_custom.py:219, which can exceed the limit for fast-forgetting channels).  Forward
-# therefore WAITS for its own status words -- and reruns the call on the fp32 pipeline when word 1 is
-# set -- whenever an overflow is plausible: on the first call on a device, and from then on while the
-# largest chunk decay seen on that device is above half the limit.  Workloads far from the limit (all
-# benchmark configurations: <= 22 of 150) pay for one synchronisation in their first call only.
-# HDLA_STRICT=1 always waits; HDLA_ASYNC_STATUS=1 never does (an overflow then raises at the next entry).
-_RING = 64
-_DECAY_LIMIT = 150.0
-_status = {}      # device index -> dict(host=pinned [RING,4] int32, events=[...], next=int, pending=[slots], decay=float|None)
+# The bf16 tensor-core kernels report in the first bytes of the workspace (see include/hdla.h): a device-side wait
+# that ran out, a chunk whose total log decay is beyond what the pipeline represents, the largest chunk decay of the
+# call.  The protocol -- a copy to pinned memory after every call, looked at when the device is used next, and a
+# forward that waits and is rerun on the fp32 pipeline while an overflow is plausible -- is in csrc/binding.cpp.
 _warned_fallback = False
 
 
-def _status_state(dev):
-    st = _status.get(dev.index)
-    if st is None:
-        st = dict(host=torch.zeros(_RING, 4, dtype=torch.int32).pin_memory(),
-                  events=[torch.cuda.Event() for _ in range(_RING)], next=0, pending=[], decay=None)
-        _status[dev.index] = st
-    return st
+def warn_fallback() -> None:
+    """Called when a forward call is rerun on the fp32 pipeline: warns the first time."""
+    global _warned_fallback
+    if not _warned_fallback:
+        _warned_fallback = True
+        warnings.warn("hdla_impl_b200: a chunk's total log decay exceeds what the bf16 tensor-core pipeline represents; "
+                      "such calls are rerun on the fp32 CUDA-core pipeline (correct, much slower)", RuntimeWarning,
+                      stacklevel=3)
 
 
-def _note_decay(st, words) -> None:
-    seen = float(torch.tensor(int(words[2]), dtype=torch.int32).view(torch.float32))
-    if seen == seen:
-        st["decay"] = seen if st["decay"] is None else max(st["decay"], seen)
+class _DecayHistory:
+    """``["decay"]``: the largest chunk decay seen on a device (None: nothing seen yet); can be set."""
+
+    def __init__(self, index: int):
+        self.index = index
+
+    def __getitem__(self, key):
+        if key != "decay":
+            raise KeyError(key)
+        return _lib.native().decay(self.index)
+
+    def __setitem__(self, key, value):
+        if key != "decay":
+            raise KeyError(key)
+        _lib.native().set_decay(self.index, value)
 
 
-def _raise_status(words):
-    if words[0]:
-        raise RuntimeError(f"libhdla: a device-side wait ran out (code {int(words[0])}); the results of that call are invalid")
-    if words[1]:
-        raise RuntimeError(
-            "libhdla: the total log decay of some chunk exceeds 150 in some channel, beyond what the bf16 "
-            "tensor-core pipeline represents; the results of that call are invalid. Set HDLA_FORCE_SIMT=1 to "
-            "use the fp32 pipeline, which has no such limit.")
+def _status_state(dev) -> _DecayHistory:
+    return _DecayHistory(dev.index if isinstance(dev, torch.device) else int(dev))
 
 
 def check_status(dev=None, wait: bool = False) -> None:
     """Raise if an earlier bf16 call on ``dev`` reported a problem. ``wait`` synchronises first."""
-    devs = list(_status) if dev is None else [dev.index if isinstance(dev, torch.device) else int(dev)]
-    for di in devs:
-        st = _status.get(di)
-        if st is None:
-            continue
-        keep = []
-        for slot in st["pending"]:
-            ev = st["events"][slot]
-            if wait:
-                ev.synchronize()
-            if ev.query():
-                words = st["host"][slot].tolist()
-                _note_decay(st, words)
-                if words[0] or words[1]:
-                    st["pending"] = [s_ for s_ in st["pending"] if s_ != slot]
-                    _raise_status(words)
-            else:
-                keep.append(slot)
-        st["pending"] = keep
+    index = -1 if dev is None else (dev.index if isinstance(dev, torch.device) else int(dev))
+    _lib.native().status_check(index, bool(wait))
 
 
 def _post_status(ws: torch.Tensor, dev) -> int:
     """Enqueue the copy of the status words of the call that just used ``ws``; returns the ring slot."""
-    st = _status_state(dev)
-    slot = st["next"]
-    st["next"] = (slot + 1) % _RING
-    if slot in st["pending"]:                       # ring wrapped: that copy finished long ago
-        st["events"][slot].synchronize()
-        check_status(dev)
-    st["host"][slot].copy_(ws[:16].view(torch.int32), non_blocking=True)
-    st["events"][slot].record(torch.cuda.current_stream(dev))
-    st["pending"].append(slot)
-    if os.environ.get("HDLA_STRICT", "0") == "1" and not torch.cuda.is_current_stream_capturing():
-        check_status(dev, wait=True)
-    return slot
-
-
-def _overflow_plausible(dev) -> bool:
-    if os.environ.get("HDLA_ASYNC_STATUS", "0") == "1" or torch.cuda.is_current_stream_capturing():
-        return False
-    st = _status_state(dev)
-    return st["decay"] is None or st["decay"] > 0.5 * _DECAY_LIMIT or os.environ.get("HDLA_STRICT", "0") == "1"
-
-
-def _wait_words(dev, slot):
-    """Wait for the status copy in ``slot`` and take it off the pending list; returns its words."""
-    st = _status_state(dev)
-    st["events"][slot].synchronize()
-    words = st["host"][slot].tolist()
-    st["pending"] = [s_ for s_ in st["pending"] if s_ != slot]
-    _note_decay(st, words)
-    return words
+    return _lib.native().status_post(ws)
 
 
 def _alloc_ws(nbytes: int, device) -> torch.Tensor:
@@ -218,52 +166,30 @@ def chunk_hrdplr_fwd(q, k, v, a, b, gk, scale, initial_state, output_final_state
 
 
 def _chunk_fwd(q, k, v, a, b, gk, scale, initial_state, output_final_state, RANK_AB, head_first, chunk_size,
-               _keep_ws: bool = False, _force_simt: bool = False, cu_seqlens=None):
+               _keep_ws: bool = False, cu_seqlens=None):
     """``chunk_hrdplr_fwd`` returning ``(o, final_state, workspace, used_fp32_pipeline)``; with ``_keep_ws`` the
     workspace is sized for, and keeps what, ``hdla_chunk_bwd(HDLA_FLAG_WS_HOLDS_FWD)`` needs."""
-    global _warned_fallback
     assert head_first is False, "head_first=True is not supported (as in the reference)"
-    dev = _lib.require_cuda(q, k, v, a, b, gk, initial_state)
+    _lib.require_cuda(q, k, v, a, b, gk, initial_state)
     N = None if cu_seqlens is None else len(cu_seqlens) - 1
     _check_shapes(q, k, v, a, b, gk, RANK_AB, initial_state, N)
-    check_status(dev)
-    lib = _lib.load()
-    dims = _dims(q, v, a, gk, RANK_AB, chunk_size, _lib.FLAG_FORCE_SIMT if _force_simt else 0, cu_seqlens)
-    B, T, H, K = q.shape
-    V = v.shape[-1]
-    h0 = None if initial_state is None else initial_state.to(torch.float32).contiguous()
-    with torch.cuda.device(dev):
-        ws = _alloc_ws(workspace_bytes(dims, _keep_ws), dev)
-        o = torch.empty_like(v)
-        ht = torch.empty(B if N is None else N, H, K, V, dtype=torch.float32, device=dev) if output_final_state else None
-        rc = lib.hdla_chunk_fwd(C.byref(dims), _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(a), _lib.ptr(b),
-                                _lib.ptr(gk), float(scale), _lib.ptr(h0), _lib.ptr(o), _lib.ptr(ht),
-                                _lib.ptr(ws), ws.numel(), _lib.stream_ptr(dev))
-        _lib.check(rc, "hdla_chunk_fwd")
-        if lib.hdla_chunk_uses_tensor_cores(C.byref(dims)):
-            slot = _post_status(ws, dev)
-            if _overflow_plausible(dev):
-                words = _wait_words(dev, slot)
-                if words[1] and not words[0]:
-                    if not _warned_fallback:
-                        _warned_fallback = True
-                        warnings.warn("hdla_impl_b200: a chunk's total log decay exceeds what the bf16 tensor-core "
-                                      "pipeline represents; such calls are rerun on the fp32 CUDA-core pipeline "
-                                      "(correct, much slower)", RuntimeWarning, stacklevel=3)
-                    del ws, o, ht
-                    if cu_seqlens is not None:
-                        _raise_status(words)           # the fp32 pipeline takes no packed batches: the caller's
-                                                       # per-sequence path has to be used for such decays
-                    return _chunk_fwd(q, k, v, a, b, gk, scale, initial_state, output_final_state, RANK_AB,
-                                      head_first, chunk_size, _keep_ws=_keep_ws, _force_simt=True)
-                if words[0] or words[1]:
-                    _raise_status(words)
-    return o, ht, (ws if _keep_ws else None), _force_simt
+    rest = (RANK_AB, float(scale), _plain(initial_state), output_final_state, chunk_size, cu_seqlens, bool(_keep_ws))
+    r = _lib.native().chunk(*[_plain(t) for t in (q, k, v, a, b, gk)], *rest)
+    if r is NotImplemented:
+        workspace_bytes(_dims(q, v, a, gk, RANK_AB, chunk_size, 0, cu_seqlens), bool(_keep_ws))      # says why
+        raise TypeError("q, k, v must share one dtype, gk and the states must be floating-point tensors")
+    return r
+
+
+def _plain(t):
+    """The tensor itself, detached and without its subclass."""
+    return t if t is None else t.detach().as_subclass(torch.Tensor)
 
 
 class ChunkDPLRDeltaRuleFunction(torch.autograd.Function):
     """Autograd wrapper (reference: HRDPLR/hrdplr.py:101-284): forward saves the inputs; backward
-    receives ``(do, dht)`` and returns gradients for q,k,v,a,b,gk and the initial state."""
+    receives ``(do, dht)`` and returns gradients for q,k,v,a,b,gk and the initial state.  (``chunk_hrdplr_delta_rule``
+    takes the same steps in native code where its arguments are plain tensors.)"""
 
     @staticmethod
     @contiguous
@@ -289,33 +215,11 @@ class ChunkDPLRDeltaRuleFunction(torch.autograd.Function):
     @autocast_custom_bwd
     def backward(ctx, do, dht):
         q, k, v, a, b, gk, initial_state = ctx.saved_tensors
-        dev = q.device
-        check_status(dev)
-        lib = _lib.load()
-        ws = ctx.ws
-        ctx.ws = None
-        flags = _lib.FLAG_WS_HOLDS_FWD if ws is not None else 0
-        if ctx.force_simt:                          # forward had to fall back to the fp32 pipeline: so does backward
-            flags |= _lib.FLAG_FORCE_SIMT
-        dims = _dims(q, v, a, gk, ctx.RANK_AB, ctx.chunk_size, flags, ctx.cu_seqlens)
-        h0 = None if initial_state is None else initial_state.to(torch.float32).contiguous()
-        if do.dtype != q.dtype:
-            do = do.to(q.dtype)
-        if dht is not None:
-            dht = dht.to(torch.float32).contiguous()
-        with torch.cuda.device(dev):
-            if ws is None:
-                ws = _alloc_ws(workspace_bytes(dims, True), dev)
-            dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-            da, db, dgk = torch.empty_like(a), torch.empty_like(b), torch.empty_like(gk)
-            dh0 = torch.empty_like(h0) if h0 is not None else None
-            rc = lib.hdla_chunk_bwd(C.byref(dims), _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(a), _lib.ptr(b),
-                                    _lib.ptr(gk), float(ctx.scale), _lib.ptr(h0), _lib.ptr(do), _lib.ptr(dht),
-                                    _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(da), _lib.ptr(db),
-                                    _lib.ptr(dgk), _lib.ptr(dh0), _lib.ptr(ws), ws.numel(), _lib.stream_ptr(dev))
-            _lib.check(rc, "hdla_chunk_bwd")
-            if lib.hdla_chunk_uses_tensor_cores(C.byref(dims)):
-                _post_status(ws, dev)                # waits that ran out in the backward kernels surface too
+        ws, ctx.ws = ctx.ws, None
+        grads = _lib.native().chunk_backward(*[_plain(t) for t in (q, k, v, a, b, gk)], ctx.RANK_AB, float(ctx.scale),
+                                             _plain(initial_state), _plain(do), _plain(dht), ws, ctx.chunk_size,
+                                             ctx.cu_seqlens, ctx.force_simt)
+        dq, dk, dv, da, db, dgk, dh0 = grads
         if dh0 is not None and initial_state.dtype != torch.float32:
             dh0 = dh0.to(initial_state.dtype)
         return dq, dk, dv, da, db, dgk, None, dh0, None, None, None, None, None
@@ -349,9 +253,15 @@ def chunk_hrdplr_delta_rule(
     ``fused_recurrent_dplr_delta_rule``; ``initial_state`` / the final state are then ``[n_seqs, H, K, V]``.  bf16
     problems of the tensor-core pipeline run packed (chunks never straddle two sequences; one scan per sequence
     and head); anything else is computed sequence by sequence."""
+    offsets = None if cu_seqlens is None else _seq_offsets(cu_seqlens)
+    if head_first is False:
+        r = (_lib._native or _lib.native()).chunk(q, k, v, a, b, gk, RANK_AB, scale, initial_state, output_final_state,
+                                                  chunk_size, offsets, None)
+        if r is not NotImplemented:
+            return r
+    # what the native path does not take: other problems of a packed batch, tensor subclasses, invalid arguments
     assert q.dtype == k.dtype == v.dtype
     scale = k.shape[-1] ** -0.5 if scale is None else scale
-    offsets = _seq_offsets(cu_seqlens)
     if offsets is not None:
         if q.shape[0] != 1:
             raise ValueError(f"The batch size is expected to be 1 rather than {q.shape[0]} when using `cu_seqlens`."

@@ -51,7 +51,7 @@ def fused_recurrent_dplr_delta_rule_fwd(q, k, v, a, b, gk, rank_ab, scale=1.0, i
                                     _lib.ptr(gk), float(scale), _lib.ptr(h0), _lib.ptr(o), _lib.ptr(ht),
                                     _lib.ptr(cu), N, int(bool(reverse)), _lib.stream_ptr(dev))
         _lib.check(rc, "hdla_recurrent_fwd")
-        _poll_status(lib, dev)
+        _poll_status(_lib.load, dev)
     return o, ht
 
 
@@ -77,19 +77,21 @@ def _poll_state(dev):
     return st
 
 
-def _poll_status(lib, dev) -> None:
-    st = _poll_state(dev)
-    if st["event"] is not None and st["event"].query():
+def _poll_status(load, dev) -> None:
+    st = _poll.get(dev.index) or _poll_state(dev)
+    event = st["event"]
+    if event is not None and not torch.cuda.is_current_stream_capturing() and event.query():
         st["event"] = None
         if int(st["host"][0]):
             raise RuntimeError("libhdla: a device-side wait ran out in the decode kernel; the results of that call "
                                "are invalid and its final state was not written")
     st["calls"] += 1
     if st["calls"] % _POLL_EVERY == 0 and st["event"] is None and not torch.cuda.is_current_stream_capturing():
-        _lib.check(lib.hdla_recurrent_read_status(_lib.ptr(st["host"]), _lib.stream_ptr(dev)),
-                   "hdla_recurrent_read_status")
-        st["event"] = torch.cuda.Event()
-        st["event"].record(torch.cuda.current_stream(dev))
+        with torch.cuda.device(dev):
+            _lib.check(load().hdla_recurrent_read_status(_lib.ptr(st["host"]), _lib.stream_ptr(dev)),
+                       "hdla_recurrent_read_status")
+            st["event"] = torch.cuda.Event()
+            st["event"].record(torch.cuda.current_stream(dev))
 
 
 def check_recurrent_status(dev, wait: bool = True) -> None:
@@ -150,6 +152,12 @@ def fused_recurrent_dplr_delta_rule(
     """Drop-in for the reference's ``fused_recurrent_dplr_delta_rule`` (HRDPLR/recurrent.py:227-319):
     S_t = diag(exp(gk_t)) S_{t-1} + sum_r b_t^(r) (a_t^(r)^T S_{t-1}) + k_t v_t^T, o_t = scale q_t^T S_t."""
     assert head_first == False, ""
+    r = (_lib._native or _lib.native()).recurrent(q, k, v, a, b, gk, rank_ab, scale, initial_state, output_final_state,
+                                                  reverse, cu_seqlens)
+    if r is not NotImplemented:
+        _poll_status(_lib.load, q.device)
+        return r
+    # what the native path does not take: inputs that require gradients, tensor subclasses, invalid arguments
     if cu_seqlens is not None:
         if q.shape[0] != 1:
             raise ValueError(
