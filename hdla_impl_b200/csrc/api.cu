@@ -84,6 +84,7 @@ size_t hdla_chunk_workspace_bytes(const HdlaDims* dims, int with_backward) {
     const size_t simt = simt_workspace_floats(*dims, with_backward) * sizeof(float);
     if (simt == 0) return 0;
     if (tc_supported(*dims)) return tc_region_bytes(*dims, with_backward);
+    if (f32_supported(*dims)) return f32_workspace_floats(*dims, with_backward) * sizeof(float);
     return simt;
 }
 
@@ -110,6 +111,9 @@ int hdla_chunk_fwd(const HdlaDims* dims, const void* q, const void* k, const voi
     if (tc_supported(*dims))
         return tc_chunk_fwd(*dims, q, k, v, a, b, gk, scale, h0, o, ht, static_cast<unsigned char*>(workspace),
                             workspace_bytes, true, static_cast<cudaStream_t>(cuda_stream));
+    if (f32_supported(*dims))
+        return f32_chunk_fwd(*dims, q, k, v, a, b, gk, scale, h0, o, ht, static_cast<float*>(workspace),
+                             workspace_bytes / sizeof(float), true, static_cast<cudaStream_t>(cuda_stream));
     return simt_chunk_fwd(*dims, q, k, v, a, b, gk, scale, h0, o, ht, static_cast<float*>(workspace), true,
                           static_cast<cudaStream_t>(cuda_stream));
 }
@@ -134,6 +138,9 @@ int hdla_chunk_bwd(const HdlaDims* dims, const void* q, const void* k, const voi
     if (tc_supported(*dims))
         return tc_chunk_bwd(*dims, q, k, v, a, b, gk, scale, h0, d_o, dht, dq, dk, dv, da, db, dgk, dh0,
                             static_cast<unsigned char*>(workspace), static_cast<cudaStream_t>(cuda_stream));
+    if (f32_supported(*dims))
+        return f32_chunk_bwd(*dims, q, k, v, a, b, gk, scale, h0, d_o, dht, dq, dk, dv, da, db, dgk, dh0,
+                             static_cast<float*>(workspace), static_cast<cudaStream_t>(cuda_stream));
     return simt_chunk_bwd(*dims, q, k, v, a, b, gk, scale, h0, d_o, dht, dq, dk, dv, da, db, dgk, dh0,
                           static_cast<float*>(workspace), static_cast<cudaStream_t>(cuda_stream));
 }

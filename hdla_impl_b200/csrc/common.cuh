@@ -104,6 +104,16 @@ int simt_chunk_bwd(const HdlaDims& d, const void* q, const void* k, const void* 
                    const void* gk, float scale, const float* h0, const void* d_o, const float* dht, void* dq,
                    void* dk, void* dv, void* da, void* db, void* dgk, float* dh0, float* ws, cudaStream_t st);
 
+// fp32 pipeline for rank 2 and head dims up to 128, chunk_f32.cu
+bool f32_supported(const HdlaDims& d);
+size_t f32_workspace_floats(const HdlaDims& d, int with_backward);
+int f32_chunk_fwd(const HdlaDims& d, const void* q, const void* k, const void* v, const void* a, const void* b,
+                  const void* gk, float scale, const float* h0, void* o, float* ht, float* ws, size_t ws_floats,
+                  bool need_o, cudaStream_t st);
+int f32_chunk_bwd(const HdlaDims& d, const void* q, const void* k, const void* v, const void* a, const void* b,
+                  const void* gk, float scale, const float* h0, const void* d_o, const float* dht, void* dq, void* dk,
+                  void* dv, void* da, void* db, void* dgk, float* dh0, float* ws, cudaStream_t st);
+
 int param_ab_launch(bool backward, const void* beta, const void* k, const void* log_f, void* a, void* b, void* dbeta,
                     void* dk, void* dlog_f, int B, int T, int H, int K, int dt, int gdt, int accumulate, int norm_k,
                     cudaStream_t st);

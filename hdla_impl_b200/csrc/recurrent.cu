@@ -9,6 +9,7 @@
 // (recurrent_bulk_kernel: bound by HBM, the fp32 state is read and written once); longer sequences keep it in
 // registers (recurrent_reg_kernel: bound by fp32 arithmetic or by the dependent steps of the recurrence).
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "sm100.cuh"
 
 namespace hdla {
@@ -27,15 +28,6 @@ struct RecParams {
     float scale;
     int T, H, K, V, dt, gdt, reverse;
 };
-
-// ---- packed fp32 pairs (two rows of the state per register pair: one FFMA2 instead of two FFMA)
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 f2_dup(float x) { f2 r; asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x)); return r; }
-__device__ __forceinline__ f2 f2_pack(float x, float y) { f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y)); return r; }
-__device__ __forceinline__ void f2_unpack(f2 a, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a)); }
-__device__ __forceinline__ float f2_sum(f2 a) { float x, y; f2_unpack(a, x, y); return x + y; }
-__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) { f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sm100::smem_u32(dst)), "l"(src) : "memory");

@@ -839,6 +839,31 @@ def test_rms_norm_fused_gate_forward_backward(dev, dtype, tol, rows, D):
         assert orc.rel_err(got, ref) < tol, n
 
 
+@pytest.mark.parametrize("B,T,H,K,V,gk_div,h0,dtype", [
+    (1, 1, 1, 64, 64, 4.0, True, torch.float32), (2, 15, 1, 65, 64, 4.0, False, torch.float32),
+    (1, 16, 3, 128, 128, 1.0, True, torch.float32), (1, 17, 1, 8, 128, 2.0, True, torch.float32),
+    (1, 50, 2, 100, 20, 4.0, False, torch.float32), (2, 83, 3, 36, 48, 4.0, True, torch.float32),
+    (1, 40, 2, 128, 64, 0.05, True, torch.float32), (1, 33, 2, 64, 128, 4.0, True, torch.bfloat16)])
+def test_fp32_pipeline_edges(dev, B, T, H, K, V, gk_div, h0, dtype, monkeypatch):
+    """The fp32 pipeline of rank-2 problems at the edges of its 16-token tiles and its padded channels (64 / 128), head
+    dims that are not multiples of 4, a decay of exp(-260) per tile, bf16 tensors."""
+    import hdla_impl_b200 as Hm
+    monkeypatch.setenv("HDLA_FORCE_SIMT", "1")
+    x = make_inputs(B, T, H, K, V, R, seed=T + K, dtype=dtype, gk_div=gk_div, h0_std=0.5, with_dht=True)
+    names = ("q", "k", "v", "a", "b", "gk")
+    lv = [x[n].to(dev).requires_grad_(True) for n in names] + ([x["h0"].to(dev).requires_grad_(True)] if h0 else [])
+    o, ht = Hm.chunk_hrdplr_delta_rule(*lv[:6], R, initial_state=lv[6] if h0 else None, output_final_state=True)
+    got = [o, ht, *torch.autograd.grad([o, ht], lv, [x["do"].to(dev), x["dht"].to(dev)])]
+    rl = [x[n].double().requires_grad_(True) for n in names] + ([x["h0"].double().requires_grad_(True)] if h0 else [])
+    ro, rht = orc.recurrent_ref(*rl[:6], R, None, rl[6] if h0 else None)
+    ref = [ro, rht, *torch.autograd.grad((ro * x["do"].double()).sum() + (rht * x["dht"].double()).sum(), rl)]
+    # fp32: sums of up to 128 products over T dependent steps, sqrt(128 T) 2^-24 < 1e-5 of the largest value (an exponential
+    # of a decay of 260 adds its argument's rounding, 260 2^-24 = 1.6e-5); a bf16 result is rounded once, 2^-9
+    tol = 1e-2 if dtype == torch.bfloat16 else 1e-5 if gk_div > 0.1 else 3e-5
+    for n, a_, b_ in zip(("o", "ht", "dq", "dk", "dv", "da", "db", "dgk", "dh0"), got, ref):
+        assert orc.rel_err(a_, b_) < tol, n
+
+
 def test_bf16_requested_chunk_16_runs_on_tensor_cores(dev, monkeypatch):
     """The reference layer passes chunk_size=16; the result is chunk-size independent, so supported bf16
     problems still take the tensor-core pipeline (10 launches for forward+backward, 7 with the one-kernel chunk
