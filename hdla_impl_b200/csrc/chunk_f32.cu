@@ -16,6 +16,11 @@
 //                  M P + w S = v2 these collapse: M^T dw = dP S^T, M^T dM M^T = dP (u + w S)^T = dP v2^T.)
 //   (other stages: HRDPLR/naive.py:107-263, HRDPLR/bwd_triton.py:17-487, 761-947)
 //
+// What bounds them (B2 T1000 H8 K=V=128: 1008 tiles, 128 scan CTAs): the tile kernels issue fp32 arithmetic and shared loads
+// from 8 warps per SM (77 and 266 us), the scans are the serial chain of 63 steps of 2.4 us from one warp per scheduler
+// (155 us each).  Checkpoints are kept transposed, [v][k], so that a scan thread's four state rows move as 16 bytes next
+// to its neighbours' (element by element they took two thirds of the scans' shared/global access slots, 262 us each).
+//
 // Decay-weighted products take the exponent difference per element (exp(g_i - g_j) with g_i <= g_j on the causal mask),
 // so nothing can overflow however strong the decay is.
 #include "common.cuh"
@@ -66,7 +71,7 @@ struct TileP {
     const float *h, *dv2, *dE, *dglp;
     void *dq, *dk, *dv, *da, *db, *dgk;
     float scale;
-    int T, H, K, V, NT, dt, gdt, nslice;
+    int T, H, K, V, NT, dt, gdt, nslice, vec_k, vec_v;
     long long rec_floats;
 };
 
@@ -78,35 +83,86 @@ struct Raw {
     float q[CT][KS], k[CT][KS], a[M2][KS], b[M2][KS], gx[CT + 1][KS];
 };
 
-template <int KP, int NTHR>
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) { *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d); }
+
+// Elements c .. c + N - 1 (N = 2 or 4) of the row of `lim` elements that starts at element `row`; zeros beyond it.  `vec`: rows
+// are a multiple of four elements and aligned, so the group exists as a whole or not at all and moves in one access.
+template <int N>
+__device__ __forceinline__ void ld_row(float (&x)[N], const void* base, size_t row, int c, int lim, int dt, int vec) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) x[j] = 0.f;
+    if (c >= lim) return;
+    if (!vec) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) if (c + j < lim) x[j] = ld_elem(base, row + c + j, dt);
+    } else if (dt == HDLA_F32) {
+        const float* p = static_cast<const float*>(base) + row + c;
+        if constexpr (N == 4) { const float4 t = ld4(p); x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w; }
+        else { const float2 t = *reinterpret_cast<const float2*>(p); x[0] = t.x; x[1] = t.y; }
+    } else {
+        const __nv_bfloat16* p = static_cast<const __nv_bfloat16*>(base) + row + c;
+        uint32_t w[N / 2];
+        if constexpr (N == 4) { const uint2 t = *reinterpret_cast<const uint2*>(p); w[0] = t.x; w[1] = t.y; }
+        else w[0] = *reinterpret_cast<const uint32_t*>(p);
+#pragma unroll
+        for (int j = 0; j < N / 2; ++j) { x[2 * j] = __uint_as_float(w[j] << 16); x[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u); }
+    }
+}
+template <int N>
+__device__ __forceinline__ void st_row(const float (&x)[N], void* base, size_t row, int c, int lim, int dt, int vec) {
+    if (c >= lim) return;
+    if (!vec) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) if (c + j < lim) st_elem(base, row + c + j, dt, x[j]);
+    } else if (dt == HDLA_F32) {
+        float* p = static_cast<float*>(base) + row + c;
+        if constexpr (N == 4) st4(p, x[0], x[1], x[2], x[3]);
+        else *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
+    } else {
+        __nv_bfloat16* p = static_cast<__nv_bfloat16*>(base) + row + c;
+        if constexpr (N == 4) *reinterpret_cast<uint2*>(p) = make_uint2(sm100::pack_bf16(x[0], x[1]), sm100::pack_bf16(x[2], x[3]));
+        else *reinterpret_cast<uint32_t*>(p) = sm100::pack_bf16(x[0], x[1]);
+    }
+}
+
+template <int KP>
 __device__ __forceinline__ void load_raw(const TileP& p, Raw<KP>& s, int b, int h, int t0, int valid) {
-    for (int e = threadIdx.x; e < CT * KP; e += NTHR) {
-        const int i = e / KP, c = e % KP;
-        float q = 0.f, k = 0.f, g = 0.f, a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
-        if (i < valid && c < p.K) {
-            const size_t tok = (size_t)b * p.T + t0 + i;
-            const size_t src = (tok * p.H + h) * p.K + c, sa = (tok * 2 * p.H + h) * p.K + c, sb = sa + (size_t)p.H * p.K;
-            q = ld_elem(p.q, src, p.dt) * p.scale;
-            k = ld_elem(p.k, src, p.dt);
-            g = ld_elem(p.gk, src, p.gdt);
-            a0 = ld_elem(p.a, sa, p.dt); a1 = ld_elem(p.a, sb, p.dt);
-            b0 = ld_elem(p.b, sa, p.dt); b1 = ld_elem(p.b, sb, p.dt);
-        }
-        s.q[i][c] = q; s.k[i][c] = k; s.gx[i + 1][c] = g;
-        s.a[2 * i][c] = a0; s.a[2 * i + 1][c] = a1; s.b[2 * i][c] = b0; s.b[2 * i + 1][c] = b1;
+    constexpr int NI = CT * (KP / 4) / 256;                   // groups of four channels per thread (256 threads)
+    float x[NI][7][4];                                        // every load is issued before the first value is stored
+#pragma unroll
+    for (int it = 0; it < NI; ++it) {
+        const int e = threadIdx.x + it * 256, i = e / (KP / 4), c = (e % (KP / 4)) * 4;
+        const size_t tok = (size_t)b * p.T + t0 + min(i, valid - 1);
+        const size_t src = (tok * p.H + h) * p.K, sa = (tok * 2 * p.H + h) * p.K, sb = sa + (size_t)p.H * p.K;
+        const int lim = i < valid ? p.K : 0;
+        ld_row<4>(x[it][0], p.q, src, c, lim, p.dt, p.vec_k);
+        ld_row<4>(x[it][1], p.k, src, c, lim, p.dt, p.vec_k);
+        ld_row<4>(x[it][2], p.gk, src, c, lim, p.gdt, p.vec_k);
+        ld_row<4>(x[it][3], p.a, sa, c, lim, p.dt, p.vec_k);
+        ld_row<4>(x[it][4], p.a, sb, c, lim, p.dt, p.vec_k);
+        ld_row<4>(x[it][5], p.b, sa, c, lim, p.dt, p.vec_k);
+        ld_row<4>(x[it][6], p.b, sb, c, lim, p.dt, p.vec_k);
+    }
+#pragma unroll
+    for (int it = 0; it < NI; ++it) {
+        const int e = threadIdx.x + it * 256, i = e / (KP / 4), c = (e % (KP / 4)) * 4;
+        auto put = [&](float* dst, const float (&y)[4], float f) { st4(dst + c, f * y[0], f * y[1], f * y[2], f * y[3]); };
+        put(s.q[i], x[it][0], p.scale); put(s.k[i], x[it][1], 1.f); put(s.gx[i + 1], x[it][2], 1.f);
+        put(s.a[2 * i], x[it][3], 1.f); put(s.a[2 * i + 1], x[it][4], 1.f);
+        put(s.b[2 * i], x[it][5], 1.f); put(s.b[2 * i + 1], x[it][6], 1.f);
     }
     __syncthreads();
     if (threadIdx.x < KP) {
-        float run = 0.f;
+        float run = 0.f, g[CT];
+#pragma unroll
+        for (int i = 0; i < CT; ++i) g[i] = s.gx[i + 1][threadIdx.x];
         s.gx[0][threadIdx.x] = 0.f;
 #pragma unroll
-        for (int i = 1; i <= CT; ++i) { run += s.gx[i][threadIdx.x]; s.gx[i][threadIdx.x] = run; }
+        for (int i = 0; i < CT; ++i) { run += g[i]; s.gx[i + 1][threadIdx.x] = run; }
     }
     __syncthreads();
 }
-
-__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) { *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d); }
 
 // ------------------------------------------------------------------------------------------ tile_fwd
 // One thread per token pair (i, j) computes the nine scores between {q_i, a_i0, a_i1} and {k_j, b_j0, b_j1}: they share
@@ -130,13 +186,14 @@ __global__ void __launch_bounds__(256) f32_tile_fwd_kernel(TileP p) {
     const int tid = threadIdx.x;
     float* rec = p.rec + g * p.rec_floats;
     float* uv = p.uv + g * RR * VP;
-    for (int e = tid; e < CT * VP; e += 256) {
-        const int i = e / VP, c = e % VP;
-        const float x = (i < valid && c < p.V) ? ld_elem(p.v, (((size_t)b * p.T + t0 + i) * p.H + h) * p.V + c, p.dt) : 0.f;
-        s.v[i][c] = x;
-        uv[e] = x;
+    for (int e = tid; e < CT * (VP / 4); e += 256) {
+        const int i = e / (VP / 4), c = (e % (VP / 4)) * 4;
+        float x[4];
+        ld_row<4>(x, p.v, (((size_t)b * p.T + t0 + min(i, valid - 1)) * p.H + h) * p.V, c, i < valid ? p.V : 0, p.dt, p.vec_v);
+        st4(&s.v[i][c], x[0], x[1], x[2], x[3]);
+        st4(uv + i * VP + c, x[0], x[1], x[2], x[3]);
     }
-    load_raw<KP, 256>(p, s.x, b, h, t0, valid);
+    load_raw<KP>(p, s.x, b, h, t0, valid);
     {   // scores
         const int i = tid >> 4, j = tid & 15;
         float acc[3][3] = {};
@@ -350,17 +407,13 @@ __global__ void __launch_bounds__(128) f32_scan_kernel(ScanP p) {
         float u[4] = {nu[0], nu[1], nu[2], nu[3]};
         // (an output of this tile overwrites u: the next fetch reads other addresses)
         if (it + 1 < p.NT) fetch(n + dn);
-        float hn[4][VPT];                        // rev: the state after this tile, for the decay gradient
-        {
-            float* ck = REV ? p.dE + ((size_t)g * KP + kg) * p.VP + c0 + vg : p.h + (((size_t)bh * (p.NT + 1) + n) * KP + kg) * p.VP + c0 + vg;
-            const float* hs = p.h + (((size_t)bh * (p.NT + 1) + n + 1) * KP + kg) * p.VP + c0 + vg;
+        float4 hn[VPT];                          // rev: the state after this tile, for the decay gradient
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                for (int c = 0; c < VPT; ++c) {
-                    if (REV) hn[j][c] = hs[(size_t)j * p.VP + c];
-                    if (REV || p.save) ck[(size_t)j * p.VP + c] = S[j][c];
-                }
+        for (int c = 0; c < VPT; ++c) {          // (checkpoints are kept transposed: [v][k])
+            const size_t at = (size_t)(c0 + vg + c) * KP + kg;
+            if (REV) hn[c] = ld4(p.h + ((size_t)bh * (p.NT + 1) + n + 1) * KP * p.VP + at);
+            if (REV) st4(p.dE + (size_t)g * KP * p.VP + at, S[0][c], S[1][c], S[2][c], S[3][c]);
+            else if (p.save) st4(p.h + ((size_t)bh * (p.NT + 1) + n) * KP * p.VP + at, S[0][c], S[1][c], S[2][c], S[3][c]);
         }
         if (!sm100::mbar_wait(&s.bar[it & 1], (it >> 1) & 1) && p.status) atomicExch(p.status, 1);
         // row product over the state's rows: fwd [w; qg] S, rev bg dS
@@ -418,13 +471,13 @@ __global__ void __launch_bounds__(128) f32_scan_kernel(ScanP p) {
             else if (p.save) p.uv[((size_t)g * RR + CT + row) * p.VP + c0 + vcol] = r[i];
         }
         if (REV) {                               // this slice's share of dgl = rowsum(dS (.) S_{n+1})
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                float x = 0.f;
-#pragma unroll
-                for (int c = 0; c < VPT; ++c) x = fmaf(S[j][c], hn[j][c], x);
-                s.red[tid / KG][kg + j] = x;
+            for (int c = 0; c < VPT; ++c) {
+                x.x = fmaf(S[0][c], hn[c].x, x.x); x.y = fmaf(S[1][c], hn[c].y, x.y);
+                x.z = fmaf(S[2][c], hn[c].z, x.z); x.w = fmaf(S[3][c], hn[c].w, x.w);
             }
+            *reinterpret_cast<float4*>(&s.red[tid / KG][kg]) = x;
         }
         __syncthreads();
         if (REV && tid < KP) {
@@ -492,18 +545,18 @@ __global__ void __launch_bounds__(128) f32_scan_kernel(ScanP p) {
         for (int c = 0; c < VPT; ++c) {
             const int k = kg + j, v = c0 + vg + c;
             if (p.fin && k < p.K && v < p.V) p.fin[((size_t)bh * p.K + k) * p.V + v] = S[j][c];
-            if (!REV && p.save) p.h[(((size_t)bh * (p.NT + 1) + p.NT) * KP + k) * p.VP + v] = S[j][c];
+            if (!REV && p.save) p.h[(((size_t)bh * (p.NT + 1) + p.NT) * p.VP + v) * KP + k] = S[j][c];
         }
 }
 
 // ------------------------------------------------------------------------------------------ tile_bwd
-// Warp w owns the tokens 2w and 2w + 1 and lane l the channels l + 32 c, for everything: the state's shares Y S^T and
+// Warp w owns the tokens 2w and 2w + 1 and a lane KP / 32 adjacent channels, for everything: the state's shares Y S^T and
 // Z dS^T, the gated score shares and the un-gating stay in the same thread's registers, up to the decay gradient's
 // running sum over the tokens.
 template <int KP, int VP>
 struct BwdSmem {
     union {
-        struct { float S[KP][VP + 4], dE[KP][VP + 4]; } st;
+        struct { float S[VP][KP + 4], dE[VP][KP + 4]; } st;          // transposed, as the scans keep them
         Raw<KP> x;
     };
     float Y[RR][VP + 4], Z[RR][VP + 4];      // [dO; dv2, then dP], [v; v2];  Y later: decay gradient terms [16][KP + 4]
@@ -511,6 +564,12 @@ struct BwdSmem {
     float M[M2][M2 + 4];
     uint64_t bar;
 };
+
+template <int N>
+__device__ __forceinline__ void ld_sm(float (&x)[N], const float* p) {       // N = 2 or 4 adjacent floats
+    if constexpr (N == 4) { const float4 t = ld4(p); x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w; }
+    else { const float2 t = *reinterpret_cast<const float2*>(p); x[0] = t.x; x[1] = t.y; }
+}
 
 template <int KP, int VP>
 __global__ void __launch_bounds__(256, KP == 128 ? 1 : 2) f32_tile_bwd_kernel(TileP p) {
@@ -526,24 +585,23 @@ __global__ void __launch_bounds__(256, KP == 128 ? 1 : 2) f32_tile_bwd_kernel(Ti
     const float *KB = rec + RR * KP, *A2 = rec + 2 * RR * KP + KP, *rM = A2 + CT * RR, *rAak = rM + M2 * M2;
     if (tid == 0) { sm100::mbar_init(&s.bar, 1); sm100::fence_mbar_init(); }
     __syncthreads();
-    if (tid == 0) sm100::mbar_expect_tx(&s.bar, (2 * KP + RR + M2) * VP * 4);
+    if (tid == 0) sm100::mbar_expect_tx(&s.bar, 2 * VP * KP * 4 + (RR + M2) * VP * 4);
     __syncthreads();
     {   // rows of the padded tiles, one bulk copy each
         const float* S = p.h + ((size_t)bh * (p.NT + 1) + n) * KP * VP;
         const float* dE = p.dE + (size_t)g * KP * VP;
-        for (int r = tid; r < 2 * KP + RR + M2; r += 256) {
-            float* dst;
-            const float* src;
-            if (r < KP) { dst = s.st.S[r]; src = S + (size_t)r * VP; }
-            else if (r < 2 * KP) { dst = s.st.dE[r - KP]; src = dE + (size_t)(r - KP) * VP; }
-            else if (r < 2 * KP + RR) { dst = s.Z[r - 2 * KP]; src = p.uv + ((size_t)g * RR + r - 2 * KP) * VP; }
-            else { dst = s.Y[CT + r - 2 * KP - RR]; src = p.dv2 + ((size_t)g * M2 + r - 2 * KP - RR) * VP; }
-            sm100::bulk_g2s(dst, src, VP * 4, &s.bar);
+        for (int r = tid; r < 2 * VP + RR + M2; r += 256) {
+            if (r < VP) sm100::bulk_g2s(s.st.S[r], S + (size_t)r * KP, KP * 4, &s.bar);
+            else if (r < 2 * VP) sm100::bulk_g2s(s.st.dE[r - VP], dE + (size_t)(r - VP) * KP, KP * 4, &s.bar);
+            else if (r < 2 * VP + RR) sm100::bulk_g2s(s.Z[r - 2 * VP], p.uv + ((size_t)g * RR + r - 2 * VP) * VP, VP * 4, &s.bar);
+            else sm100::bulk_g2s(s.Y[CT + r - 2 * VP - RR], p.dv2 + ((size_t)g * M2 + r - 2 * VP - RR) * VP, VP * 4, &s.bar);
         }
     }
-    for (int e = tid; e < CT * VP; e += 256) {
-        const int i = e / VP, c = e % VP;
-        s.Y[i][c] = (i < valid && c < p.V) ? ld_elem(p.d_o, (((size_t)b * p.T + t0 + i) * p.H + h) * p.V + c, p.dt) : 0.f;
+    for (int e = tid; e < CT * (VP / 4); e += 256) {
+        const int i = e / (VP / 4), c = (e % (VP / 4)) * 4;
+        float x[4];
+        ld_row<4>(x, p.d_o, (((size_t)b * p.T + t0 + min(i, valid - 1)) * p.H + h) * p.V, c, i < valid ? p.V : 0, p.dt, p.vec_v);
+        st4(&s.Y[i][c], x[0], x[1], x[2], x[3]);
     }
     for (int e = tid; e < M2 * M2; e += 256) s.M[e / M2][e % M2] = rM[e];
     sm100::mbar_wait(&s.bar, 0);
@@ -597,89 +655,88 @@ __global__ void __launch_bounds__(256, KP == 128 ? 1 : 2) f32_tile_bwd_kernel(Ti
     }
     // state shares: rows q_i, a_i0, a_i1 of Y S^T and k_i, b_i0, b_i1 of Z dS^T for this warp's tokens
     float dX[2][3][CPT], dW[2][3][CPT];
-    auto state_share = [&](const float (*L)[VP + 4], const float (*R)[VP + 4], float (&out)[2][3][CPT]) {
-        f2 acc[2][3][CPT];
+    const int ch = lane * CPT;                                   // this lane's first channel
+    auto state_share = [&](const float (*L)[VP + 4], const float (*R)[KP + 4], float (&out)[2][3][CPT]) {
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
             for (int r = 0; r < 3; ++r)
 #pragma unroll
-                for (int c = 0; c < CPT; ++c) acc[t][r][c] = 0ull;
+                for (int c = 0; c < CPT; ++c) out[t][r][c] = 0.f;
 #pragma unroll 2
         for (int v = 0; v < VP; v += 4) {
-            ulonglong2 y[CPT];
+            float y[4][CPT];
 #pragma unroll
-            for (int c = 0; c < CPT; ++c) y[c] = *reinterpret_cast<const ulonglong2*>(&R[lane + 32 * c][v]);
+            for (int e = 0; e < 4; ++e) ld_sm<CPT>(y[e], &R[v + e][ch]);
 #pragma unroll
             for (int t = 0; t < 2; ++t)
 #pragma unroll
                 for (int r = 0; r < 3; ++r) {
                     const int i = 2 * warp + t;
-                    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(&L[r == 0 ? i : CT + 2 * i + r - 1][v]);
+                    const float4 x = ld4(&L[r == 0 ? i : CT + 2 * i + r - 1][v]);
 #pragma unroll
-                    for (int c = 0; c < CPT; ++c) acc[t][r][c] = f2_fma(x.y, y[c].y, f2_fma(x.x, y[c].x, acc[t][r][c]));
+                    for (int c = 0; c < CPT; ++c)
+                        out[t][r][c] = fmaf(x.w, y[3][c], fmaf(x.z, y[2][c], fmaf(x.y, y[1][c], fmaf(x.x, y[0][c], out[t][r][c]))));
                 }
+        }
+    };
+    state_share(s.Y, s.st.S, dX);
+    state_share(s.Z, s.st.dE, dW);
+    {   // dv = kg dS + Aqk^T dO + Aak^T dP: this warp's tokens, columns lane + 32 e
+        constexpr int NV = VP / 32;
+        f2 acc[2][NV];
+        float sum[2][NV];
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int e = 0; e < NV; ++e) acc[t][e] = 0ull;
+        const float *k0 = KB + (2 * warp) * KP, *k1 = k0 + KP;
+#pragma unroll 4
+        for (int k = 0; k < KP; k += 4) {
+            const ulonglong2 x0 = __ldg(reinterpret_cast<const ulonglong2*>(k0 + k)), x1 = __ldg(reinterpret_cast<const ulonglong2*>(k1 + k));
+#pragma unroll
+            for (int e = 0; e < NV; ++e) {
+                const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(&s.st.dE[lane + 32 * e][k]);
+                acc[0][e] = f2_fma(x0.y, y.y, f2_fma(x0.x, y.x, acc[0][e]));
+                acc[1][e] = f2_fma(x1.y, y.y, f2_fma(x1.x, y.x, acc[1][e]));
+            }
         }
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
-            for (int r = 0; r < 3; ++r)
+            for (int e = 0; e < NV; ++e) sum[t][e] = f2_sum(acc[t][e]);
+#pragma unroll 8
+        for (int r = 0; r < RR; ++r) {
+            const float2 x = __ldg(reinterpret_cast<const float2*>((r < CT ? A2 + r * RR : rAak + (r - CT) * CT) + 2 * warp));
 #pragma unroll
-                for (int c = 0; c < CPT; ++c) out[t][r][c] = f2_sum(acc[t][r][c]);
-    };
-    state_share(s.Y, s.st.S, dX);
-    state_share(s.Z, s.st.dE, dW);
-    {   // dv = kg dS + Aqk^T dO + Aak^T dP: this warp's tokens, VP / 32 adjacent columns per lane
-        constexpr int NV = VP / 32;
-        float acc[2][NV] = {};
-        const int v = lane * NV;
-        auto row = [&](const float* y, float x0, float x1) {
-#pragma unroll
-            for (int e = 0; e < NV; ++e) { acc[0][e] = fmaf(x0, y[e], acc[0][e]); acc[1][e] = fmaf(x1, y[e], acc[1][e]); }
-        };
-        const float *k0 = KB + (2 * warp) * KP, *k1 = k0 + KP;
-#pragma unroll 2
-        for (int k = 0; k < KP; k += 4) {
-            const float4 x0 = __ldg(reinterpret_cast<const float4*>(k0 + k)), x1 = __ldg(reinterpret_cast<const float4*>(k1 + k));
-            row(&s.st.dE[k][v], x0.x, x1.x); row(&s.st.dE[k + 1][v], x0.y, x1.y);
-            row(&s.st.dE[k + 2][v], x0.z, x1.z); row(&s.st.dE[k + 3][v], x0.w, x1.w);
-        }
-#pragma unroll 4
-        for (int i = 0; i < CT; ++i) {
-            const float2 x = __ldg(reinterpret_cast<const float2*>(A2 + i * RR + 2 * warp));
-            row(&s.Y[i][v], x.x, x.y);
-        }
-#pragma unroll 4
-        for (int r = 0; r < M2; ++r) {
-            const float2 x = __ldg(reinterpret_cast<const float2*>(rAak + r * CT + 2 * warp));
-            row(&s.Y[CT + r][v], x.x, x.y);
+            for (int e = 0; e < NV; ++e) {
+                const float y = s.Y[r][lane + 32 * e];
+                sum[0][e] = fmaf(x.x, y, sum[0][e]); sum[1][e] = fmaf(x.y, y, sum[1][e]);
+            }
         }
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
             for (int e = 0; e < NV; ++e)
-                if (2 * warp + t < valid && v + e < p.V)
-                    st_elem(p.dv, (((size_t)b * p.T + t0 + 2 * warp + t) * p.H + h) * p.V + v + e, p.dt, acc[t][e]);
+                if (2 * warp + t < valid && lane + 32 * e < p.V)
+                    st_elem(p.dv, (((size_t)b * p.T + t0 + 2 * warp + t) * p.H + h) * p.V + lane + 32 * e, p.dt, sum[t][e]);
     }
     __syncthreads();                                             // the states have been read: the raw inputs take their place
-    load_raw<KP, 256>(p, s.x, b, h, t0, valid);
+    load_raw<KP>(p, s.x, b, h, t0, valid);
 #pragma unroll
     for (int t = 0; t < 2; ++t)                                  // un-gate the state shares
 #pragma unroll
         for (int c = 0; c < CPT; ++c) {
-            const int i = 2 * warp + t, ch = lane + 32 * c;
-            const float gi = s.x.gx[i + 1][ch], ei = __expf(gi), ee = __expf(s.x.gx[i][ch]), el = __expf(s.x.gx[CT][ch] - gi);
+            const int i = 2 * warp + t;
+            const float gi = s.x.gx[i + 1][ch + c], ei = __expf(gi), ee = __expf(s.x.gx[i][ch + c]), el = __expf(s.x.gx[CT][ch + c] - gi);
             dX[t][0][c] *= ei; dX[t][1][c] *= ee; dX[t][2][c] *= ee;
             dW[t][0][c] *= el; dW[t][1][c] *= el; dW[t][2][c] *= el;
         }
     // score shares of the rows: tokens j <= i
     for (int j = 0; j <= 2 * warp + 1; ++j) {
         float y[3][CPT], gj[CPT];
-#pragma unroll
-        for (int c = 0; c < CPT; ++c) {
-            const int ch = lane + 32 * c;
-            y[0][c] = s.x.k[j][ch]; y[1][c] = s.x.b[2 * j][ch]; y[2][c] = s.x.b[2 * j + 1][ch]; gj[c] = s.x.gx[j + 1][ch];
-        }
+        ld_sm<CPT>(y[0], &s.x.k[j][ch]); ld_sm<CPT>(y[1], &s.x.b[2 * j][ch]); ld_sm<CPT>(y[2], &s.x.b[2 * j + 1][ch]);
+        ld_sm<CPT>(gj, &s.x.gx[j + 1][ch]);
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
             const int i = 2 * warp + t;
@@ -692,10 +749,11 @@ __global__ void __launch_bounds__(256, KP == 128 ? 1 : 2) f32_tile_bwd_kernel(Ti
                 const float2 x = *reinterpret_cast<const float2*>(&s.dA[row][CT + 2 * j]);
                 co[r][1] = x.x; co[r][2] = x.y;
             }
+            float gi[CPT], ge[CPT];
+            ld_sm<CPT>(gi, &s.x.gx[i + 1][ch]); ld_sm<CPT>(ge, &s.x.gx[i][ch]);
 #pragma unroll
             for (int c = 0; c < CPT; ++c) {
-                const int ch = lane + 32 * c;
-                const float e1 = __expf(s.x.gx[i + 1][ch] - gj[c]), e2 = j < i ? __expf(s.x.gx[i][ch] - gj[c]) : 0.f;
+                const float e1 = __expf(gi[c] - gj[c]), e2 = j < i ? __expf(ge[c] - gj[c]) : 0.f;
 #pragma unroll
                 for (int r = 0; r < 3; ++r)
                     dX[t][r][c] = fmaf(r == 0 ? e1 : e2, fmaf(co[r][0], y[0][c], fmaf(co[r][1], y[1][c], co[r][2] * y[2][c])), dX[t][r][c]);
@@ -705,12 +763,8 @@ __global__ void __launch_bounds__(256, KP == 128 ? 1 : 2) f32_tile_bwd_kernel(Ti
     // score shares of the columns: tokens i >= j
     for (int i = 2 * warp; i < CT; ++i) {
         float x[3][CPT], gi[CPT], ge[CPT];
-#pragma unroll
-        for (int c = 0; c < CPT; ++c) {
-            const int ch = lane + 32 * c;
-            x[0][c] = s.x.q[i][ch]; x[1][c] = s.x.a[2 * i][ch]; x[2][c] = s.x.a[2 * i + 1][ch];
-            gi[c] = s.x.gx[i + 1][ch]; ge[c] = s.x.gx[i][ch];
-        }
+        ld_sm<CPT>(x[0], &s.x.q[i][ch]); ld_sm<CPT>(x[1], &s.x.a[2 * i][ch]); ld_sm<CPT>(x[2], &s.x.a[2 * i + 1][ch]);
+        ld_sm<CPT>(gi, &s.x.gx[i + 1][ch]); ld_sm<CPT>(ge, &s.x.gx[i][ch]);
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
             const int j = 2 * warp + t;
@@ -723,10 +777,11 @@ __global__ void __launch_bounds__(256, KP == 128 ? 1 : 2) f32_tile_bwd_kernel(Ti
                 const float2 y = *reinterpret_cast<const float2*>(&s.dA[row][CT + 2 * j]);
                 co[r][1] = y.x; co[r][2] = y.y;
             }
+            float gj[CPT];
+            ld_sm<CPT>(gj, &s.x.gx[j + 1][ch]);
 #pragma unroll
             for (int c = 0; c < CPT; ++c) {
-                const float gj = s.x.gx[j + 1][lane + 32 * c];
-                const float e1 = __expf(gi[c] - gj), e2 = i > j ? __expf(ge[c] - gj) : 0.f;
+                const float e1 = __expf(gi[c] - gj[c]), e2 = i > j ? __expf(ge[c] - gj[c]) : 0.f;
                 const float xq = x[0][c] * e1, x0 = x[1][c] * e2, x1 = x[2][c] * e2;
 #pragma unroll
                 for (int r = 0; r < 3; ++r) dW[t][r][c] = fmaf(co[0][r], xq, fmaf(co[1][r], x0, fmaf(co[2][r], x1, dW[t][r][c])));
@@ -737,38 +792,43 @@ __global__ void __launch_bounds__(256, KP == 128 ? 1 : 2) f32_tile_bwd_kernel(Ti
     float (*D)[KP + 4] = reinterpret_cast<float (*)[KP + 4]>(&s.Y[0][0]);
     float dge[2][CPT];
 #pragma unroll
-    for (int t = 0; t < 2; ++t)
+    for (int t = 0; t < 2; ++t) {
+        const int i = 2 * warp + t;
+        float q[CPT], k[CPT], a0[CPT], a1[CPT], b0[CPT], b1[CPT];
+        ld_sm<CPT>(q, &s.x.q[i][ch]); ld_sm<CPT>(k, &s.x.k[i][ch]);
+        ld_sm<CPT>(a0, &s.x.a[2 * i][ch]); ld_sm<CPT>(a1, &s.x.a[2 * i + 1][ch]);
+        ld_sm<CPT>(b0, &s.x.b[2 * i][ch]); ld_sm<CPT>(b1, &s.x.b[2 * i + 1][ch]);
 #pragma unroll
         for (int c = 0; c < CPT; ++c) {
-            const int i = 2 * warp + t, ch = lane + 32 * c;
-            dge[t][c] = s.x.a[2 * i][ch] * dX[t][1][c] + s.x.a[2 * i + 1][ch] * dX[t][2][c];
-            D[i][ch] = s.x.q[i][ch] * dX[t][0][c] - s.x.k[i][ch] * dW[t][0][c] - s.x.b[2 * i][ch] * dW[t][1][c]
-                       - s.x.b[2 * i + 1][ch] * dW[t][2][c] + dge[t][c];
-            if (i < valid && ch < p.K) {
-                const size_t tok = (size_t)b * p.T + t0 + i;
-                const size_t at = (tok * p.H + h) * p.K + ch, a0 = (tok * 2 * p.H + h) * p.K + ch, a1 = a0 + (size_t)p.H * p.K;
-                st_elem(p.dq, at, p.dt, dX[t][0][c] * p.scale);
-                st_elem(p.dk, at, p.dt, dW[t][0][c]);
-                st_elem(p.da, a0, p.dt, dX[t][1][c]); st_elem(p.da, a1, p.dt, dX[t][2][c]);
-                st_elem(p.db, a0, p.dt, dW[t][1][c]); st_elem(p.db, a1, p.dt, dW[t][2][c]);
-            }
+            dge[t][c] = a0[c] * dX[t][1][c] + a1[c] * dX[t][2][c];
+            D[i][ch + c] = q[c] * dX[t][0][c] - k[c] * dW[t][0][c] - b0[c] * dW[t][1][c] - b1[c] * dW[t][2][c] + dge[t][c];
+            dX[t][0][c] *= p.scale;
         }
+        if (i < valid) {
+            const size_t tok = (size_t)b * p.T + t0 + i;
+            const size_t at = (tok * p.H + h) * p.K, r0 = (tok * 2 * p.H + h) * p.K, r1 = r0 + (size_t)p.H * p.K;
+            st_row<CPT>(dX[t][0], p.dq, at, ch, p.K, p.dt, p.vec_k);
+            st_row<CPT>(dW[t][0], p.dk, at, ch, p.K, p.dt, p.vec_k);
+            st_row<CPT>(dX[t][1], p.da, r0, ch, p.K, p.dt, p.vec_k); st_row<CPT>(dX[t][2], p.da, r1, ch, p.K, p.dt, p.vec_k);
+            st_row<CPT>(dW[t][1], p.db, r0, ch, p.K, p.dt, p.vec_k); st_row<CPT>(dW[t][2], p.db, r1, ch, p.K, p.dt, p.vec_k);
+        }
+    }
     __syncthreads();
     if (tid < KP) {
-        float run = 0.f;                                         // + the gradient of the chunk-end decay, from all slices
+        float run = 0.f;                                         // the gradient of the chunk-end decay, from all slices ...
         for (int w = 0; w < p.nslice; ++w) run += p.dglp[((size_t)g * p.nslice + w) * KP + tid];
 #pragma unroll
-        for (int i = CT - 1; i >= 0; --i) { run += D[i][tid]; D[i][tid] = run; }
+        for (int i = CT - 1; i >= 0; --i) { run += D[i][tid]; D[i][tid] = run; }      // ... and the running sum
     }
     __syncthreads();
 #pragma unroll
-    for (int t = 0; t < 2; ++t)
+    for (int t = 0; t < 2; ++t) {
+        const int i = 2 * warp + t;
+        float x[CPT];
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) {
-            const int i = 2 * warp + t, ch = lane + 32 * c;
-            if (i < valid && ch < p.K)
-                st_elem(p.dgk, (((size_t)b * p.T + t0 + i) * p.H + h) * p.K + ch, p.gdt, D[i][ch] - dge[t][c]);
-        }
+        for (int c = 0; c < CPT; ++c) x[c] = D[i][ch + c] - dge[t][c];
+        if (i < valid) st_row<CPT>(x, p.dgk, (((size_t)b * p.T + t0 + i) * p.H + h) * p.K, ch, p.K, p.gdt, p.vec_k);
+    }
 }
 
 // ------------------------------------------------------------------------------------------ host side
@@ -803,6 +863,9 @@ TileP tile_params(const HdlaDims& d, const F32Plan& pl, float* ws, const void* q
     p.scale = scale;
     p.T = d.T; p.H = d.H; p.K = d.K; p.V = d.V; p.NT = pl.NT; p.dt = d.dtype; p.gdt = d.gk_dtype; p.nslice = pl.nslice;
     p.rec_floats = pl.rec_floats;
+    p.vec_k = d.K % 4 == 0; p.vec_v = d.V % 4 == 0;
+    for (const void* x : {q, k, v, a, b, gk})
+        if (reinterpret_cast<uintptr_t>(x) % 16 != 0) p.vec_k = p.vec_v = 0;
     return p;
 }
 ScanP scan_params(const HdlaDims& d, const F32Plan& pl, float* ws) {
@@ -863,6 +926,8 @@ int f32_chunk_bwd(const HdlaDims& d, const void* q, const void* k, const void* v
     if (!(d.flags & HDLA_FLAG_WS_HOLDS_FWD))
         TRY(f32_chunk_fwd(d, q, k, v, a, b, gk, scale, h0, nullptr, nullptr, ws, (size_t)pl.total, false, st));
     TileP tp = tile_params(d, pl, ws, q, k, v, a, b, gk, scale);
+    for (const void* x : {d_o, (const void*)dq, (const void*)dk, (const void*)dv, (const void*)da, (const void*)db, (const void*)dgk})
+        if (reinterpret_cast<uintptr_t>(x) % 16 != 0) tp.vec_k = tp.vec_v = 0;
     tp.d_o = d_o; tp.dq = dq; tp.dk = dk; tp.dv = dv; tp.da = da; tp.db = db; tp.dgk = dgk;
     ScanP sp = scan_params(d, pl, ws);
     sp.d_o = d_o; sp.init = dht; sp.fin = dh0;
