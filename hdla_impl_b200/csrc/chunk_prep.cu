@@ -32,12 +32,12 @@ using t8::Tile;
 struct ChunkPrepP {
     const __nv_bfloat16 *q, *k, *v, *a, *b;
     const void* gk;
-    uint4 *Qh, *Kh, *Ah, *Bh, *Vc, *Aqk, *Aqb, *Aak, *M, *W, *P, *U;
+    uint4 *Qh, *Kh, *Ah, *Bh, *Vc, *Aqk, *Aqb, *Aak, *M, *W, *U;
     float* E;
     __nv_bfloat16* ghat;                  // e^{gi - half} per (token, channel), bf16 row-major [64][128]
     float scale;
     int T, H, NT, gdt;
-    int save_bwd;                         // also store Ah, Aak, M, P, ghat (read only by the backward kernels)
+    int save_bwd;                         // also store Ah, Aak, M, ghat (read only by the backward kernels)
     int* status;
     const int2* chunk_tab;                // variable-length batches: (first token, tokens) per chunk, else null
 };
@@ -514,10 +514,6 @@ __global__ void __launch_bounds__(128, 2) chunk_prep_tc_kernel(ChunkPrepP p, lon
         tc_fence_after();
         t8::mma_chain<false, true>(tmem, tD, 0, 0, tP, 0, 0, 128, 128, false);           // u = M P
         umma_commit(&mma_bar);
-        if (p.save_bwd) {
-            bulk_s2g(p.P + g * CH128, sP, 32768);
-            bulk_commit();
-        }
     }
     // Wh while u runs: into the Ah slot (Wh = M Ah is complete, Ah's copy to global memory was waited for before
     // the Aak epilogue), from where one bulk copy takes it to global memory
@@ -569,7 +565,7 @@ int tc_launch_chunk_prep(const TcPlan& pl, const HdlaDims& d, const void* q, con
     typedef const __nv_bfloat16* bp;
     ChunkPrepP pp{(bp)q, (bp)k, (bp)v, (bp)a, (bp)b, gk,
                   U4(pl.Qh), U4(pl.Kh), U4(pl.Ah), U4(pl.Bh), U4(pl.Vc), U4(pl.Aqk), U4(pl.Aqb), U4(pl.Aak), U4(pl.M),
-                  U4(pl.W), U4(pl.P), U4(pl.U), reinterpret_cast<float*>(ws + pl.E),
+                  U4(pl.W), U4(pl.U), reinterpret_cast<float*>(ws + pl.E),
                   reinterpret_cast<__nv_bfloat16*>(ws + pl.ghat), scale, d.T, d.H, pl.NT, d.gk_dtype, save_bwd ? 1 : 0,
                   reinterpret_cast<int*>(ws + pl.status),
                   pl.nseq ? reinterpret_cast<const int2*>(ws + pl.chunk_tab) : nullptr};

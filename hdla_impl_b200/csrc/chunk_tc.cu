@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(128) inverse_tc_kernel(InvP p) {
 // ------------------------------------------------------------------------------------------
 struct WuP {
     const uint4 *M, *Ah, *Aak, *Vc;
-    uint4 *P, *U, *W;
+    uint4 *U, *W;
     int* status;
 };
 
@@ -564,9 +564,7 @@ __global__ void __launch_bounds__(128) wu_tc_kernel(WuP p) {
         tmem_row64(t8::taddr(tmem, warp, hh * 64), f);
 #pragma unroll
         for (int cg = 0; cg < 8; ++cg) {
-            const uint4 c = t8::pack8(f + cg * 8);
-            sP[(hh * 8 + cg) * 128 + tid] = c;
-            p.P[g * CH128 + (hh * 8 + cg) * 128 + tid] = c;
+            sP[(hh * 8 + cg) * 128 + tid] = t8::pack8(f + cg * 8);
         }
     }
     fence_proxy_async();
@@ -868,177 +866,96 @@ __global__ void __launch_bounds__(256) scan_tc_kernel(ScanTcP p) {
 
 // ------------------------------------------------------------------------------------------
 // backward through the WY representation, one kernel per chunk   (HRDPLR/bwd_triton.py:489-612)
-//   dWh = dv2 St^T ; dP = M^T dv2 ; dAak = smask(dP v^T) ; dM = dv2 P^T + dWh Ah^T ;
-//   dAab = smask(M^T dM M^T)
-// Six operand tiles are loaded once (176 KB); dWh, dP, dM and M^T dM are produced as bf16 operand
-// tiles in shared memory (over buffers whose contents are no longer needed) and feed the next
-// product directly, so only dWh, dP, dAak and dAab go back to HBM.
+//   dP = M^T dv2 ; dAak = smask(dP v^T) ; dAab = smask(dP v2^T)
+// The reference goes through dWh = dv2 St^T and dM = dv2 P^T + dWh Ah^T to dAab = smask(M^T dM M^T).  With u = M P,
+// Wh = M Ah and v2 = Wh St + u that is  M^T dv2 (P^T M^T + St^T Ah^T M^T) = dP (u + Wh St)^T = dP v2^T,  and the
+// share of dAh that went through dWh is  M^T dWh = dP St^T  (grad_tc_kernel): neither P, Ah and St are read here nor
+// dWh, dM and M^T dM formed.
+// Bound by memory: 112 KB in, 80 KB out per tile, against 176 + 112 KB of the longer form (which also left room for
+// one CTA per SM only).  dP takes M's place in shared memory, so 112 KB hold a tile and two CTAs per SM cover each
+// other's round trips.
 // ------------------------------------------------------------------------------------------
 struct WyBwdP {
-    const uint4 *M, *DV2, *Hs, *Vc, *P, *Ah;
-    uint4 *dW, *dP, *dAak, *dAab;
+    const uint4 *M, *DV2, *Vc, *V2;
+    uint4 *dP, *dAak, *dAab;
     int* status;
-    long long G;           // number of tiles; the grid is persistent
 };
 
-// Persistent: one CTA per SM walks over the tiles g = blockIdx.x, blockIdx.x + gridDim.x, ...  The 208 KB of operand
-// slots leave no room for a second CTA, so the next tile's operands are requested as soon as the slot they go to has
-// been read for the last time (St, v, Ah after phase 2, dv2 after phase 3, M and P after phase 4): the loads of tile
-// n+1 run under phases 3 and 4 of tile n.
 __global__ void __launch_bounds__(128) wy_bwd_tc_kernel(WyBwdP p) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    uint4* bM = reinterpret_cast<uint4*>(smem);      // M
-    uint4* bDV2 = bM + CH128;                        // dv2, later dM
-    uint4* bHs = bDV2 + CH128;                       // St, later dWh
-    uint4* bP = bHs + CH128;                         // P, later M^T dM
-    uint4* bAh = bP + CH128;                         // Ah
-    uint4* bdP = bAh + CH128;                        // dP
-    uint4* bVc = bdP + CH128;                        // v  [64 x 128]
+    uint4* bM = reinterpret_cast<uint4*>(smem);      // M, later dP
+    uint4* bDV2 = bM + CH128;                        // dv2
+    uint4* bV2 = bDV2 + CH128;                       // v2
+    uint4* bVc = bV2 + CH128;                        // v  [64 x 128]
     __shared__ __align__(8) uint64_t ld1, ld2, mma_bar;
     __shared__ uint32_t tmem_s;
+    const long long g = blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5;
     if (warp == 0) { tmem_alloc(&tmem_s, 256); tmem_relinquish(); }
     if (tid == 0) {
         mbar_init(&ld1, 1); mbar_init(&ld2, 1); mbar_init(&mma_bar, 1); fence_mbar_init();
-        const long long g = blockIdx.x;
-        if (g < p.G) {
-            mbar_expect_tx(&ld1, 98304);
-            bulk_g2s(bDV2, p.DV2 + g * CH128, 32768, &ld1);
-            bulk_g2s(bHs, p.Hs + g * CH128, 32768, &ld1);
-            bulk_g2s(bM, p.M + g * CH128, 32768, &ld1);
-            mbar_expect_tx(&ld2, 81920);
-            bulk_g2s(bVc, p.Vc + g * CH64, 16384, &ld2);
-            bulk_g2s(bP, p.P + g * CH128, 32768, &ld2);
-            bulk_g2s(bAh, p.Ah + g * CH128, 32768, &ld2);
-        }
+        mbar_expect_tx(&ld1, 65536);
+        bulk_g2s(bM, p.M + g * CH128, 32768, &ld1);
+        bulk_g2s(bDV2, p.DV2 + g * CH128, 32768, &ld1);
+        mbar_expect_tx(&ld2, 49152);
+        bulk_g2s(bVc, p.Vc + g * CH64, 16384, &ld2);
+        bulk_g2s(bV2, p.V2 + g * CH128, 32768, &ld2);
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_s;
-    const Tile tM = t8::tile(bM, 128), tDV2 = t8::tile(bDV2, 128), tHs = t8::tile(bHs, 128), tP = t8::tile(bP, 128),
-               tAh = t8::tile(bAh, 128), tdP = t8::tile(bdP, 128), tVc = t8::tile(bVc, 64);
-    const int r = tid;
+    const Tile tM = t8::tile(bM, 128), tDV2 = t8::tile(bDV2, 128), tV2 = t8::tile(bV2, 128), tVc = t8::tile(bVc, 64);
+    const int r = tid, i = r >> 1;
     float f[64];
-    uint32_t it = 0;
-    for (long long g = blockIdx.x; g < p.G; g += gridDim.x, ++it) {
-        const uint32_t ph = it & 1;
-        const long long gn = g + gridDim.x;              // next tile of this CTA
-        const bool more = gn < p.G;
-        // ---- phase 1: dWh = dv2 St^T (cols 0..127), dP = M^T dv2 (cols 128..255)
-        wait_or_flag(&ld1, ph, p.status, 30);
-        if (tid == 0) {
-            tc_fence_after();
-            t8::mma_chain<false, false>(tmem, tDV2, 0, 0, tHs, 0, 0, 128, 128, false);
-            t8::mma_chain<true, true>(tmem + 128, tM, 0, 0, tDV2, 0, 0, 128, 128, false);
-            umma_commit(&mma_bar);
-        }
-        wait_or_flag(&mma_bar, 0, p.status, 31);
-        tc_fence_after();
-#pragma unroll 1
-        for (int hh = 0; hh < 2; ++hh) {
-            tmem_row64(t8::taddr(tmem, warp, hh * 64), f);
-#pragma unroll
-            for (int c8 = 0; c8 < 8; ++c8) {
-                const uint4 c = t8::pack8(f + c8 * 8);
-                bHs[(hh * 8 + c8) * 128 + r] = c;                       // dWh replaces St
-                p.dW[g * CH128 + (hh * 8 + c8) * 128 + r] = c;
-            }
-            tmem_row64(t8::taddr(tmem, warp, 128 + hh * 64), f);
-#pragma unroll
-            for (int c8 = 0; c8 < 8; ++c8) {
-                const uint4 c = t8::pack8(f + c8 * 8);
-                bdP[(hh * 8 + c8) * 128 + r] = c;
-                p.dP[g * CH128 + (hh * 8 + c8) * 128 + r] = c;
-            }
-        }
-        fence_proxy_async();
-        tc_fence_before();
-        __syncthreads();
-        // ---- phase 2: dAak = dP v^T (cols 0..63), dM = dv2 P^T + dWh Ah^T (cols 128..255)
-        wait_or_flag(&ld2, ph, p.status, 32);
-        if (tid == 0) {
-            tc_fence_after();
-            t8::mma_chain<false, false>(tmem, tdP, 0, 0, tVc, 0, 0, 64, 128, false);
-            t8::mma_chain<false, false>(tmem + 128, tDV2, 0, 0, tP, 0, 0, 128, 128, false);
-            t8::mma_chain<false, false>(tmem + 128, tHs, 0, 0, tAh, 0, 0, 128, 128, true);
-            umma_commit(&mma_bar);
-        }
-        wait_or_flag(&mma_bar, 1, p.status, 33);
-        tc_fence_after();
-        if (tid == 0 && more) {                          // St, v, Ah slots have been read for the last time
-            mbar_expect_tx(&ld1, 98304);
-            bulk_g2s(bHs, p.Hs + gn * CH128, 32768, &ld1);
-            mbar_expect_tx(&ld2, 81920);
-            bulk_g2s(bVc, p.Vc + gn * CH64, 16384, &ld2);
-            bulk_g2s(bAh, p.Ah + gn * CH128, 32768, &ld2);
-        }
-        {
-            const int i = r >> 1;
-            tmem_row64(t8::taddr(tmem, warp, 0), f);
-#pragma unroll
-            for (int c8 = 0; c8 < 8; ++c8) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) if (!((c8 * 8 + j) < i)) f[c8 * 8 + j] = 0.f;
-                p.dAak[g * CH64 + c8 * 128 + r] = t8::pack8(f + c8 * 8);
-            }
-#pragma unroll 1
-            for (int hh = 0; hh < 2; ++hh) {
-                tmem_row64(t8::taddr(tmem, warp, 128 + hh * 64), f);
-#pragma unroll
-                for (int c8 = 0; c8 < 8; ++c8) bDV2[(hh * 8 + c8) * 128 + r] = t8::pack8(f + c8 * 8);   // dM replaces dv2
-            }
-        }
-        fence_proxy_async();
-        tc_fence_before();
-        __syncthreads();
-        // ---- phase 3: tmp = M^T dM
-        if (tid == 0) {
-            tc_fence_after();
-            t8::mma_chain<true, true>(tmem, tM, 0, 0, tDV2, 0, 0, 128, 128, false);
-            umma_commit(&mma_bar);
-        }
-        wait_or_flag(&mma_bar, 0, p.status, 34);
-        tc_fence_after();
-        if (tid == 0 && more) bulk_g2s(bDV2, p.DV2 + gn * CH128, 32768, &ld1);     // dM has been consumed
-#pragma unroll 1
-        for (int hh = 0; hh < 2; ++hh) {
-            tmem_row64(t8::taddr(tmem, warp, hh * 64), f);
-#pragma unroll
-            for (int c8 = 0; c8 < 8; ++c8) bP[(hh * 8 + c8) * 128 + r] = t8::pack8(f + c8 * 8);         // tmp replaces P
-        }
-        fence_proxy_async();
-        tc_fence_before();
-        __syncthreads();
-        // ---- phase 4: dAab = smask(tmp M^T)
-        if (tid == 0) {
-            tc_fence_after();
-            t8::mma_chain<false, false>(tmem + 128, tP, 0, 0, tM, 0, 0, 128, 128, false);
-            umma_commit(&mma_bar);
-        }
-        wait_or_flag(&mma_bar, 1, p.status, 35);
-        tc_fence_after();
-        if (tid == 0 && more) {                          // M and tmp have been consumed
-            bulk_g2s(bM, p.M + gn * CH128, 32768, &ld1);
-            bulk_g2s(bP, p.P + gn * CH128, 32768, &ld2);
-        }
-        {
-            const int i = r >> 1;
-#pragma unroll 1
-            for (int hh = 0; hh < 2; ++hh) {
-                tmem_row64(t8::taddr(tmem, warp, 128 + hh * 64), f);
-#pragma unroll
-                for (int c8 = 0; c8 < 8; ++c8) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) if (!(((hh * 64 + c8 * 8 + j) >> 1) < i)) f[c8 * 8 + j] = 0.f;
-                    p.dAab[g * CH128 + (hh * 8 + c8) * 128 + r] = t8::pack8(f + c8 * 8);
-                }
-            }
-        }
-        // the accumulators are read; the next tile's first products overwrite them
-        tc_fence_before();
-        __syncthreads();
+    wait_or_flag(&ld1, 0, p.status, 30);
+    if (tid == 0) {
+        t8::mma_chain<true, true>(tmem, tM, 0, 0, tDV2, 0, 0, 128, 128, false);          // dP = M^T dv2
+        umma_commit(&mma_bar);
     }
+    wait_or_flag(&mma_bar, 0, p.status, 31);
+    tc_fence_after();
+#pragma unroll 1
+    for (int hh = 0; hh < 2; ++hh) {
+        tmem_row64(t8::taddr(tmem, warp, hh * 64), f);
+#pragma unroll
+        for (int c8 = 0; c8 < 8; ++c8) {
+            const uint4 c = t8::pack8(f + c8 * 8);
+            bM[(hh * 8 + c8) * 128 + r] = c;                            // dP replaces M
+            p.dP[g * CH128 + (hh * 8 + c8) * 128 + r] = c;
+        }
+    }
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
+    wait_or_flag(&ld2, 0, p.status, 32);
+    if (tid == 0) {
+        tc_fence_after();
+        t8::mma_chain<false, false>(tmem, tM, 0, 0, tVc, 0, 0, 64, 128, false);          // dP v^T
+        t8::mma_chain<false, false>(tmem + 64, tM, 0, 0, tV2, 0, 0, 128, 128, false);    // dP v2^T
+        umma_commit(&mma_bar);
+    }
+    wait_or_flag(&mma_bar, 1, p.status, 33);
+    tc_fence_after();
+    tmem_row64(t8::taddr(tmem, warp, 0), f);
+#pragma unroll
+    for (int c8 = 0; c8 < 8; ++c8) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) if (!((c8 * 8 + j) < i)) f[c8 * 8 + j] = 0.f;
+        p.dAak[g * CH64 + c8 * 128 + r] = t8::pack8(f + c8 * 8);
+    }
+#pragma unroll 1
+    for (int hh = 0; hh < 2; ++hh) {
+        tmem_row64(t8::taddr(tmem, warp, 64 + hh * 64), f);
+#pragma unroll
+        for (int c8 = 0; c8 < 8; ++c8) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) if (!(((hh * 64 + c8 * 8 + j) >> 1) < i)) f[c8 * 8 + j] = 0.f;
+            p.dAab[g * CH128 + (hh * 8 + c8) * 128 + r] = t8::pack8(f + c8 * 8);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, 256);
 }
 
@@ -1254,6 +1171,24 @@ __global__ void c8_to_rowmajor_kernel(const uint4* src, float* dst, int rows, in
     }
 }
 
+// debugging aid: product of two C8 tiles, X [128 x n] times Y [n x 128] (or Y^T, Y [128 x n]) -> fp32 row-major, for
+// the intermediates that the pipeline itself no longer forms
+__global__ void c8_product_kernel(const uint4* x, const uint4* y, float* dst, int n, int y_transposed) {
+    const long long g = blockIdx.x;
+    const int yr = y_transposed ? 128 : n;
+    const __nv_bfloat16* xt = reinterpret_cast<const __nv_bfloat16*>(x + g * (n * 16));
+    const __nv_bfloat16* yt = reinterpret_cast<const __nv_bfloat16*>(y + g * (n * 16));
+    auto at = [](const __nv_bfloat16* t, int rows, int r, int c) {
+        return __bfloat162float(t[(((c >> 3) * rows + r) << 3) + (c & 7)]);
+    };
+    for (int e = threadIdx.x; e < 128 * 128; e += blockDim.x) {
+        const int r = e >> 7, c = e & 127;
+        float s = 0.f;
+        for (int j = 0; j < n; ++j) s = fmaf(at(xt, 128, r, j), y_transposed ? at(yt, yr, c, j) : at(yt, yr, j, c), s);
+        dst[(size_t)g * 128 * 128 + e] = s;
+    }
+}
+
 // ------------------------------------------------------------------------------------------
 // backward, last stage: gradients of the hat operands, dv, un-gating and dgk in one kernel
 //   (HRDPLR/bwd_triton.py: dv 227-290, bwd_o 295-487, score-gradient applications of intra 761-827,
@@ -1261,15 +1196,17 @@ __global__ void c8_to_rowmajor_kernel(const uint4* src, float* dst, int rows, in
 // Five products, all evaluated transposed so that the accumulator lane is the channel k (or v):
 //   P1 dQh^T = St dO^T   + Kh^T dAqk^T + Bh^T dAqb^T        [k x 64 tokens]
 //   P2 dv^T  = dSt^T Kh^T + dO^T Aqk   + dP^T Aak           [v x 64 tokens]
-//   P3 dAh^T = dWh^T M   + Kh^T dAak^T + Bh^T dAab^T        [k x 128 rows]
+//   P3 dAh^T = St dP^T   + Kh^T dAak^T + Bh^T dAab^T        [k x 128 rows]   (M^T dWh = dP St^T, see wy_bwd_tc_kernel)
 //   P4 dBh^T = dSt V2^T  + Qh^T dAqb   + Ah^T dAab          [k x 128 rows]
 //   P5 dKh^T = dSt v^T   + Qh^T dAqk   + Ah^T dAak          [k x 64 tokens]
-// They read 18 distinct tiles (416 KB) -- more than shared memory holds -- so the tiles go through
+// They read 16 distinct tiles (352 KB) -- more than shared memory holds -- so the tiles go through
 // a fixed slot schedule: five 32 KB slots A..E, three 16 KB slots a..c, two 8 KB slots x, y; a tile
 // is loaded (bulk copy) as soon as the product that last read its slot has completed:
-//   at the start: St->A dO->a Aqk->y dP->D Aak->E Kh->b dAqk->x Bh->B dAqb->c dSt->C
-//   dWh->A once St dO^T is complete, dAak->a once dO^T Aqk is, M->D and dAab->E once dP^T Aak is;
-//   Ah->B once Bh^T dAab^T is complete, V2->A, Qh->D.lo, v->D.hi once dWh^T M is.
+//   first: dP->D Aak->E.lo St->A dO->a Aqk->y Kh->b dAqk->x Bh->B dAqb->c dSt->C v->E.hi
+//   Qh->E.lo once dP^T Aak is complete, V2->A and dAab->D once St dP^T is, dAak->a once dO^T Aqk is;
+//   Ah->B once Bh^T dAab^T is.
+// Slots that the epilogue does not read (A C D a c x y) take the next tile's first tiles as soon as this tile's last
+// product is complete, while the epilogue warps still write its gradients.
 // Every group of tiles has its own load barrier, and a chain is issued when its own operands have landed.
 // All five accumulators stay in TMEM (448 columns). Sixteen epilogue warps un-gate them (dq = scale e^{gi-half}
 // dQh, ...) and write every gradient in the public layout (a warp writes 32 adjacent channels of one token)
@@ -1277,7 +1214,7 @@ __global__ void c8_to_rowmajor_kernel(const uint4* src, float* dst, int rows, in
 // and after P4/P5 walk their tokens backwards for dk, db and the running sum of dgk.
 // ------------------------------------------------------------------------------------------
 struct GradP {
-    const uint4 *Hs, *Bh, *dOc, *Kh, *dAqb, *dAqk, *DE, *dP, *Aak, *Aqk, *dW, *M, *dAab, *dAak, *V2, *Ah, *Qh, *Vc;
+    const uint4 *Hs, *Bh, *dOc, *Kh, *dAqb, *dAqk, *DE, *dP, *Aak, *Aqk, *dAab, *dAak, *V2, *Ah, *Qh, *Vc;
     const __nv_bfloat16* ghat;            // e^{gi - half}, bf16 [64][128] per tile
     const float *E, *dgl;                 // e^{half} per (tile, channel); dgL from the reverse scan
     __nv_bfloat16 *dq, *dk, *dv, *da, *db;
@@ -1308,8 +1245,9 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
     uint4* sx = sc + CH64;                               // 8 KB slots
     uint4* sy = sx + 512;
     // load barriers (one per group of tiles that a chain waits for) and commit barriers (chains or whole products)
-    __shared__ __align__(8) uint64_t ld[13], mc1, mc5, mc6, mc7, mc9, m1, m2, m3, m4;
-    enum { T_StdO, T_Aqk, T_dPAak, T_KhdAqk, T_BhdAqb, T_dSt, T_dW, T_dAak, T_M, T_dAab, T_V2, T_QhVc, T_Ah };
+    __shared__ __align__(8) uint64_t ld[13], mc1, mc5, mc6, mc9, m1, m2, m3, m4;
+    __shared__ float group_total[4][K];
+    enum { T_dP, T_Aak, T_StdO, T_Aqk, T_dAq, T_Kh, T_Bh, T_dSt, T_Vc, T_Qh, T_V2, T_dAab, T_dAakAh };
     __shared__ uint32_t tmem_s;
     const int tid = threadIdx.x, warp = tid >> 5;
     const bool producer = tid == 512;                   // lane 0 of the seventeenth warp loads tiles and issues MMAs
@@ -1317,7 +1255,7 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
     if (producer) {
 #pragma unroll
         for (int i = 0; i < 13; ++i) mbar_init(&ld[i], 1);
-        mbar_init(&mc1, 1); mbar_init(&mc5, 1); mbar_init(&mc6, 1); mbar_init(&mc7, 1); mbar_init(&mc9, 1);
+        mbar_init(&mc1, 1); mbar_init(&mc5, 1); mbar_init(&mc6, 1); mbar_init(&mc9, 1);
         mbar_init(&m1, 1); mbar_init(&m2, 1); mbar_init(&m3, 1); mbar_init(&m4, 1);
         fence_mbar_init();
     }
@@ -1326,95 +1264,94 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
     tc_fence_after();
     const uint32_t tmem = tmem_s;
     // TMEM columns: dQh^T 0..63, dv^T 64..127, dAh^T 128..255, dBh^T 256..383, dKh^T 384..447
+    // tiles whose slots the epilogue of the tile before does not read
+    auto load_ahead = [&](long long g) {
+        mbar_expect_tx(&ld[T_dP], 32768);
+        bulk_g2s(sD, p.dP + g * CH128, 32768, &ld[T_dP]);
+        mbar_expect_tx(&ld[T_StdO], 32768 + 16384);
+        bulk_g2s(sA, p.Hs + g * CH128, 32768, &ld[T_StdO]);
+        bulk_g2s(sa, p.dOc + g * CH64, 16384, &ld[T_StdO]);
+        mbar_expect_tx(&ld[T_Aqk], 8192);
+        bulk_g2s(sy, p.Aqk + g * 512, 8192, &ld[T_Aqk]);
+        mbar_expect_tx(&ld[T_dAq], 8192 + 16384);
+        bulk_g2s(sx, p.dAqk + g * 512, 8192, &ld[T_dAq]);
+        bulk_g2s(sc, p.dAqb + g * CH64, 16384, &ld[T_dAq]);
+        mbar_expect_tx(&ld[T_dSt], 32768);
+        bulk_g2s(sC, p.DE + g * CH128, 32768, &ld[T_dSt]);
+    };
+    if (producer && (long long)blockIdx.x < p.G) load_ahead(blockIdx.x);
     uint32_t it = 0;
 #pragma unroll 1
     for (long long g = blockIdx.x; g < p.G; g += gridDim.x, ++it) {
     const uint32_t ph = it & 1;
     if (producer) {
         TL(0);
-        // first loads, in the order the chains need them (the chain that frees two slots for the next
-        // generation of tiles comes first)
-        mbar_expect_tx(&ld[T_dPAak], 32768 + 16384);
-        bulk_g2s(sD, p.dP + g * CH128, 32768, &ld[T_dPAak]);
-        bulk_g2s(sE, p.Aak + g * CH64, 16384, &ld[T_dPAak]);
-        mbar_expect_tx(&ld[T_StdO], 32768 + 16384);
-        bulk_g2s(sA, p.Hs + g * CH128, 32768, &ld[T_StdO]);
-        bulk_g2s(sa, p.dOc + g * CH64, 16384, &ld[T_StdO]);
-        mbar_expect_tx(&ld[T_Aqk], 8192);
-        bulk_g2s(sy, p.Aqk + g * 512, 8192, &ld[T_Aqk]);
-        mbar_expect_tx(&ld[T_KhdAqk], 16384 + 8192);
-        bulk_g2s(sb, p.Kh + g * CH64, 16384, &ld[T_KhdAqk]);
-        bulk_g2s(sx, p.dAqk + g * 512, 8192, &ld[T_KhdAqk]);
-        mbar_expect_tx(&ld[T_BhdAqb], 32768 + 16384);
-        bulk_g2s(sB, p.Bh + g * CH128, 32768, &ld[T_BhdAqb]);
-        bulk_g2s(sc, p.dAqb + g * CH64, 16384, &ld[T_BhdAqb]);
-        mbar_expect_tx(&ld[T_dSt], 32768);
-        bulk_g2s(sC, p.DE + g * CH128, 32768, &ld[T_dSt]);
+        mbar_expect_tx(&ld[T_Aak], 16384);
+        bulk_g2s(sE, p.Aak + g * CH64, 16384, &ld[T_Aak]);
+        mbar_expect_tx(&ld[T_Kh], 16384);
+        bulk_g2s(sb, p.Kh + g * CH64, 16384, &ld[T_Kh]);
+        mbar_expect_tx(&ld[T_Bh], 32768);
+        bulk_g2s(sB, p.Bh + g * CH128, 32768, &ld[T_Bh]);
+        mbar_expect_tx(&ld[T_Vc], 16384);
+        bulk_g2s(sE + CH64, p.Vc + g * CH64, 16384, &ld[T_Vc]);
         // Chains are issued as soon as their own tiles have landed, and the chains that read a slot for the last
         // time are issued first and committed on their own, so that the slot is refilled while the rest of the
         // product still runs.
-        wait_or_flag(&ld[T_dPAak], ph, p.status, 72);
-        chain0<true, true>(tmem + 64, t8::tile(sD, 128), t8::tile(sE, 128), 64, 128, false);      // P2: dP^T Aak
-        umma_commit(&mc6);                                                                        // slots D, E free
         wait_or_flag(&ld[T_StdO], ph, p.status, 70);
         chain0<false, false>(tmem, t8::tile(sA, 128), t8::tile(sa, 64), 64, 128, false);          // P1: St dO^T
+        wait_or_flag(&ld[T_dP], ph, p.status, 72);
+        chain0<false, false>(tmem + 128, t8::tile(sA, 128), t8::tile(sD, 128), 128, 128, false);  // P3: St dP^T
         umma_commit(&mc1);                                                                        // slot A free
         wait_or_flag(&ld[T_Aqk], ph, p.status, 71);
-        chain0<true, true>(tmem + 64, t8::tile(sa, 64), t8::tile(sy, 64), 64, 64, true);          // P2: dO^T Aqk
+        chain0<true, true>(tmem + 64, t8::tile(sa, 64), t8::tile(sy, 64), 64, 64, false);         // P2: dO^T Aqk
         umma_commit(&mc5);                                                                        // slots a, y free
-        wait_or_flag(&mc6, ph, p.status, 77);
-        mbar_expect_tx(&ld[T_M], 32768);
-        bulk_g2s(sD, p.M + g * CH128, 32768, &ld[T_M]);
-        mbar_expect_tx(&ld[T_dAab], 32768);
-        bulk_g2s(sE, p.dAab + g * CH128, 32768, &ld[T_dAab]);
-        wait_or_flag(&mc1, ph, p.status, 73);
-        mbar_expect_tx(&ld[T_dW], 32768);
-        bulk_g2s(sA, p.dW + g * CH128, 32768, &ld[T_dW]);
-        wait_or_flag(&ld[T_KhdAqk], ph, p.status, 74);
-        chain0<true, false>(tmem, t8::tile(sb, 64), t8::tile(sx, 64), 64, 64, true);              // P1: Kh^T dAqk^T
+        wait_or_flag(&ld[T_Aak], ph, p.status, 73);
+        chain0<true, true>(tmem + 64, t8::tile(sD, 128), t8::tile(sE, 128), 64, 128, true);       // P2: dP^T Aak
+        umma_commit(&mc6);                                                                        // slots D, E.lo free
+        wait_or_flag(&mc1, ph, p.status, 74);
+        mbar_expect_tx(&ld[T_V2], 32768);
+        bulk_g2s(sA, p.V2 + g * CH128, 32768, &ld[T_V2]);
         wait_or_flag(&mc5, ph, p.status, 75);
-        mbar_expect_tx(&ld[T_dAak], 16384);
-        bulk_g2s(sa, p.dAak + g * CH64, 16384, &ld[T_dAak]);
-        wait_or_flag(&ld[T_BhdAqb], ph, p.status, 76);
+        mbar_expect_tx(&ld[T_dAakAh], 16384 + 32768);          // (Ah follows when slot B is free)
+        bulk_g2s(sa, p.dAak + g * CH64, 16384, &ld[T_dAakAh]);
+        wait_or_flag(&mc6, ph, p.status, 76);
+        mbar_expect_tx(&ld[T_dAab], 32768);
+        bulk_g2s(sD, p.dAab + g * CH128, 32768, &ld[T_dAab]);
+        mbar_expect_tx(&ld[T_Qh], 16384);
+        bulk_g2s(sE, p.Qh + g * CH64, 16384, &ld[T_Qh]);
+        wait_or_flag(&ld[T_Kh], ph, p.status, 77);
+        wait_or_flag(&ld[T_dAq], ph, p.status, 78);
+        chain0<true, false>(tmem, t8::tile(sb, 64), t8::tile(sx, 64), 64, 64, true);              // P1: Kh^T dAqk^T
+        wait_or_flag(&ld[T_Bh], ph, p.status, 79);
         chain0<true, false>(tmem, t8::tile(sB, 128), t8::tile(sc, 64), 64, 128, true);            // P1: Bh^T dAqb^T
         umma_commit(&m1);
-        wait_or_flag(&ld[T_dSt], ph, p.status, 78);
+        wait_or_flag(&ld[T_dSt], ph, p.status, 80);
         chain0<true, false>(tmem + 64, t8::tile(sC, 128), t8::tile(sb, 64), 64, 128, true);       // P2: dSt^T Kh^T
         umma_commit(&m2);
         TL(4);
-        wait_or_flag(&ld[T_dAab], ph, p.status, 79);
-        chain0<true, false>(tmem + 128, t8::tile(sB, 128), t8::tile(sE, 128), 128, 128, false);   // P3: Bh^T dAab^T
+        wait_or_flag(&ld[T_Vc], ph, p.status, 81);
+        chain0<false, false>(tmem + 384, t8::tile(sC, 128), t8::tile(sE + CH64, 64), 64, 128, false);  // P5: dSt v^T
+        wait_or_flag(&ld[T_dAab], ph, p.status, 82);
+        chain0<true, false>(tmem + 128, t8::tile(sB, 128), t8::tile(sD, 128), 128, 128, true);    // P3: Bh^T dAab^T
         umma_commit(&mc9);                                                                        // slot B free
-        wait_or_flag(&ld[T_dW], ph, p.status, 80);
-        wait_or_flag(&ld[T_M], ph, p.status, 81);
-        chain0<true, true>(tmem + 128, t8::tile(sA, 128), t8::tile(sD, 128), 128, 128, true);     // P3: dWh^T M
-        umma_commit(&mc7);                                                                        // slots A, D free
-        wait_or_flag(&ld[T_dAak], ph, p.status, 82);
+        wait_or_flag(&ld[T_V2], ph, p.status, 83);
+        chain0<false, false>(tmem + 256, t8::tile(sC, 128), t8::tile(sA, 128), 128, 128, false);  // P4: dSt V2^T
+        wait_or_flag(&ld[T_Qh], ph, p.status, 84);
+        chain0<true, true>(tmem + 256, t8::tile(sE, 64), t8::tile(sc, 64), 128, 64, true);        // P4: Qh^T dAqb
+        chain0<true, true>(tmem + 384, t8::tile(sE, 64), t8::tile(sx, 64), 64, 64, true);         // P5: Qh^T dAqk
+        wait_or_flag(&mc9, ph, p.status, 85);
+        TL(6);
+        bulk_g2s(sB, p.Ah + g * CH128, 32768, &ld[T_dAakAh]);
+        wait_or_flag(&ld[T_dAakAh], ph, p.status, 86);
         chain0<true, false>(tmem + 128, t8::tile(sb, 64), t8::tile(sa, 128), 128, 64, true);      // P3: Kh^T dAak^T
         umma_commit(&m3);
-        wait_or_flag(&mc9, ph, p.status, 83);
-        mbar_expect_tx(&ld[T_Ah], 32768);
-        bulk_g2s(sB, p.Ah + g * CH128, 32768, &ld[T_Ah]);
-        wait_or_flag(&mc7, ph, p.status, 84);
-        TL(6);
-        mbar_expect_tx(&ld[T_V2], 32768);
-        bulk_g2s(sA, p.V2 + g * CH128, 32768, &ld[T_V2]);
-        mbar_expect_tx(&ld[T_QhVc], 16384 + 16384);
-        bulk_g2s(sD, p.Qh + g * CH64, 16384, &ld[T_QhVc]);
-        bulk_g2s(sD + CH64, p.Vc + g * CH64, 16384, &ld[T_QhVc]);
-        wait_or_flag(&ld[T_V2], ph, p.status, 85);
-        chain0<false, false>(tmem + 256, t8::tile(sC, 128), t8::tile(sA, 128), 128, 128, false);  // P4: dSt V2^T
-        wait_or_flag(&ld[T_QhVc], ph, p.status, 86);
-        chain0<false, false>(tmem + 384, t8::tile(sC, 128), t8::tile(sD + CH64, 64), 64, 128, false);  // P5: dSt v^T
-        chain0<true, true>(tmem + 256, t8::tile(sD, 64), t8::tile(sc, 64), 128, 64, true);        // P4: Qh^T dAqb
-        chain0<true, true>(tmem + 384, t8::tile(sD, 64), t8::tile(sx, 64), 64, 64, true);         // P5: Qh^T dAqk
-        wait_or_flag(&ld[T_Ah], ph, p.status, 87);
         TL(7);
-        chain0<true, true>(tmem + 256, t8::tile(sB, 128), t8::tile(sE, 128), 128, 128, true);     // P4: Ah^T dAab
+        chain0<true, true>(tmem + 256, t8::tile(sB, 128), t8::tile(sD, 128), 128, 128, true);     // P4: Ah^T dAab
         chain0<true, true>(tmem + 384, t8::tile(sB, 128), t8::tile(sa, 128), 64, 128, true);      // P5: Ah^T dAak
         umma_commit(&m4);
         wait_or_flag(&m4, ph, p.status, 88);
         TL(8);
+        if (g + gridDim.x < p.G) load_ahead(g + gridDim.x);
     }
     if (warp < 16) {
         // Sixteen epilogue warps in four token groups: group w owns tokens 48-16w .. 63-16w of the chunk and
@@ -1422,7 +1359,6 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
         // producer is still loading: the decay factors and this thread's Bh elements are fetched from global
         // memory into registers at once, dv and dq are written as soon as P1 and P2 are complete, da after P3;
         // only dk, db and the dgk sums wait for P4 and P5.
-        float (*group_total)[K] = reinterpret_cast<float (*)[K]>(sy);      // 2 KB in the (consumed) Aqk slot
         const int bh = (int)(g / p.NT), n = (int)(g % p.NT);
         const int b = bh / p.H, h = bh % p.H;
         const int k = tid & 127, wg = tid >> 7;
@@ -1499,7 +1435,7 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
         tc_fence_after();
         if (tid == 0) TL(9);
         // per-thread element pointers into the hat tiles still in shared memory (token i sits 16 bytes after token i-1)
-        const __nv_bfloat16* eq = reinterpret_cast<const __nv_bfloat16*>(sD + (k >> 3) * 64) + (k & 7) + i_lo * 8;
+        const __nv_bfloat16* eq = reinterpret_cast<const __nv_bfloat16*>(sE + (k >> 3) * 64) + (k & 7) + i_lo * 8;
         const __nv_bfloat16* ek = reinterpret_cast<const __nv_bfloat16*>(sb + (k >> 3) * 64) + (k & 7) + i_lo * 8;
         const __nv_bfloat16* ea = reinterpret_cast<const __nv_bfloat16*>(sB + (k >> 3) * 128) + (k & 7) + i_lo * 16;
         float run = 0.f;
@@ -1681,7 +1617,7 @@ __global__ void wait_timeout_probe_kernel(int* status, unsigned long long budget
 }
 
 constexpr int kGradSmem = 5 * 32768 + 3 * 16384 + 2 * 8192;
-constexpr int kWySmem = 6 * 32768 + 16384;
+constexpr int kWySmem = 3 * 32768 + 16384;
 
 template <typename Kern>
 int set_smem(Kern kern, int bytes) {
@@ -1812,7 +1748,7 @@ int tc_chunk_fwd(const HdlaDims& d, const void* q, const void* k, const void* v,
             InvP ivp{U4(pl.Aab), U4(pl.M), status};
             launch(inverse_tc_kernel, dim3(G), dim3(128), 32768, st, ivp);
             HDLA_CHECK_LAUNCH("inverse_tc_kernel");
-            WuP wp{U4(pl.M), U4(pl.Ah), U4(pl.Aak), U4(pl.Vc), U4(pl.P), U4(pl.U), U4(pl.W), status};
+            WuP wp{U4(pl.M), U4(pl.Ah), U4(pl.Aak), U4(pl.Vc), U4(pl.U), U4(pl.W), status};
             launch(wu_tc_kernel, dim3(G), dim3(128), 98304, st, wp);
             HDLA_CHECK_LAUNCH("wu_tc_kernel");
         }
@@ -2005,15 +1941,13 @@ int tc_chunk_bwd(const HdlaDims& d, const void* q, const void* k, const void* v,
         launch(scan_tc_kernel, dim3(pl.BH), dim3(256), 196608, st, sp);
         HDLA_CHECK_LAUNCH("scan_tc_kernel");
     }
-    // --- wy: dWh, dP, dAak, dAab in one kernel
-    WyBwdP wyp{U4(pl.M), U4(pl.DV2), U4(pl.Hs), U4(pl.Vc), U4(pl.P), U4(pl.Ah), U4(pl.dW), U4(pl.dP), U4(pl.dAak),
-               U4(pl.dAab), status, (long long)G};
-    const unsigned wy_grid = G < (unsigned)sm_count() ? G : (unsigned)sm_count();      // one persistent CTA per SM
-    launch(wy_bwd_tc_kernel, dim3(wy_grid), dim3(128), kWySmem, st, wyp);
+    // --- wy: dP, dAak, dAab in one kernel
+    WyBwdP wyp{U4(pl.M), U4(pl.DV2), U4(pl.Vc), U4(pl.V2), U4(pl.dP), U4(pl.dAak), U4(pl.dAab), status};
+    launch(wy_bwd_tc_kernel, dim3(G), dim3(128), kWySmem, st, wyp);
     HDLA_CHECK_LAUNCH("wy_bwd_tc_kernel");
     // --- everything else: hat-operand gradients, dv, un-gating, dgk
     GradP gp{U4(pl.Hs), U4(pl.Bh), U4(pl.dOc), U4(pl.Kh), U4(pl.dAqb), U4(pl.dAqk), U4(pl.DE), U4(pl.dP), U4(pl.Aak),
-             U4(pl.Aqk), U4(pl.dW), U4(pl.M), U4(pl.dAab), U4(pl.dAak), U4(pl.V2), U4(pl.Ah), U4(pl.Qh), U4(pl.Vc),
+             U4(pl.Aqk), U4(pl.dAab), U4(pl.dAak), U4(pl.V2), U4(pl.Ah), U4(pl.Qh), U4(pl.Vc),
              (bp)(ws + pl.ghat), F(pl.E), F(pl.dgl), (bp)dq, (bp)dk, (bp)dv, param_ab ? (bp)(ws + pl.dab) : (bp)da,
              param_ab ? (bp)(ws + pl.dab + pl.dab_half) : (bp)db, dgk, scale, d.T, d.H, pl.NT, d.gk_dtype,
              status, (long long)G, d.K, d.V, chunk_tab};
@@ -2033,10 +1967,10 @@ int tc_debug_buffer(const HdlaDims& d, const unsigned char* ws, const char* name
     const Ent tab[] = {{"Qh", pl.Qh, 64, 128}, {"Kh", pl.Kh, 64, 128}, {"Ah", pl.Ah, 128, 128}, {"Bh", pl.Bh, 128, 128},
                        {"Vc", pl.Vc, 64, 128}, {"Aqk", pl.Aqk, 64, 64}, {"Aqb", pl.Aqb, 64, 128},
                        {"Aak", pl.Aak, 128, 64}, {"M", pl.M, 128, 128},
-                       {"W", pl.W, 128, 128}, {"P", pl.P, 128, 128}, {"U", pl.U, 128, 128}, {"Hs", pl.Hs, 128, 128},
+                       {"W", pl.W, 128, 128}, {"U", pl.U, 128, 128}, {"Hs", pl.Hs, 128, 128},
                        {"V2", pl.V2, 128, 128},
                        {"dOc", pl.dOc, 64, 128}, {"dAqk", pl.dAqk, 64, 64}, {"dAqb", pl.dAqb, 64, 128},
-                       {"DV2", pl.DV2, 128, 128}, {"DE", pl.DE, 128, 128}, {"dW", pl.dW, 128, 128},
+                       {"DV2", pl.DV2, 128, 128}, {"DE", pl.DE, 128, 128},
                        {"dP", pl.dP, 128, 128}, {"dAak", pl.dAak, 128, 64}, {"dAab", pl.dAab, 128, 128}};
     for (const Ent& e : tab)
         if (!strcmp(e.n, name)) {
@@ -2045,6 +1979,14 @@ int tc_debug_buffer(const HdlaDims& d, const unsigned char* ws, const char* name
             HDLA_CHECK_LAUNCH("c8_to_rowmajor_kernel");
             return HDLA_OK;
         }
+    if (!strcmp(name, "P") || !strcmp(name, "dW")) {         // P = Aak v,  dWh = dv2 St^T
+        const bool fwd = name[0] == 'P';
+        c8_product_kernel<<<(unsigned)pl.G, 128, 0, st>>>(reinterpret_cast<const uint4*>(ws + (fwd ? pl.Aak : pl.DV2)),
+                                                          reinterpret_cast<const uint4*>(ws + (fwd ? pl.Vc : pl.Hs)), out,
+                                                          fwd ? 64 : 128, fwd ? 0 : 1);
+        HDLA_CHECK_LAUNCH("c8_product_kernel");
+        return HDLA_OK;
+    }
     if (!strcmp(name, "E")) {
         cudaMemcpyAsync(out, ws + pl.E, (size_t)pl.G * K * 4, cudaMemcpyDeviceToDevice, st);
         return HDLA_OK;

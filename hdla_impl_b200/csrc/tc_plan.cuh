@@ -19,11 +19,11 @@ constexpr int CH128 = 16 * 128;    // chunks of a [128 x 128] tile
 struct TcPlan {
     int B, T, H, NT, BH;               // NT: chunks per sequence (all chunks of the packed batch with cu_seqlens);
     long long G;                       // BH: (sequence, head) pairs = scans and states;  G = tiles = H * chunks
-    size_t status, Qh, Kh, Ah, Bh, Vc, E, ghat, Aqk, Aqb, Aak, Aab, M, W, P, U, Hs, V2, HT, zero;
+    size_t status, Qh, Kh, Ah, Bh, Vc, E, ghat, Aqk, Aqb, Aak, Aab, M, W, U, Hs, V2, HT, zero;
     int nseg, seg_len;                 // two-level scan: segments per sequence, chunks per segment
     int lead_real;                     // the first segment in scan order is scanned for real in the first pass
     size_t Tseg, Fseg, Sin;            // per (b, h, segment): transition [K,K], state from zero [K,V], entering state [K,V]
-    size_t dOc, dAqk, dAqb, DV2, DE, dgl, dW, dP, dAak, dAab;
+    size_t dOc, dAqk, dAqb, DV2, DE, dgl, dP, dAak, dAab;
     size_t dab, dab_half;              // in-operator a/b parametrisation: da then db, dab_half bytes each
     size_t total_fwd, total;
     int nseq;                          // sequences of a packed variable-length batch, 0 otherwise
@@ -64,7 +64,7 @@ inline TcPlan make_tc_plan(const HdlaDims& d) {
     p.chunk_tab = off; off += p.nseq ? (((size_t)p.NT * 8 + 255) / 256) * 256 : 0;
     p.seq_tab = off; off += p.nseq ? (((size_t)p.nseq * 8 + 255) / 256) * 256 : 0;
     // forward region: what the scan and the output kernel read.  The fused preparation kernel (HDLA_FLAG_FUSED_PREP)
-    // keeps Aab on chip and writes Ah, Aak, M, P and the un-gating factors only for a backward pass, so with it
+    // keeps Aab on chip and writes Ah, Aak, M and the un-gating factors only for a backward pass, so with it
     // those live in the backward region; the four-kernel preparation passes them from kernel to kernel.
     // (it needs full head dims and does not form a and b itself)
     const bool fused = (d.flags & HDLA_FLAG_FUSED_PREP) != 0 && d.K == K && d.V == V && !(d.flags & HDLA_FLAG_PARAM_AB);
@@ -73,7 +73,7 @@ inline TcPlan make_tc_plan(const HdlaDims& d) {
     p.Aqk = take(8192); p.Aqb = take(16384);
     p.W = take(32768); p.U = take(32768); p.Hs = take(32768); p.V2 = take(32768);
     if (!fused) {
-        p.Ah = take(32768); p.ghat = take(C * K * 2); p.Aak = take(16384); p.M = take(32768); p.P = take(32768);
+        p.Ah = take(32768); p.ghat = take(C * K * 2); p.Aak = take(16384); p.M = take(32768);
         p.Aab = take(32768);
     }
     p.HT = off; off += (((size_t)p.BH * K * V * 4 + 255) / 256) * 256;
@@ -108,11 +108,11 @@ inline TcPlan make_tc_plan(const HdlaDims& d) {
     p.total_fwd = off;
     // backward region: forward intermediates that only the backward kernels read, then the backward's own
     if (fused) {
-        p.Ah = take(32768); p.ghat = take(C * K * 2); p.Aak = take(16384); p.M = take(32768); p.P = take(32768);
+        p.Ah = take(32768); p.ghat = take(C * K * 2); p.Aak = take(16384); p.M = take(32768);
         p.Aab = 0;                                         // never leaves the SM
     }
     p.dOc = take(16384); p.dAqk = take(8192); p.dAqb = take(16384); p.DV2 = take(32768); p.DE = take(32768);
-    p.dgl = take(K * 4); p.dW = take(32768); p.dP = take(32768); p.dAak = take(16384); p.dAab = take(32768);
+    p.dgl = take(K * 4); p.dP = take(32768); p.dAak = take(16384); p.dAab = take(32768);
     // in-operator a/b parametrisation: da and db, each [B, 2T, H, K] bf16 in the public layout, stay here for the
     // parametrisation's backward kernel
     p.dab_half = (((size_t)d.B * d.T * R * d.H * d.K * 2 + 255) / 256) * 256;
