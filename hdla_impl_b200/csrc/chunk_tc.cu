@@ -11,6 +11,11 @@
 //     v2 = Wh St + u ;  o = Qh St + Aqk v + Aqb v2 ;  S' = E (.) (St + Kh^T v + Bh^T v2)
 // and no product needs an operand scaled by more than e^{|g_last|/2}.
 //
+// Head dims below 128: a [rows x channels] tile keeps its 128-wide slot but only its first KW (VW) = head dim rounded
+// up to 16 columns are written, moved and multiplied -- column groups are contiguous in C8, so that is a prefix -- and a
+// state tile is [KW x VW] with a row pitch of KW.  The kernels exist twice: FULL (128 x 128, extents are constants) and
+// with the extents as arguments.  B4 T2001 H16 K=V=64 fwd+bwd: 866 us with zero-padded 128-wide tiles, 749 us so.
+//
 // All matrices between kernels are bf16 in the C8 blocked layout (tc_tiles.cuh) and move with
 // bulk asynchronous copies; all products run on tcgen05.mma with fp32 accumulation in TMEM.
 #include <cstring>
@@ -42,6 +47,7 @@ struct PrepP {
     int* status;
     int Kd, Vd;                           // head dims of the public tensors (multiples of 8, <= 128); the tiles are padded with zeros
     const int2* chunk_tab;                // variable-length batches: (first token, tokens) per chunk, else null
+    int KW, VW;                           // widths of the tiles (head dims rounded up to 16), <= 128
     const __nv_bfloat16* beta;            // in-operator a/b parametrisation: [B,T,H]; a and b are not read, gk is log_f
     int norm_k;                           // ... with k normalised on the way: k <- k / sqrt(sum_K k^2 + kNormEps)
 };
@@ -54,9 +60,7 @@ struct PrepIn { uint4 q, k, v, a0, a1, b0, b1; };
 // replaced by zeros where the data is used (a load inside a condition, merged with a default after it, can be waited
 // for where the condition ends, which would undo the request one step ahead).
 template <bool AB>
-__device__ __forceinline__ PrepIn prep_load(const PrepP& p, int b, int h, int t0, int valid, int blk, int lane) {
-    const int r = (blk >> 2) * 8 + (lane & 7);
-    const int kc = (blk & 3) * 4 + (lane >> 3);
+__device__ __forceinline__ PrepIn prep_load(const PrepP& p, int b, int h, int t0, int valid, int r, int kc) {
     const uint4 zero = make_uint4(0, 0, 0, 0);
     const bool row_ok = r < valid, k_ok = row_ok && kc * 8 < p.Kd, v_ok = row_ok && kc * 8 < p.Vd;
     const int rc = row_ok ? r : valid - 1;
@@ -85,7 +89,7 @@ __device__ __forceinline__ PrepIn prep_load(const PrepP& p, int b, int h, int t0
 // of k and reduces ef k^2 over the warp; ef of a piece in the hat loop is e^{gi - ge}.  With norm_k the layer's
 // l2_norm of k (HRDPLR/hdla_custom.py:248, normalizations/l2_norm.py:4-14) happens here too: the same phase reduces
 // k^2, and every use of k below is k / sqrt(sum_K k^2 + eps).
-template <bool AB>
+template <bool AB, bool FULL>
 __global__ void __launch_bounds__(128) prep_hat_kernel(PrepP p) {
     __shared__ float gis[C][K + 4];
     __shared__ float tot[4][K];
@@ -100,7 +104,9 @@ __global__ void __launch_bounds__(128) prep_hat_kernel(PrepP p) {
     // before the decay sums (they do not depend on them), and inside the loop the next step's pieces are
     // requested before the current step's arithmetic and stores.
     if (tid == 0) TL(0);
-    PrepIn cur = prep_load<AB>(p, b, h, t0, valid, warp * 8, lane);
+    const int KW = FULL ? K : p.KW, VW = FULL ? V : p.VW;
+    const int nq = FULL ? 4 : (max(KW, VW) + 31) >> 5;            // blocks of four column groups that hold data
+    PrepIn cur = prep_load<AB>(p, b, h, t0, valid, warp * 16 + (lane & 7), lane >> 3);
     {   // two-level cumulative sum: warp w owns rows [16w, 16w+16), lane owns 4 columns
         // (all sixteen loads are issued before the first value is used: the dtype branch stays outside the loops)
         float4 x[16];
@@ -185,13 +191,15 @@ __global__ void __launch_bounds__(128) prep_hat_kernel(PrepP p) {
     }
     // hat operands: per instruction a warp covers 8 rows x 4 column groups, so every global access
     // is a run of full 32-byte sectors (64 B per row in, 128 B per column group out)
+    int rb = warp * 16, qd = 0;                        // block of (8 rows from rb x 4 column groups from 4 qd)
 #pragma unroll 2
-    for (int it = 0; it < 8; ++it) {
-        const int blk = warp * 8 + it;                 // 32 blocks of (8 rows x 4 column groups)
-        const int r = (blk >> 2) * 8 + (lane & 7);
-        const int kc = (blk & 3) * 4 + (lane >> 3);
+    for (int it = 0; it < 2 * nq; ++it) {
+        const int r = rb + (lane & 7);
+        const int kc = qd * 4 + (lane >> 3);
+        if (++qd == nq) { qd = 0; rb += 8; }
         PrepIn nxt = cur;
-        if (it < 7) nxt = prep_load<AB>(p, b, h, t0, valid, blk + 1, lane);
+        if (it + 1 < 2 * nq) nxt = prep_load<AB>(p, b, h, t0, valid, rb + (lane & 7), qd * 4 + (lane >> 3));
+        const bool k_in = FULL || kc * 8 < KW, v_in = FULL || kc * 8 < VW;      // inside the tiles
         float gi[8], ge[8], hf[8];
         {
             const float4 g0 = *reinterpret_cast<const float4*>(&gis[r][kc * 8]);
@@ -218,7 +226,7 @@ __global__ void __launch_bounds__(128) prep_hat_kernel(PrepP p) {
         t8::unpack8(cur.q, x);
 #pragma unroll
         for (int j = 0; j < 8; ++j) y[j] = x[j] * (p.scale * mk) * ep[j];
-        p.Qh[(size_t)g * CH64 + kc * 64 + r] = t8::pack8(y);
+        if (k_in) p.Qh[(size_t)g * CH64 + kc * 64 + r] = t8::pack8(y);
         t8::unpack8(cur.k, x);
         if (AB) {
             const float rn = beta_s[r].z;
@@ -227,8 +235,8 @@ __global__ void __launch_bounds__(128) prep_hat_kernel(PrepP p) {
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) y[j] = x[j] * em[j];
-        p.Kh[(size_t)g * CH64 + kc * 64 + r] = t8::pack8(y);
-        p.Vc[(size_t)g * CH64 + kc * 64 + r] = (r < valid && kc * 8 < p.Vd) ? cur.v : make_uint4(0, 0, 0, 0);
+        if (k_in) p.Kh[(size_t)g * CH64 + kc * 64 + r] = t8::pack8(y);
+        if (v_in) p.Vc[(size_t)g * CH64 + kc * 64 + r] = (r < valid && kc * 8 < p.Vd) ? cur.v : make_uint4(0, 0, 0, 0);
         if (AB) {   // x still holds this piece of k
             const float4 bs = beta_s[r];
             float a0[8], z[8];
@@ -239,13 +247,13 @@ __global__ void __launch_bounds__(128) prep_hat_kernel(PrepP p) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) { z[j] = __expf(gi[j] - ge[j]); y[j] = a0[j] * (z[j] + bs.y) * ea[j]; }
             c1 = t8::pack8(y);
-            sm100::st_global_32B(p.Ah + (size_t)g * CH128 + kc * 128 + r * R, c0, c1);
+            if (k_in) sm100::st_global_32B(p.Ah + (size_t)g * CH128 + kc * 128 + r * R, c0, c1);
 #pragma unroll
             for (int j = 0; j < 8; ++j) { y[j] = z[j] * x[j] * em[j]; z[j] = x[j] * em[j]; }
             c0 = t8::pack8(y);
             c1 = t8::pack8(z);
-            sm100::st_global_32B(p.Bh + (size_t)g * CH128 + kc * 128 + r * R, c0, c1);
-            *reinterpret_cast<uint4*>(p.ghat + (size_t)g * C * K + (size_t)r * K + kc * 8) = t8::pack8(ep);
+            if (k_in) sm100::st_global_32B(p.Bh + (size_t)g * CH128 + kc * 128 + r * R, c0, c1);
+            if (k_in) *reinterpret_cast<uint4*>(p.ghat + (size_t)g * C * K + (size_t)r * K + kc * 8) = t8::pack8(ep);
         } else {   // rows 2r, 2r+1 of Ah / Bh are adjacent chunks: one 32-byte store each
             uint4 c0, c1;
             t8::unpack8(cur.a0, x);
@@ -256,7 +264,7 @@ __global__ void __launch_bounds__(128) prep_hat_kernel(PrepP p) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) y[j] = x[j] * ea[j];
             c1 = t8::pack8(y);
-            sm100::st_global_32B(p.Ah + (size_t)g * CH128 + kc * 128 + r * R, c0, c1);
+            if (k_in) sm100::st_global_32B(p.Ah + (size_t)g * CH128 + kc * 128 + r * R, c0, c1);
             t8::unpack8(cur.b0, x);
 #pragma unroll
             for (int j = 0; j < 8; ++j) y[j] = x[j] * em[j];
@@ -265,10 +273,10 @@ __global__ void __launch_bounds__(128) prep_hat_kernel(PrepP p) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) y[j] = x[j] * em[j];
             c1 = t8::pack8(y);
-            sm100::st_global_32B(p.Bh + (size_t)g * CH128 + kc * 128 + r * R, c0, c1);
+            if (k_in) sm100::st_global_32B(p.Bh + (size_t)g * CH128 + kc * 128 + r * R, c0, c1);
             // the un-gating factors of the backward pass, e^{gi - half}, in bf16 (their error, 2^-9, is below the
             // rounding of the bf16 gradients they scale)
-            *reinterpret_cast<uint4*>(p.ghat + (size_t)g * C * K + (size_t)r * K + kc * 8) = t8::pack8(ep);
+            if (k_in) *reinterpret_cast<uint4*>(p.ghat + (size_t)g * C * K + (size_t)r * K + kc * 8) = t8::pack8(ep);
         }
         cur = nxt;
         if (tid == 0) TL(2 + it);
@@ -285,9 +293,12 @@ struct GramP {
     const uint4 *Qh, *Kh, *Ah, *Bh;
     uint4 *Aqk, *Aqb, *Aak, *Aab;
     int* status;
+    int KW;
 };
 
+template <bool FULL>
 __global__ void __launch_bounds__(128) gram_tc_kernel(GramP p) {
+    const int KW = FULL ? K : p.KW;
     extern __shared__ __align__(1024) unsigned char smem[];
     uint4* sQ = reinterpret_cast<uint4*>(smem);                  // [64 x 128]  16 KB
     uint4* sK = sQ + CH64;                                       // [64 x 128]  16 KB
@@ -300,11 +311,11 @@ __global__ void __launch_bounds__(128) gram_tc_kernel(GramP p) {
     if (warp == 0) { tmem_alloc(&tmem_s, 256); tmem_relinquish(); }
     if (tid == 0) {
         mbar_init(&ld_bar, 1); mbar_init(&mma_bar, 1); fence_mbar_init();
-        mbar_expect_tx(&ld_bar, 98304);
-        bulk_g2s(sQ, p.Qh + g * CH64, 16384, &ld_bar);
-        bulk_g2s(sK, p.Kh + g * CH64, 16384, &ld_bar);
-        bulk_g2s(sA, p.Ah + g * CH128, 32768, &ld_bar);
-        bulk_g2s(sB, p.Bh + g * CH128, 32768, &ld_bar);
+        mbar_expect_tx(&ld_bar, 768 * KW);
+        bulk_g2s(sQ, p.Qh + g * CH64, 128 * KW, &ld_bar);
+        bulk_g2s(sK, p.Kh + g * CH64, 128 * KW, &ld_bar);
+        bulk_g2s(sA, p.Ah + g * CH128, 256 * KW, &ld_bar);
+        bulk_g2s(sB, p.Bh + g * CH128, 256 * KW, &ld_bar);
     }
     tc_fence_before();
     __syncthreads();
@@ -313,8 +324,8 @@ __global__ void __launch_bounds__(128) gram_tc_kernel(GramP p) {
     const Tile tQ = t8::tile(sQ, 64), tK = t8::tile(sK, 64), tA = t8::tile(sA, 128), tB = t8::tile(sB, 128);
     wait_or_flag(&ld_bar, 0, p.status, 2);
     if (tid == 0) {
-        t8::mma_chain<false, false>(tmem, tA, 0, 0, tK, 0, 0, 64, K, false);
-        t8::mma_chain<false, false>(tmem + 64, tA, 0, 0, tB, 0, 0, 128, K, false);
+        t8::mma_chain<false, false>(tmem, tA, 0, 0, tK, 0, 0, 64, KW, false);
+        t8::mma_chain<false, false>(tmem + 64, tA, 0, 0, tB, 0, 0, 128, KW, false);
         umma_commit(&mma_bar);
     }
     wait_or_flag(&mma_bar, 0, p.status, 3);
@@ -345,8 +356,8 @@ __global__ void __launch_bounds__(128) gram_tc_kernel(GramP p) {
     tc_fence_after();
     if (tid == 0) {
         // Qh has 64 rows: the upper 64 lanes of this M=128 product read past the tile and are ignored
-        t8::mma_chain<false, false>(tmem, tQ, 0, 0, tK, 0, 0, 64, K, false);
-        t8::mma_chain<false, false>(tmem + 64, tQ, 0, 0, tB, 0, 0, 128, K, false);
+        t8::mma_chain<false, false>(tmem, tQ, 0, 0, tK, 0, 0, 64, KW, false);
+        t8::mma_chain<false, false>(tmem + 64, tQ, 0, 0, tB, 0, 0, 128, KW, false);
         umma_commit(&mma_bar);
     }
     wait_or_flag(&mma_bar, 1, p.status, 4);
@@ -522,9 +533,12 @@ struct WuP {
     const uint4 *M, *Ah, *Aak, *Vc;
     uint4 *U, *W;
     int* status;
+    int KW, VW;
 };
 
+template <bool FULL>
 __global__ void __launch_bounds__(128) wu_tc_kernel(WuP p) {
+    const int KW = FULL ? K : p.KW, VW = FULL ? V : p.VW;
     extern __shared__ __align__(1024) unsigned char smem[];
     uint4* sM = reinterpret_cast<uint4*>(smem);                  // 32 KB
     uint4* sA = sM + CH128;                                      // 32 KB  Ah
@@ -538,11 +552,11 @@ __global__ void __launch_bounds__(128) wu_tc_kernel(WuP p) {
     if (warp == 0) { tmem_alloc(&tmem_s, 256); tmem_relinquish(); }
     if (tid == 0) {
         mbar_init(&ld_bar, 1); mbar_init(&mma_bar, 1); fence_mbar_init();
-        mbar_expect_tx(&ld_bar, 98304);
+        mbar_expect_tx(&ld_bar, 16384 + 128 * VW + 32768 + 256 * KW);
         bulk_g2s(sAak, p.Aak + g * CH64, 16384, &ld_bar);
-        bulk_g2s(sV, p.Vc + g * CH64, 16384, &ld_bar);
+        bulk_g2s(sV, p.Vc + g * CH64, 128 * VW, &ld_bar);
         bulk_g2s(sM, p.M + g * CH128, 32768, &ld_bar);
-        bulk_g2s(sA, p.Ah + g * CH128, 32768, &ld_bar);
+        bulk_g2s(sA, p.Ah + g * CH128, 256 * KW, &ld_bar);
     }
     tc_fence_before();
     __syncthreads();
@@ -552,19 +566,19 @@ __global__ void __launch_bounds__(128) wu_tc_kernel(WuP p) {
                tP = t8::tile(sP, 128);
     wait_or_flag(&ld_bar, 0, p.status, 8);
     if (tid == 0) {
-        t8::mma_chain<false, true>(tmem, tAak, 0, 0, tV, 0, 0, 128, 64, false);          // P = Aak v
-        t8::mma_chain<false, true>(tmem + 128, tM, 0, 0, tA, 0, 0, 128, 128, false);     // Wh = M Ah
+        t8::mma_chain<false, true>(tmem, tAak, 0, 0, tV, 0, 0, VW, 64, false);           // P = Aak v
+        t8::mma_chain<false, true>(tmem + 128, tM, 0, 0, tA, 0, 0, KW, 128, false);      // Wh = M Ah
         umma_commit(&mma_bar);
     }
     wait_or_flag(&mma_bar, 0, p.status, 9);
     tc_fence_after();
 #pragma unroll 1
-    for (int hh = 0; hh < 2; ++hh) {
+    for (int hh = 0; hh * 64 < VW; ++hh) {
         float f[64];
         tmem_row64(t8::taddr(tmem, warp, hh * 64), f);
 #pragma unroll
         for (int cg = 0; cg < 8; ++cg) {
-            sP[(hh * 8 + cg) * 128 + tid] = t8::pack8(f + cg * 8);
+            if (FULL || (hh * 8 + cg) * 8 < VW) sP[(hh * 8 + cg) * 128 + tid] = t8::pack8(f + cg * 8);
         }
     }
     fence_proxy_async();
@@ -572,24 +586,24 @@ __global__ void __launch_bounds__(128) wu_tc_kernel(WuP p) {
     __syncthreads();
     if (tid == 0) {
         tc_fence_after();
-        t8::mma_chain<false, true>(tmem, tM, 0, 0, tP, 0, 0, 128, 128, false);           // u = M P
+        t8::mma_chain<false, true>(tmem, tM, 0, 0, tP, 0, 0, VW, 128, false);            // u = M P
         umma_commit(&mma_bar);
     }
 #pragma unroll 1
-    for (int hh = 0; hh < 2; ++hh) {                                                      // Wh while u runs
+    for (int hh = 0; hh * 64 < KW; ++hh) {                                                // Wh while u runs
         float f[64];
         tmem_row64(t8::taddr(tmem, warp, 128 + hh * 64), f);
 #pragma unroll
-        for (int cg = 0; cg < 8; ++cg) p.W[g * CH128 + (hh * 8 + cg) * 128 + tid] = t8::pack8(f + cg * 8);
+        for (int cg = 0; cg < 8; ++cg) if (FULL || (hh * 8 + cg) * 8 < KW) p.W[g * CH128 + (hh * 8 + cg) * 128 + tid] = t8::pack8(f + cg * 8);
     }
     wait_or_flag(&mma_bar, 1, p.status, 10);
     tc_fence_after();
 #pragma unroll 1
-    for (int hh = 0; hh < 2; ++hh) {
+    for (int hh = 0; hh * 64 < VW; ++hh) {
         float f[64];
         tmem_row64(t8::taddr(tmem, warp, hh * 64), f);
 #pragma unroll
-        for (int cg = 0; cg < 8; ++cg) p.U[g * CH128 + (hh * 8 + cg) * 128 + tid] = t8::pack8(f + cg * 8);
+        for (int cg = 0; cg < 8; ++cg) if (FULL || (hh * 8 + cg) * 8 < VW) p.U[g * CH128 + (hh * 8 + cg) * 128 + tid] = t8::pack8(f + cg * 8);
     }
     tc_fence_before();
     __syncthreads();
@@ -644,12 +658,14 @@ struct ScanTcP {
     // head dims of the PUBLIC state tensors (h0 / ht / dht / dh0, [.., Kd, Vd]); states kept in the workspace
     // (the by-slot ones, the transition result and fin2) are always K x V = 128 x 128
     int Kd, Vd;
+    int KW, VW;                              // widths of the tiles (head dims rounded up to 16); a T / checkpoint tile is [KW x VW]
     // variable-length batches: pair bh = (sequence, head) scans chunks seq_tab[sequence] = (first chunk, chunks) of
     // head h's row of tiles (tile = h * NT + chunk); null for uniform batches (pair bh scans tiles bh * NT ..)
     const int2* seq_tab;
     int H;
 };
 
+template <bool FULL>
 __global__ void __launch_bounds__(256) scan_tc_kernel(ScanTcP p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     uint4* sA1 = reinterpret_cast<uint4*>(smem);     // 32 KB
@@ -676,6 +692,11 @@ __global__ void __launch_bounds__(256) scan_tc_kernel(ScanTcP p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row = (warp & 3) * 32 + lane;
     const int half = warp >> 2;
+    const int KW = FULL ? K : p.KW;
+    const int VW = FULL ? V : p.init_identity ? p.KW : p.VW;          // the transition's state is K x K
+    const int HC = FULL ? 64 : VW >> 1;                               // columns of this thread: half * HC ..  (a multiple of 8)
+    const bool row_in = FULL || row < KW;
+    const uint32_t a_bytes = 256 * KW, y_bytes = 256 * VW, l_bytes = 128 * KW, r_bytes = 128 * VW;
     TLS(0);
     if (warp == 0) { tmem_alloc(&tmem_s, 256); tmem_relinquish(); }
     long long g0 = (long long)bh * p.NT;
@@ -694,26 +715,28 @@ __global__ void __launch_bounds__(256) scan_tc_kernel(ScanTcP p) {
         // (an empty sequence of a packed batch has no chunk: nothing is requested -- nothing would wait for it and
         //  the CTA must not leave with copies into its shared memory in flight -- and its final state is its initial one)
         if (steps > 0) {
-            mbar_expect_tx(&ldA, 65536);
-            bulk_g2s(sA1, p.A1 + g * CH128, 32768, &ldA);
-            bulk_g2s(sADD, p.ADD + g * p.add_stride * CH128, 32768, &ldA);
-            mbar_expect_tx(&ldB, 65536);
-            bulk_g2s(sL1, p.L1 + g * p.r1_stride * CH64, 16384, &ldB);
-            bulk_g2s(sR1, p.R1 + g * p.r1_stride * CH64, 16384, &ldB);
-            bulk_g2s(sL2, p.L2 + g * CH128, 32768, &ldB);
+            mbar_expect_tx(&ldA, a_bytes + y_bytes);
+            bulk_g2s(sA1, p.A1 + g * CH128, a_bytes, &ldA);
+            bulk_g2s(sADD, p.ADD + g * p.add_stride * CH128, y_bytes, &ldA);
+            mbar_expect_tx(&ldB, l_bytes + r_bytes + a_bytes);
+            bulk_g2s(sL1, p.L1 + g * p.r1_stride * CH64, l_bytes, &ldB);
+            bulk_g2s(sR1, p.R1 + g * p.r1_stride * CH64, r_bytes, &ldB);
+            bulk_g2s(sL2, p.L2 + g * CH128, a_bytes, &ldB);
         }
     }
     float S[64];
     if (p.init_identity) {
 #pragma unroll
-        for (int j = 0; j < 64; ++j) S[j] = (half * 64 + j == row) ? 1.f : 0.f;
+        for (int j = 0; j < 64; ++j) S[j] = ((FULL || j < HC) && half * HC + j == row) ? 1.f : 0.f;
     } else if (p.init) {
         const size_t is = p.init_by_slot ? (size_t)slot : (size_t)bh;
         const int kd = p.init_by_slot ? K : p.Kd, vd = p.init_by_slot ? V : p.Vd;
-        const float4* src = reinterpret_cast<const float4*>(p.init + (is * kd + row) * vd + half * 64);
+        const float4* src = reinterpret_cast<const float4*>(p.init + (is * kd + row) * vd + half * HC);
+        // (rows and columns beyond the tile: a by-slot state holds nothing there)
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            const float4 x = (row < kd && half * 64 + 4 * j < vd) ? src[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 x = (row < kd && row_in && half * HC + 4 * j < vd && (FULL || 4 * j < HC)) ? src[j]
+                                                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
             S[4 * j] = x.x; S[4 * j + 1] = x.y; S[4 * j + 2] = x.z; S[4 * j + 3] = x.w;
         }
     } else {
@@ -725,7 +748,7 @@ __global__ void __launch_bounds__(256) scan_tc_kernel(ScanTcP p) {
     tc_fence_after();
     const uint32_t tmem = tmem_s;
     const Tile tA1 = t8::tile(sA1, 128), tL1 = t8::tile(sL1, 64), tR1 = t8::tile(sR1, 64), tL2 = t8::tile(sL2, 128),
-               tT = t8::tile(sT, 128), tY = t8::tile(sY, 128);
+               tT = t8::tile(sT, KW), tY = t8::tile(sY, 128);
     float e_next = steps > 0 ? p.E[(size_t)(g0 + n_first) * K + row] : 0.f;
     const bool want_dgl = p.reverse && !p.no_store;
     uint4 hs[8];                                                 // reverse scan: St of the following chunk, for dgl
@@ -733,7 +756,8 @@ __global__ void __launch_bounds__(256) scan_tc_kernel(ScanTcP p) {
     if (want_dgl && steps > 0 && n_first + 1 < NTp) {            // a segment that does not end the sequence
         e_hs = p.E[(size_t)(g0 + n_first + 1) * K + row];
 #pragma unroll
-        for (int c8 = 0; c8 < 8; ++c8) hs[c8] = __ldg(p.Hs + (g0 + n_first + 1) * CH128 + (half * 8 + c8) * 128 + row);
+        for (int c8 = 0; c8 < 8; ++c8)
+            if (FULL || (row_in && c8 * 8 < HC)) hs[c8] = __ldg(p.Hs + (g0 + n_first + 1) * CH128 + ((half * HC >> 3) + c8) * KW + row);
     }
     TLS(1);
     for (int it = 0; it < steps; ++it) {
@@ -749,18 +773,20 @@ __global__ void __launch_bounds__(256) scan_tc_kernel(ScanTcP p) {
             // step's): requested here, used after the first product is issued -- the pack, the barrier and the issue
             // in between cover most of the round trip
 #pragma unroll
-            for (int c8 = 0; c8 < 8; ++c8) hs[c8] = __ldg(p.Hs + (g + 1) * CH128 + (half * 8 + c8) * 128 + row);
+            for (int c8 = 0; c8 < 8; ++c8)
+                if (FULL || (row_in && c8 * 8 < HC)) hs[c8] = __ldg(p.Hs + (g + 1) * CH128 + ((half * HC >> 3) + c8) * KW + row);
         }
         // T = E (.) X  -> operand tile and checkpoint
 #pragma unroll
         for (int c8 = 0; c8 < 8; ++c8) {
+            if (!FULL && !(row_in && c8 * 8 < HC)) continue;
             float f[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) f[j] = e * S[c8 * 8 + j];
             const uint4 c = t8::pack8(f);
-            const int cg = half * 8 + c8;
-            sT[cg * 128 + row] = c;
-            if (!p.no_store) p.CK[g * CH128 + cg * 128 + row] = c;
+            const int cg = (half * HC >> 3) + c8;
+            sT[cg * KW + row] = c;
+            if (!p.no_store) p.CK[g * CH128 + cg * KW + row] = c;
         }
         fence_proxy_async();
         tc_fence_before();
@@ -768,11 +794,11 @@ __global__ void __launch_bounds__(256) scan_tc_kernel(ScanTcP p) {
         if (tid == 0) {
             wait_or_flag(&ldA, ph, p.status, 11);
             tc_fence_after();
-            t8::mma_chain<false, true>(tmem, tA1, 0, 0, tT, 0, 0, 128, 128, false);      // A1 T
+            t8::mma_chain<false, true>(tmem, tA1, 0, 0, tT, 0, 0, VW, KW, false);         // A1 T
             umma_commit(&barA);
             // L1^T R1 does not depend on Y: it runs on the tensor pipe while the threads turn A1 T into Y
             wait_or_flag(&ldB, ph, p.status, 14);
-            t8::mma_chain<true, true>(tmem + 128, tL1, 0, 0, tR1, 0, 0, 128, 64, false);   // L1^T R1
+            t8::mma_chain<true, true>(tmem + 128, tL1, 0, 0, tR1, 0, 0, VW, 64, false);    // L1^T R1
         }
         float part = 0.f;
         if (p.reverse && !p.no_store) {       // dgl = rowsum(dS (.) S_{n+1}), computed while the product runs
@@ -780,15 +806,17 @@ __global__ void __launch_bounds__(256) scan_tc_kernel(ScanTcP p) {
                 const float inv = 1.f / e_hs;
 #pragma unroll
                 for (int c8 = 0; c8 < 8; ++c8) {
+                    if (!FULL && !(row_in && c8 * 8 < HC)) continue;
                     float f[8];
                     t8::unpack8(hs[c8], f);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) part = fmaf(S[c8 * 8 + j], f[j] * inv, part);
                 }
             } else {
-                const float4* src = reinterpret_cast<const float4*>(p.HT + ((size_t)bh * K + row) * V + half * 64);
+                const float4* src = reinterpret_cast<const float4*>(p.HT + ((size_t)bh * K + row) * V + half * HC);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
+                    if (!FULL && !(row_in && 4 * j < HC)) continue;
                     const float4 x = src[j];
                     part = fmaf(S[4 * j], x.x, part); part = fmaf(S[4 * j + 1], x.y, part);
                     part = fmaf(S[4 * j + 2], x.z, part); part = fmaf(S[4 * j + 3], x.w, part);
@@ -802,10 +830,12 @@ __global__ void __launch_bounds__(256) scan_tc_kernel(ScanTcP p) {
         tc_fence_after();
         {
             float acc[64];
-            tmem_row64(t8::taddr(tmem, warp, half * 64), acc);
+            if (FULL || HC > 32) tmem_row64(t8::taddr(tmem, warp, half * HC), acc);
+            else tmem_row32(t8::taddr(tmem, warp, half * HC), acc);
 #pragma unroll
             for (int c8 = 0; c8 < 8; ++c8) {
-                const int cg = half * 8 + c8;
+                if (!FULL && c8 * 8 >= HC) continue;
+                const int cg = (half * HC >> 3) + c8;
                 float u[8];
                 t8::unpack8(sADD[cg * 128 + row], u);
 #pragma unroll
@@ -821,27 +851,29 @@ __global__ void __launch_bounds__(256) scan_tc_kernel(ScanTcP p) {
         if (p.reverse && !p.no_store && half == 0) p.dgl[(size_t)g * K + row] = part + red[row];
         if (tid == 0) {
             if (more) {                                // A1 and ADD buffers are free: prefetch the next chunk's
-                mbar_expect_tx(&ldA, 65536);
-                bulk_g2s(sA1, p.A1 + (g + dn) * CH128, 32768, &ldA);
-                bulk_g2s(sADD, p.ADD + (g + dn) * p.add_stride * CH128, 32768, &ldA);
+                mbar_expect_tx(&ldA, a_bytes + y_bytes);
+                bulk_g2s(sA1, p.A1 + (g + dn) * CH128, a_bytes, &ldA);
+                bulk_g2s(sADD, p.ADD + (g + dn) * p.add_stride * CH128, y_bytes, &ldA);
             }
             tc_fence_after();
-            t8::mma_chain<true, true>(tmem + 128, tL2, 0, 0, tY, 0, 0, 128, 128, true);    // + L2^T Y
+            t8::mma_chain<true, true>(tmem + 128, tL2, 0, 0, tY, 0, 0, VW, 128, true);     // + L2^T Y
             umma_commit(&barB);
         }
         wait_or_flag(&barB, ph, p.status, 15);
         tc_fence_after();
         if (tid == 0 && more) {
-            mbar_expect_tx(&ldB, 65536);
-            bulk_g2s(sL1, p.L1 + (g + dn) * p.r1_stride * CH64, 16384, &ldB);
-            bulk_g2s(sR1, p.R1 + (g + dn) * p.r1_stride * CH64, 16384, &ldB);
-            bulk_g2s(sL2, p.L2 + (g + dn) * CH128, 32768, &ldB);
+            mbar_expect_tx(&ldB, l_bytes + r_bytes + a_bytes);
+            bulk_g2s(sL1, p.L1 + (g + dn) * p.r1_stride * CH64, l_bytes, &ldB);
+            bulk_g2s(sR1, p.R1 + (g + dn) * p.r1_stride * CH64, r_bytes, &ldB);
+            bulk_g2s(sL2, p.L2 + (g + dn) * CH128, a_bytes, &ldB);
         }
         {
             float acc[64];
-            tmem_row64(t8::taddr(tmem, warp, 128 + half * 64), acc);
+            if (FULL || HC > 32) tmem_row64(t8::taddr(tmem, warp, 128 + half * HC), acc);
+            else tmem_row32(t8::taddr(tmem, warp, 128 + half * HC), acc);
 #pragma unroll
-            for (int j = 0; j < 64; ++j) S[j] = e * fmaf(e, S[j], acc[j]);
+            for (int j = 0; j < 64; ++j)
+                if (FULL || j < HC) S[j] = e * fmaf(e, S[j], acc[j]);
         }
         tc_fence_before();
     }
@@ -850,12 +882,13 @@ __global__ void __launch_bounds__(256) scan_tc_kernel(ScanTcP p) {
     if (!p.fin_last_only || ends_scan) {
         const size_t fs = p.fin_by_slot ? (size_t)slot : (size_t)bh;
         const int kd = p.fin_by_slot ? K : p.Kd, vd = p.fin_by_slot ? V : p.Vd;
-        const size_t off = (fs * kd + row) * vd + half * 64;
-        const size_t off2 = ((size_t)bh * K + row) * V + half * 64;
+        const size_t off = (fs * kd + row) * vd + half * HC;
+        const size_t off2 = ((size_t)bh * K + row) * V + half * HC;
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
+            if (!FULL && !(row_in && 4 * j < HC)) continue;
             const float4 x = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
-            if (p.fin && row < kd && half * 64 + 4 * j < vd) reinterpret_cast<float4*>(p.fin + off)[j] = x;
+            if (p.fin && row < kd && half * HC + 4 * j < vd) reinterpret_cast<float4*>(p.fin + off)[j] = x;
             if (p.fin2) reinterpret_cast<float4*>(p.fin2 + off2)[j] = x;
         }
     }
@@ -879,9 +912,12 @@ struct WyBwdP {
     const uint4 *M, *DV2, *Vc, *V2;
     uint4 *dP, *dAak, *dAab;
     int* status;
+    int VW;
 };
 
+template <bool FULL>
 __global__ void __launch_bounds__(128) wy_bwd_tc_kernel(WyBwdP p) {
+    const int VW = FULL ? V : p.VW;
     extern __shared__ __align__(1024) unsigned char smem[];
     uint4* bM = reinterpret_cast<uint4*>(smem);      // M, later dP
     uint4* bDV2 = bM + CH128;                        // dv2
@@ -894,12 +930,12 @@ __global__ void __launch_bounds__(128) wy_bwd_tc_kernel(WyBwdP p) {
     if (warp == 0) { tmem_alloc(&tmem_s, 256); tmem_relinquish(); }
     if (tid == 0) {
         mbar_init(&ld1, 1); mbar_init(&ld2, 1); mbar_init(&mma_bar, 1); fence_mbar_init();
-        mbar_expect_tx(&ld1, 65536);
+        mbar_expect_tx(&ld1, 32768 + 256 * VW);
         bulk_g2s(bM, p.M + g * CH128, 32768, &ld1);
-        bulk_g2s(bDV2, p.DV2 + g * CH128, 32768, &ld1);
-        mbar_expect_tx(&ld2, 49152);
-        bulk_g2s(bVc, p.Vc + g * CH64, 16384, &ld2);
-        bulk_g2s(bV2, p.V2 + g * CH128, 32768, &ld2);
+        bulk_g2s(bDV2, p.DV2 + g * CH128, 256 * VW, &ld1);
+        mbar_expect_tx(&ld2, 128 * VW + 256 * VW);
+        bulk_g2s(bVc, p.Vc + g * CH64, 128 * VW, &ld2);
+        bulk_g2s(bV2, p.V2 + g * CH128, 256 * VW, &ld2);
     }
     tc_fence_before();
     __syncthreads();
@@ -910,16 +946,17 @@ __global__ void __launch_bounds__(128) wy_bwd_tc_kernel(WyBwdP p) {
     float f[64];
     wait_or_flag(&ld1, 0, p.status, 30);
     if (tid == 0) {
-        t8::mma_chain<true, true>(tmem, tM, 0, 0, tDV2, 0, 0, 128, 128, false);          // dP = M^T dv2
+        t8::mma_chain<true, true>(tmem, tM, 0, 0, tDV2, 0, 0, VW, 128, false);           // dP = M^T dv2
         umma_commit(&mma_bar);
     }
     wait_or_flag(&mma_bar, 0, p.status, 31);
     tc_fence_after();
 #pragma unroll 1
-    for (int hh = 0; hh < 2; ++hh) {
+    for (int hh = 0; hh * 64 < VW; ++hh) {
         tmem_row64(t8::taddr(tmem, warp, hh * 64), f);
 #pragma unroll
         for (int c8 = 0; c8 < 8; ++c8) {
+            if (!FULL && (hh * 8 + c8) * 8 >= VW) continue;
             const uint4 c = t8::pack8(f + c8 * 8);
             bM[(hh * 8 + c8) * 128 + r] = c;                            // dP replaces M
             p.dP[g * CH128 + (hh * 8 + c8) * 128 + r] = c;
@@ -931,8 +968,8 @@ __global__ void __launch_bounds__(128) wy_bwd_tc_kernel(WyBwdP p) {
     wait_or_flag(&ld2, 0, p.status, 32);
     if (tid == 0) {
         tc_fence_after();
-        t8::mma_chain<false, false>(tmem, tM, 0, 0, tVc, 0, 0, 64, 128, false);          // dP v^T
-        t8::mma_chain<false, false>(tmem + 64, tM, 0, 0, tV2, 0, 0, 128, 128, false);    // dP v2^T
+        t8::mma_chain<false, false>(tmem, tM, 0, 0, tVc, 0, 0, 64, VW, false);           // dP v^T
+        t8::mma_chain<false, false>(tmem + 64, tM, 0, 0, tV2, 0, 0, 128, VW, false);     // dP v2^T
         umma_commit(&mma_bar);
     }
     wait_or_flag(&mma_bar, 1, p.status, 33);
@@ -971,11 +1008,13 @@ struct DauP {
     uint4 *dOc, *dAqk, *dAqb, *DV2;
     int T, H, NT;
     int* status;
-    int Vd;
+    int Vd, VW;
     const int2* chunk_tab;
 };
 
+template <bool FULL>
 __global__ void __launch_bounds__(128) dau_tc_kernel(DauP p) {
+    const int VW = FULL ? V : p.VW;
     extern __shared__ __align__(1024) unsigned char smem[];
     uint4* sdO = reinterpret_cast<uint4*>(smem);     // 16 KB [64 x 128]
     uint4* sAqb = sdO + CH64;                        // 16 KB [64 x 128]
@@ -988,10 +1027,10 @@ __global__ void __launch_bounds__(128) dau_tc_kernel(DauP p) {
     if (warp == 0) { tmem_alloc(&tmem_s, 256); tmem_relinquish(); }
     if (tid == 0) {
         mbar_init(&ld_bar, 1); mbar_init(&mma_bar, 1); fence_mbar_init();
-        mbar_expect_tx(&ld_bar, 65536);
+        mbar_expect_tx(&ld_bar, 16384 + 384 * VW);
         bulk_g2s(sAqb, p.Aqb + g * CH64, 16384, &ld_bar);
-        bulk_g2s(sVc, p.Vc + g * CH64, 16384, &ld_bar);
-        bulk_g2s(sV2, p.V2 + g * CH128, 32768, &ld_bar);
+        bulk_g2s(sVc, p.Vc + g * CH64, 128 * VW, &ld_bar);
+        bulk_g2s(sV2, p.V2 + g * CH128, 256 * VW, &ld_bar);
     }
     {
         const int bh = (int)(g / p.NT), n = (int)(g % p.NT);
@@ -1015,7 +1054,7 @@ __global__ void __launch_bounds__(128) dau_tc_kernel(DauP p) {
             const int r = (blk >> 2) * 8 + (lane & 7);
             const int kc = (blk & 3) * 4 + (lane >> 3);
             sdO[kc * 64 + r] = c[it];
-            p.dOc[g * CH64 + kc * 64 + r] = c[it];
+            if (FULL || kc * 8 < VW) p.dOc[g * CH64 + kc * 64 + r] = c[it];
         }
     }
     fence_proxy_async();
@@ -1026,8 +1065,8 @@ __global__ void __launch_bounds__(128) dau_tc_kernel(DauP p) {
     const Tile tdO = t8::tile(sdO, 64), tAqb = t8::tile(sAqb, 64), tVc = t8::tile(sVc, 64), tV2 = t8::tile(sV2, 128);
     wait_or_flag(&ld_bar, 0, p.status, 50);
     if (tid == 0) {
-        t8::mma_chain<false, false>(tmem, tdO, 0, 0, tV2, 0, 0, 128, 128, false);        // dO v2^T
-        t8::mma_chain<true, true>(tmem + 128, tAqb, 0, 0, tdO, 0, 0, 128, 64, false);    // Aqb^T dO
+        t8::mma_chain<false, false>(tmem, tdO, 0, 0, tV2, 0, 0, 128, VW, false);         // dO v2^T
+        t8::mma_chain<true, true>(tmem + 128, tAqb, 0, 0, tdO, 0, 0, VW, 64, false);     // Aqb^T dO
         umma_commit(&mma_bar);
     }
     wait_or_flag(&mma_bar, 0, p.status, 51);
@@ -1044,15 +1083,16 @@ __global__ void __launch_bounds__(128) dau_tc_kernel(DauP p) {
                 p.dAqb[g * CH64 + (hh * 8 + c8) * 64 + tid] = t8::pack8(f + c8 * 8);
             }
         }
+        if (!FULL && hh * 64 >= VW) continue;
         tmem_row64(t8::taddr(tmem, warp, 128 + hh * 64), f);
 #pragma unroll
-        for (int c8 = 0; c8 < 8; ++c8) p.DV2[g * CH128 + (hh * 8 + c8) * 128 + tid] = t8::pack8(f + c8 * 8);
+        for (int c8 = 0; c8 < 8; ++c8) if (FULL || (hh * 8 + c8) * 8 < VW) p.DV2[g * CH128 + (hh * 8 + c8) * 128 + tid] = t8::pack8(f + c8 * 8);
     }
     tc_fence_before();
     __syncthreads();
     if (tid == 0) {
         tc_fence_after();
-        t8::mma_chain<false, false>(tmem, tdO, 0, 0, tVc, 0, 0, 64, 128, false);         // dO v^T
+        t8::mma_chain<false, false>(tmem, tdO, 0, 0, tVc, 0, 0, 64, VW, false);          // dO v^T
         umma_commit(&mma_bar);
     }
     wait_or_flag(&mma_bar, 1, p.status, 52);
@@ -1079,11 +1119,13 @@ struct OutP {
     __nv_bfloat16* o;
     int T, H, NT;
     int* status;
-    int Vd;
+    int Vd, KW, VW;
     const int2* chunk_tab;
 };
 
+template <bool FULL>
 __global__ void __launch_bounds__(128) out_tc_kernel(OutP p) {
+    const int KW = FULL ? K : p.KW, VW = FULL ? V : p.VW;
     extern __shared__ __align__(1024) unsigned char smem[];
     // 72 KB, three CTAs per SM: the operands of the last product (Aqb, v2) take the place of the first
     // product's (Qh, St) once that has completed; the other CTAs on the SM cover the extra round trip.
@@ -1098,11 +1140,11 @@ __global__ void __launch_bounds__(128) out_tc_kernel(OutP p) {
     if (warp == 0) { tmem_alloc(&tmem_s, 128); tmem_relinquish(); }
     if (tid == 0) {
         mbar_init(&ld_bar, 1); mbar_init(&ld2_bar, 1); mbar_init(&mma_bar, 1); mbar_init(&mma2_bar, 1); fence_mbar_init();
-        mbar_expect_tx(&ld_bar, 16384 + 32768 + 8192 + 16384);
-        bulk_g2s(sQ, p.Qh + g * CH64, 16384, &ld_bar);
-        bulk_g2s(sH, p.Hs + g * CH128, 32768, &ld_bar);
+        mbar_expect_tx(&ld_bar, 128 * KW + 2 * KW * VW + 8192 + 128 * VW);
+        bulk_g2s(sQ, p.Qh + g * CH64, 128 * KW, &ld_bar);
+        bulk_g2s(sH, p.Hs + g * CH128, 2 * KW * VW, &ld_bar);
         bulk_g2s(sAqk, p.Aqk + g * 512, 8192, &ld_bar);
-        bulk_g2s(sV, p.Vc + g * CH64, 16384, &ld_bar);
+        bulk_g2s(sV, p.Vc + g * CH64, 128 * VW, &ld_bar);
     }
     tc_fence_before();
     __syncthreads();
@@ -1111,16 +1153,16 @@ __global__ void __launch_bounds__(128) out_tc_kernel(OutP p) {
     if (tid == 0) {
         // the three A operands have 64 rows; lanes 64..127 of the accumulator are never read
         wait_or_flag(&ld_bar, 0, p.status, 16);
-        t8::mma_chain<false, true>(tmem, t8::tile(sQ, 64), 0, 0, t8::tile(sH, 128), 0, 0, 128, 128, false);
-        t8::mma_chain<false, true>(tmem, t8::tile(sAqk, 64), 0, 0, t8::tile(sV, 64), 0, 0, 128, 64, true);
+        t8::mma_chain<false, true>(tmem, t8::tile(sQ, 64), 0, 0, t8::tile(sH, KW), 0, 0, VW, KW, false);
+        t8::mma_chain<false, true>(tmem, t8::tile(sAqk, 64), 0, 0, t8::tile(sV, 64), 0, 0, VW, 64, true);
         umma_commit(&mma_bar);
         wait_or_flag(&mma_bar, 0, p.status, 17);
-        mbar_expect_tx(&ld2_bar, 16384 + 32768);
+        mbar_expect_tx(&ld2_bar, 16384 + 256 * VW);
         bulk_g2s(sQ, p.Aqb + g * CH64, 16384, &ld2_bar);
-        bulk_g2s(sH, p.V2 + g * CH128, 32768, &ld2_bar);
+        bulk_g2s(sH, p.V2 + g * CH128, 256 * VW, &ld2_bar);
         wait_or_flag(&ld2_bar, 0, p.status, 18);
         tc_fence_after();
-        t8::mma_chain<false, true>(tmem, t8::tile(sQ, 64), 0, 0, t8::tile(sH, 128), 0, 0, 128, 128, true);
+        t8::mma_chain<false, true>(tmem, t8::tile(sQ, 64), 0, 0, t8::tile(sH, 128), 0, 0, VW, 128, true);
         umma_commit(&mma2_bar);
     }
     if (warp < 2) wait_idle_or_flag(&mma2_bar, 0, p.status, 19);
@@ -1133,7 +1175,7 @@ __global__ void __launch_bounds__(128) out_tc_kernel(OutP p) {
         const int t = t0 + tid;
         uint4* dst = reinterpret_cast<uint4*>(p.o + (((size_t)b * p.T + t) * p.H + h) * p.Vd);
 #pragma unroll 1
-        for (int hh = 0; hh < 2; ++hh) {
+        for (int hh = 0; hh * 64 < VW; ++hh) {
             float f[64];
             tmem_row64(t8::taddr(tmem, warp, hh * 64), f);
             if (tid < valid) {
@@ -1160,13 +1202,15 @@ __global__ void __launch_bounds__(128) out_tc_kernel(OutP p) {
 }
 
 // debugging aid: C8 bf16 tile -> fp32 row-major
-__global__ void c8_to_rowmajor_kernel(const uint4* src, float* dst, int rows, int cols) {
+// (tiles of narrow heads hold w_rows x w_cols elements of it, the rest is written as zero)
+__global__ void c8_to_rowmajor_kernel(const uint4* src, float* dst, int rows, int cols, int w_rows, int w_cols) {
     const long long g = blockIdx.x;
     const int nch = rows * cols / 8;
     for (int e = threadIdx.x; e < nch; e += blockDim.x) {
         const int cg = e / rows, r = e % rows;
         float f[8];
-        t8::unpack8(src[g * nch + e], f);
+        const bool kept = r < w_rows && cg * 8 < w_cols;
+        t8::unpack8(kept ? src[g * nch + cg * w_rows + r] : make_uint4(0, 0, 0, 0), f);
         for (int j = 0; j < 8; ++j) dst[(size_t)g * rows * cols + (size_t)r * cols + cg * 8 + j] = f[j];
     }
 }
@@ -1224,6 +1268,7 @@ struct GradP {
     int* status;
     long long G;           // number of tiles; the grid is persistent
     int Kd, Vd;            // head dims of the public tensors (channels beyond them are padding and are not written)
+    int KW, VW;
     const int2* chunk_tab;
 };
 
@@ -1232,7 +1277,10 @@ __device__ __forceinline__ void chain0(uint32_t tm, Tile A, Tile B, int N, int k
     t8::mma_chain<A_MN, B_MN>(tm, A, 0, 0, B, 0, 0, N, kdim, acc);
 }
 
+template <bool FULL>
 __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
+    const int KW = FULL ? K : p.KW, VW = FULL ? V : p.VW;
+    const uint32_t k64 = 128 * KW, k128 = 256 * KW, v64 = 128 * VW, v128 = 256 * VW, kv = 2 * KW * VW;     // tile bytes
     extern __shared__ __align__(1024) unsigned char smem[];
     uint4* sA = reinterpret_cast<uint4*>(smem);          // 32 KB slots
     uint4* sB = sA + CH128;
@@ -1266,18 +1314,18 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
     // TMEM columns: dQh^T 0..63, dv^T 64..127, dAh^T 128..255, dBh^T 256..383, dKh^T 384..447
     // tiles whose slots the epilogue of the tile before does not read
     auto load_ahead = [&](long long g) {
-        mbar_expect_tx(&ld[T_dP], 32768);
-        bulk_g2s(sD, p.dP + g * CH128, 32768, &ld[T_dP]);
-        mbar_expect_tx(&ld[T_StdO], 32768 + 16384);
-        bulk_g2s(sA, p.Hs + g * CH128, 32768, &ld[T_StdO]);
-        bulk_g2s(sa, p.dOc + g * CH64, 16384, &ld[T_StdO]);
+        mbar_expect_tx(&ld[T_dP], v128);
+        bulk_g2s(sD, p.dP + g * CH128, v128, &ld[T_dP]);
+        mbar_expect_tx(&ld[T_StdO], kv + v64);
+        bulk_g2s(sA, p.Hs + g * CH128, kv, &ld[T_StdO]);
+        bulk_g2s(sa, p.dOc + g * CH64, v64, &ld[T_StdO]);
         mbar_expect_tx(&ld[T_Aqk], 8192);
         bulk_g2s(sy, p.Aqk + g * 512, 8192, &ld[T_Aqk]);
         mbar_expect_tx(&ld[T_dAq], 8192 + 16384);
         bulk_g2s(sx, p.dAqk + g * 512, 8192, &ld[T_dAq]);
         bulk_g2s(sc, p.dAqb + g * CH64, 16384, &ld[T_dAq]);
-        mbar_expect_tx(&ld[T_dSt], 32768);
-        bulk_g2s(sC, p.DE + g * CH128, 32768, &ld[T_dSt]);
+        mbar_expect_tx(&ld[T_dSt], kv);
+        bulk_g2s(sC, p.DE + g * CH128, kv, &ld[T_dSt]);
     };
     if (producer && (long long)blockIdx.x < p.G) load_ahead(blockIdx.x);
     uint32_t it = 0;
@@ -1288,19 +1336,19 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
         TL(0);
         mbar_expect_tx(&ld[T_Aak], 16384);
         bulk_g2s(sE, p.Aak + g * CH64, 16384, &ld[T_Aak]);
-        mbar_expect_tx(&ld[T_Kh], 16384);
-        bulk_g2s(sb, p.Kh + g * CH64, 16384, &ld[T_Kh]);
-        mbar_expect_tx(&ld[T_Bh], 32768);
-        bulk_g2s(sB, p.Bh + g * CH128, 32768, &ld[T_Bh]);
-        mbar_expect_tx(&ld[T_Vc], 16384);
-        bulk_g2s(sE + CH64, p.Vc + g * CH64, 16384, &ld[T_Vc]);
+        mbar_expect_tx(&ld[T_Kh], k64);
+        bulk_g2s(sb, p.Kh + g * CH64, k64, &ld[T_Kh]);
+        mbar_expect_tx(&ld[T_Bh], k128);
+        bulk_g2s(sB, p.Bh + g * CH128, k128, &ld[T_Bh]);
+        mbar_expect_tx(&ld[T_Vc], v64);
+        bulk_g2s(sE + CH64, p.Vc + g * CH64, v64, &ld[T_Vc]);
         // Chains are issued as soon as their own tiles have landed, and the chains that read a slot for the last
         // time are issued first and committed on their own, so that the slot is refilled while the rest of the
         // product still runs.
         wait_or_flag(&ld[T_StdO], ph, p.status, 70);
-        chain0<false, false>(tmem, t8::tile(sA, 128), t8::tile(sa, 64), 64, 128, false);          // P1: St dO^T
+        chain0<false, false>(tmem, t8::tile(sA, KW), t8::tile(sa, 64), 64, VW, false);            // P1: St dO^T
         wait_or_flag(&ld[T_dP], ph, p.status, 72);
-        chain0<false, false>(tmem + 128, t8::tile(sA, 128), t8::tile(sD, 128), 128, 128, false);  // P3: St dP^T
+        chain0<false, false>(tmem + 128, t8::tile(sA, KW), t8::tile(sD, 128), 128, VW, false);    // P3: St dP^T
         umma_commit(&mc1);                                                                        // slot A free
         wait_or_flag(&ld[T_Aqk], ph, p.status, 71);
         chain0<true, true>(tmem + 64, t8::tile(sa, 64), t8::tile(sy, 64), 64, 64, false);         // P2: dO^T Aqk
@@ -1309,16 +1357,16 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
         chain0<true, true>(tmem + 64, t8::tile(sD, 128), t8::tile(sE, 128), 64, 128, true);       // P2: dP^T Aak
         umma_commit(&mc6);                                                                        // slots D, E.lo free
         wait_or_flag(&mc1, ph, p.status, 74);
-        mbar_expect_tx(&ld[T_V2], 32768);
-        bulk_g2s(sA, p.V2 + g * CH128, 32768, &ld[T_V2]);
+        mbar_expect_tx(&ld[T_V2], v128);
+        bulk_g2s(sA, p.V2 + g * CH128, v128, &ld[T_V2]);
         wait_or_flag(&mc5, ph, p.status, 75);
-        mbar_expect_tx(&ld[T_dAakAh], 16384 + 32768);          // (Ah follows when slot B is free)
+        mbar_expect_tx(&ld[T_dAakAh], 16384 + k128);          // (Ah follows when slot B is free)
         bulk_g2s(sa, p.dAak + g * CH64, 16384, &ld[T_dAakAh]);
         wait_or_flag(&mc6, ph, p.status, 76);
         mbar_expect_tx(&ld[T_dAab], 32768);
         bulk_g2s(sD, p.dAab + g * CH128, 32768, &ld[T_dAab]);
-        mbar_expect_tx(&ld[T_Qh], 16384);
-        bulk_g2s(sE, p.Qh + g * CH64, 16384, &ld[T_Qh]);
+        mbar_expect_tx(&ld[T_Qh], k64);
+        bulk_g2s(sE, p.Qh + g * CH64, k64, &ld[T_Qh]);
         wait_or_flag(&ld[T_Kh], ph, p.status, 77);
         wait_or_flag(&ld[T_dAq], ph, p.status, 78);
         chain0<true, false>(tmem, t8::tile(sb, 64), t8::tile(sx, 64), 64, 64, true);              // P1: Kh^T dAqk^T
@@ -1326,22 +1374,22 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
         chain0<true, false>(tmem, t8::tile(sB, 128), t8::tile(sc, 64), 64, 128, true);            // P1: Bh^T dAqb^T
         umma_commit(&m1);
         wait_or_flag(&ld[T_dSt], ph, p.status, 80);
-        chain0<true, false>(tmem + 64, t8::tile(sC, 128), t8::tile(sb, 64), 64, 128, true);       // P2: dSt^T Kh^T
+        chain0<true, false>(tmem + 64, t8::tile(sC, KW), t8::tile(sb, 64), 64, KW, true);         // P2: dSt^T Kh^T
         umma_commit(&m2);
         TL(4);
         wait_or_flag(&ld[T_Vc], ph, p.status, 81);
-        chain0<false, false>(tmem + 384, t8::tile(sC, 128), t8::tile(sE + CH64, 64), 64, 128, false);  // P5: dSt v^T
+        chain0<false, false>(tmem + 384, t8::tile(sC, KW), t8::tile(sE + CH64, 64), 64, VW, false);    // P5: dSt v^T
         wait_or_flag(&ld[T_dAab], ph, p.status, 82);
         chain0<true, false>(tmem + 128, t8::tile(sB, 128), t8::tile(sD, 128), 128, 128, true);    // P3: Bh^T dAab^T
         umma_commit(&mc9);                                                                        // slot B free
         wait_or_flag(&ld[T_V2], ph, p.status, 83);
-        chain0<false, false>(tmem + 256, t8::tile(sC, 128), t8::tile(sA, 128), 128, 128, false);  // P4: dSt V2^T
+        chain0<false, false>(tmem + 256, t8::tile(sC, KW), t8::tile(sA, 128), 128, VW, false);    // P4: dSt V2^T
         wait_or_flag(&ld[T_Qh], ph, p.status, 84);
         chain0<true, true>(tmem + 256, t8::tile(sE, 64), t8::tile(sc, 64), 128, 64, true);        // P4: Qh^T dAqb
         chain0<true, true>(tmem + 384, t8::tile(sE, 64), t8::tile(sx, 64), 64, 64, true);         // P5: Qh^T dAqk
         wait_or_flag(&mc9, ph, p.status, 85);
         TL(6);
-        bulk_g2s(sB, p.Ah + g * CH128, 32768, &ld[T_dAakAh]);
+        bulk_g2s(sB, p.Ah + g * CH128, k128, &ld[T_dAakAh]);
         wait_or_flag(&ld[T_dAakAh], ph, p.status, 86);
         chain0<true, false>(tmem + 128, t8::tile(sb, 64), t8::tile(sa, 128), 128, 64, true);      // P3: Kh^T dAak^T
         umma_commit(&m3);
@@ -1377,7 +1425,7 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
             const float e_half = __ldg(p.E + (size_t)g * K + k);
 #pragma unroll
             for (int j = 0; j < 17; ++j)
-                eg[j] = (i_lo + j - 1 >= 0) ? __uint_as_float((uint32_t)__ldg(egp + (size_t)(i_lo + j - 1) * K) << 16) : 0.f;
+                eg[j] = (i_lo + j - 1 >= 0 && k_ok) ? __uint_as_float((uint32_t)__ldg(egp + (size_t)(i_lo + j - 1) * K) << 16) : 0.f;
             if (i_lo == 0) eg[0] = __frcp_rn(e_half);        // e^{ge - half} of the chunk's first token
         }
         const float dgl = __ldg(p.dgl + (size_t)g * K + k);
@@ -1426,6 +1474,7 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
             const unsigned short* bg = reinterpret_cast<const unsigned short*>(p.Bh + g * CH128 + (k >> 3) * 128) + (k & 7);
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
+                if (!FULL && !k_ok) { bhp[j] = 0; continue; }
                 const uint32_t lo = __ldg(bg + (size_t)(2 * (i_lo + j)) * 8), hi = __ldg(bg + (size_t)(2 * (i_lo + j) + 1) * 8);
                 bhp[j] = lo | (hi << 16);
             }
@@ -1518,7 +1567,7 @@ __global__ void __launch_bounds__(256) compose_segments_kernel(const float* T, c
                                                                int s0_identity, int lead_final, long long bh_stride,
                                                                long long seg_stride, long long t_bh_stride,
                                                                long long t_seg_stride, const float* pre,
-                                                               const float* post) {
+                                                               const float* post, int kw) {
     constexpr int CB = kComposeCols, CT = 8;                                     // columns per CTA / per thread
     extern __shared__ __align__(16) float csm[];
     float (*sT)[129] = reinterpret_cast<float (*)[129]>(csm);                    // sT[j][k] = factor of cur[j] in row k
@@ -1581,7 +1630,7 @@ __global__ void __launch_bounds__(256) compose_segments_kernel(const float* T, c
         __syncthreads();
         if (apply) {
 #pragma unroll 4
-            for (int j = 0; j < K; ++j) {
+            for (int j = 0; j < kw; ++j) {                  // (nothing beyond the tile's width is written by the scans)
                 const float t = sT[j][k];
                 const float4 v0 = *reinterpret_cast<const float4*>(&cur[j][ch * CT]);        // the same address for a
                 const float4 v1 = *reinterpret_cast<const float4*>(&cur[j][ch * CT + 4]);    // whole warp: a broadcast
@@ -1654,7 +1703,7 @@ int tc_compose_states(const float* T, const float* F, const float* S0, const flo
         attr_dev = dev;
     }
     launch(compose_segments_kernel, dim3(dim3(BH, V / kComposeCols)), dim3(256), kComposeSmem, st, T, F, S0, nullptr, out, count, reverse,
-                                                                                 0, 0, 1, f_stride, 1, t_stride, pre, post);
+                                                                                 0, 0, 1, f_stride, 1, t_stride, pre, post, K);
     HDLA_CHECK_LAUNCH("compose_segments_kernel");
     return HDLA_OK;
 }
@@ -1689,20 +1738,28 @@ int tc_chunk_fwd(const HdlaDims& d, const void* q, const void* k, const void* v,
     // a workspace sized for the backward pass also receives what only the backward kernels read
     const bool save_bwd = ws_bytes >= pl.total;
     const bool param_ab = (d.flags & HDLA_FLAG_PARAM_AB) != 0;
+    const bool full = pl.KW == K && pl.VW == V;              // tiles of the full width: the kernels' extents are constants
     // the one-kernel form needs full head dims and reads a and b as tensors
     const bool unfused = !(d.flags & HDLA_FLAG_FUSED_PREP) || d.K != K || d.V != V || param_ab;
     static thread_local int attr_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_dev != dev) {
-        TRY(set_smem(gram_tc_kernel, 98304 + 1024));
+        TRY(set_smem(gram_tc_kernel<true>, 98304 + 1024));
+        TRY(set_smem(gram_tc_kernel<false>, 98304 + 1024));
         TRY(set_smem(inverse_tc_kernel, 32768));
-        TRY(set_smem(wu_tc_kernel, 98304));
-        TRY(set_smem(scan_tc_kernel, 196608));
-        TRY(set_smem(out_tc_kernel, 73728));
-        TRY(set_smem(wy_bwd_tc_kernel, kWySmem));
-        TRY(set_smem(grad_tc_kernel, kGradSmem));
-        TRY(set_smem(dau_tc_kernel, 81920));
+        TRY(set_smem(wu_tc_kernel<true>, 98304));
+        TRY(set_smem(wu_tc_kernel<false>, 98304));
+        TRY(set_smem(scan_tc_kernel<true>, 196608));
+        TRY(set_smem(scan_tc_kernel<false>, 196608));
+        TRY(set_smem(out_tc_kernel<true>, 73728));
+        TRY(set_smem(out_tc_kernel<false>, 73728));
+        TRY(set_smem(wy_bwd_tc_kernel<true>, kWySmem));
+        TRY(set_smem(wy_bwd_tc_kernel<false>, kWySmem));
+        TRY(set_smem(grad_tc_kernel<true>, kGradSmem));
+        TRY(set_smem(grad_tc_kernel<false>, kGradSmem));
+        TRY(set_smem(dau_tc_kernel<true>, 81920));
+        TRY(set_smem(dau_tc_kernel<false>, 81920));
         TRY(set_smem(compose_segments_kernel, kComposeSmem));
         attr_dev = dev;
     }
@@ -1737,19 +1794,19 @@ int tc_chunk_fwd(const HdlaDims& d, const void* q, const void* k, const void* v,
             TRY(tc_launch_chunk_prep(pl, d, q, k, v, a, b, gk, scale, ws, save_bwd, st));
         } else {
             PrepP pp{(bp)q, (bp)k, (bp)v, (bp)a, (bp)b, gk, U4(pl.Qh), U4(pl.Kh), U4(pl.Ah), U4(pl.Bh), U4(pl.Vc),
-                     F(pl.E), (__nv_bfloat16*)(ws + pl.ghat), scale, d.T, d.H, pl.NT, d.gk_dtype, status, d.K, d.V, chunk_tab,
+                     F(pl.E), (__nv_bfloat16*)(ws + pl.ghat), scale, d.T, d.H, pl.NT, d.gk_dtype, status, d.K, d.V, chunk_tab, pl.KW, pl.VW,
                      param_ab ? (bp)a : nullptr, (d.flags & HDLA_FLAG_NORM_K) ? 1 : 0};
-            if (param_ab) launch(prep_hat_kernel<true>, dim3(G), dim3(128), 0, st, pp);
-            else launch(prep_hat_kernel<false>, dim3(G), dim3(128), 0, st, pp);
+            if (param_ab) launch(full ? prep_hat_kernel<true, true> : prep_hat_kernel<true, false>, dim3(G), dim3(128), 0, st, pp);
+            else launch(full ? prep_hat_kernel<false, true> : prep_hat_kernel<false, false>, dim3(G), dim3(128), 0, st, pp);
             HDLA_CHECK_LAUNCH("prep_hat_kernel");
-            GramP gp{U4(pl.Qh), U4(pl.Kh), U4(pl.Ah), U4(pl.Bh), U4(pl.Aqk), U4(pl.Aqb), U4(pl.Aak), U4(pl.Aab), status};
-            launch(gram_tc_kernel, dim3(G), dim3(128), 98304 + 1024, st, gp);
+            GramP gp{U4(pl.Qh), U4(pl.Kh), U4(pl.Ah), U4(pl.Bh), U4(pl.Aqk), U4(pl.Aqb), U4(pl.Aak), U4(pl.Aab), status, pl.KW};
+            launch(full ? gram_tc_kernel<true> : gram_tc_kernel<false>, dim3(G), dim3(128), 98304 + 1024, st, gp);
             HDLA_CHECK_LAUNCH("gram_tc_kernel");
             InvP ivp{U4(pl.Aab), U4(pl.M), status};
             launch(inverse_tc_kernel, dim3(G), dim3(128), 32768, st, ivp);
             HDLA_CHECK_LAUNCH("inverse_tc_kernel");
-            WuP wp{U4(pl.M), U4(pl.Ah), U4(pl.Aak), U4(pl.Vc), U4(pl.U), U4(pl.W), status};
-            launch(wu_tc_kernel, dim3(G), dim3(128), 98304, st, wp);
+            WuP wp{U4(pl.M), U4(pl.Ah), U4(pl.Aak), U4(pl.Vc), U4(pl.U), U4(pl.W), status, pl.KW, pl.VW};
+            launch(full ? wu_tc_kernel<true> : wu_tc_kernel<false>, dim3(G), dim3(128), 98304, st, wp);
             HDLA_CHECK_LAUNCH("wu_tc_kernel");
         }
         if (phase == HDLA_PHASE_PRE) return HDLA_OK;
@@ -1760,7 +1817,7 @@ int tc_chunk_fwd(const HdlaDims& d, const void* q, const void* k, const void* v,
         sp.init = init; sp.CK = ck; sp.Y = y; sp.fin = fin; sp.fin2 = fin2;
         sp.NT = pl.NT; sp.reverse = 0; sp.status = status; sp.add_stride = 1; sp.r1_stride = 1; sp.no_store = no_store;
         sp.nseg = 1; sp.seg_len = pl.NT; sp.zero_tile = U4(pl.zero);
-        sp.Kd = d.K; sp.Vd = d.V; sp.seq_tab = seq_tab; sp.H = d.H;
+        sp.Kd = d.K; sp.Vd = d.V; sp.KW = pl.KW; sp.VW = pl.VW; sp.seq_tab = seq_tab; sp.H = d.H;
         return sp;
     };
     if (phase == HDLA_PHASE_TRANSITION) {
@@ -1772,17 +1829,17 @@ int tc_chunk_fwd(const HdlaDims& d, const void* q, const void* k, const void* v,
             // both stay in the workspace for the STATE and POST phases of this sequence slice
             ScanTcP s1 = scan_params(nullptr, nullptr, nullptr, F(pl.Fseg), nullptr, 1);
             s1.nseg = pl.nseg; s1.seg_len = pl.seg_len; s1.fin_by_slot = 1; s1.fin_transition = F(pl.Tseg);
-            launch(scan_tc_kernel, dim3(dim3(pl.BH * pl.nseg, 2)), dim3(256), 196608, st, s1);
+            launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(dim3(pl.BH * pl.nseg, 2)), dim3(256), 196608, st, s1);
             HDLA_CHECK_LAUNCH("scan_tc_kernel");
             launch(compose_segments_kernel, dim3(dim3(pl.BH, V / kComposeCols)), dim3(256), kComposeSmem, st, F(pl.Tseg), F(pl.Fseg), nullptr, nullptr, ht,
-                                                                         pl.nseg, 0, 1, 0, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr);
+                                                                         pl.nseg, 0, 1, 0, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr, pl.KW);
             HDLA_CHECK_LAUNCH("compose_segments_kernel");
             return HDLA_OK;
         }
         ScanTcP sp = scan_params(nullptr, nullptr, nullptr, ht, nullptr, 1);
         sp.ADD = U4(pl.zero); sp.R1 = U4(pl.zero); sp.L1 = U4(pl.zero); sp.add_stride = 0; sp.r1_stride = 0;
         sp.init_identity = 1;
-        launch(scan_tc_kernel, dim3(pl.BH), dim3(256), 196608, st, sp);
+        launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(pl.BH), dim3(256), 196608, st, sp);
         HDLA_CHECK_LAUNCH("scan_tc_kernel");
         return HDLA_OK;
     }
@@ -1790,12 +1847,12 @@ int tc_chunk_fwd(const HdlaDims& d, const void* q, const void* k, const void* v,
         if (!ht) return fail(HDLA_ERR_INVALID, "state pass needs the output pointer (ht)");
         if (pl.nseg > 1) {                    // affine maps of the segments are in the workspace (TRANSITION phase)
             launch(compose_segments_kernel, dim3(dim3(pl.BH, V / kComposeCols)), dim3(256), kComposeSmem, st, F(pl.Tseg), F(pl.Fseg), h0, nullptr, ht,
-                                                                         pl.nseg, 0, 0, 0, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr);
+                                                                         pl.nseg, 0, 0, 0, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr, pl.KW);
             HDLA_CHECK_LAUNCH("compose_segments_kernel");
             return HDLA_OK;
         }
         ScanTcP sp = scan_params(h0, nullptr, nullptr, ht, nullptr, 1);
-        launch(scan_tc_kernel, dim3(pl.BH), dim3(256), 196608, st, sp);
+        launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(pl.BH), dim3(256), 196608, st, sp);
         HDLA_CHECK_LAUNCH("scan_tc_kernel");
         return HDLA_OK;
     }
@@ -1805,43 +1862,43 @@ int tc_chunk_fwd(const HdlaDims& d, const void* q, const void* k, const void* v,
         ScanTcP s1 = scan_params(nullptr, U4(pl.Hs), U4(pl.V2), F(pl.Fseg), nullptr, 1);
         s1.nseg = pl.nseg; s1.seg_len = pl.seg_len; s1.fin_by_slot = 1; s1.fin_transition = F(pl.Tseg);
         s1.seg_off = 0; s1.seg_cnt = pl.nseg - 1; s1.lead_real = 1; s1.lead_init = h0;
-        launch(scan_tc_kernel, dim3(dim3(pl.BH * (pl.nseg - 1), 2)), dim3(256), 196608, st, s1);
+        launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(dim3(pl.BH * (pl.nseg - 1), 2)), dim3(256), 196608, st, s1);
         HDLA_CHECK_LAUNCH("scan_tc_kernel");
         // ... the state entering every later segment follows from the first segment's final state ...
         launch(compose_segments_kernel, dim3(dim3(pl.BH, V / kComposeCols)), dim3(256), kComposeSmem, st, F(pl.Tseg), F(pl.Fseg), nullptr, F(pl.Sin), nullptr,
-                                                                     pl.nseg, 0, 0, 1, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr);
+                                                                     pl.nseg, 0, 0, 1, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr, pl.KW);
         HDLA_CHECK_LAUNCH("compose_segments_kernel");
         // ... and the remaining segments are scanned for real at once
         ScanTcP s2 = scan_params(F(pl.Sin), U4(pl.Hs), U4(pl.V2), ht, F(pl.HT), 0);
         s2.nseg = pl.nseg; s2.seg_len = pl.seg_len; s2.init_by_slot = 1; s2.fin_last_only = 1;
         s2.seg_off = 1; s2.seg_cnt = pl.nseg - 1;
-        launch(scan_tc_kernel, dim3(pl.BH * (pl.nseg - 1)), dim3(256), 196608, st, s2);
+        launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(pl.BH * (pl.nseg - 1)), dim3(256), 196608, st, s2);
         HDLA_CHECK_LAUNCH("scan_tc_kernel");
     } else     if (pl.nseg > 1) {
         // two-level scan: per segment, transition and state-from-zero side by side (grid.y = 2) ...
         if (phase == HDLA_PHASE_ALL) {        // (a phased POST call finds them in the workspace)
             ScanTcP s1 = scan_params(nullptr, nullptr, nullptr, F(pl.Fseg), nullptr, 1);
             s1.nseg = pl.nseg; s1.seg_len = pl.seg_len; s1.fin_by_slot = 1; s1.fin_transition = F(pl.Tseg);
-            launch(scan_tc_kernel, dim3(dim3(pl.BH * pl.nseg, 2)), dim3(256), 196608, st, s1);
+            launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(dim3(pl.BH * pl.nseg, 2)), dim3(256), 196608, st, s1);
             HDLA_CHECK_LAUNCH("scan_tc_kernel");
         }
         // ... composed into the state entering every segment ...
-        launch(compose_segments_kernel, dim3(dim3(pl.BH, V / kComposeCols)), dim3(256), kComposeSmem, st, F(pl.Tseg), F(pl.Fseg), h0, F(pl.Sin), nullptr, pl.nseg, 0, 0, 0, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr);
+        launch(compose_segments_kernel, dim3(dim3(pl.BH, V / kComposeCols)), dim3(256), kComposeSmem, st, F(pl.Tseg), F(pl.Fseg), h0, F(pl.Sin), nullptr, pl.nseg, 0, 0, 0, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr, pl.KW);
         HDLA_CHECK_LAUNCH("compose_segments_kernel");
         // ... and the real scan of all segments at once
         ScanTcP s2 = scan_params(F(pl.Sin), U4(pl.Hs), U4(pl.V2), ht, F(pl.HT), 0);
         s2.nseg = pl.nseg; s2.seg_len = pl.seg_len; s2.init_by_slot = 1; s2.fin_last_only = 1;
-        launch(scan_tc_kernel, dim3(pl.BH * pl.nseg), dim3(256), 196608, st, s2);
+        launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(pl.BH * pl.nseg), dim3(256), 196608, st, s2);
         HDLA_CHECK_LAUNCH("scan_tc_kernel");
     } else {
         ScanTcP sp = scan_params(h0, U4(pl.Hs), U4(pl.V2), ht, F(pl.HT), 0);
-        launch(scan_tc_kernel, dim3(pl.BH), dim3(256), 196608, st, sp);
+        launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(pl.BH), dim3(256), 196608, st, sp);
         HDLA_CHECK_LAUNCH("scan_tc_kernel");
     }
     if (need_o) {
         OutP op{U4(pl.Qh), U4(pl.Aqk), U4(pl.Aqb), U4(pl.Vc), U4(pl.Hs), U4(pl.V2), (__nv_bfloat16*)o, d.T, d.H,
-                pl.NT, status, d.V, chunk_tab};
-        launch(out_tc_kernel, dim3(G), dim3(128), 73728, st, op);
+                pl.NT, status, d.V, pl.KW, pl.VW, chunk_tab};
+        launch(full ? out_tc_kernel<true> : out_tc_kernel<false>, dim3(G), dim3(128), 73728, st, op);
         HDLA_CHECK_LAUNCH("out_tc_kernel");
     }
     return HDLA_OK;
@@ -1860,6 +1917,7 @@ int tc_chunk_bwd(const HdlaDims& d, const void* q, const void* k, const void* v,
     }
     const TcPlan pl = make_tc_plan(d);
     const bool param_ab = (d.flags & HDLA_FLAG_PARAM_AB) != 0;
+    const bool full = pl.KW == K && pl.VW == V;              // tiles of the full width: the kernels' extents are constants
     auto U4 = [&](size_t off) { return reinterpret_cast<uint4*>(ws + off); };
     auto F = [&](size_t off) { return reinterpret_cast<float*>(ws + off); };
     int* status = reinterpret_cast<int*>(ws + pl.status);
@@ -1871,8 +1929,8 @@ int tc_chunk_bwd(const HdlaDims& d, const void* q, const void* k, const void* v,
 
     if (phase == HDLA_PHASE_ALL || phase == HDLA_PHASE_PRE) {
         DauP dp{(const __nv_bfloat16*)d_o, U4(pl.Vc), U4(pl.V2), U4(pl.Aqb), U4(pl.dOc), U4(pl.dAqk), U4(pl.dAqb),
-                U4(pl.DV2), d.T, d.H, pl.NT, status, d.V, chunk_tab};
-        launch(dau_tc_kernel, dim3(G), dim3(128), 81920, st, dp);
+                U4(pl.DV2), d.T, d.H, pl.NT, status, d.V, pl.VW, chunk_tab};
+        launch(full ? dau_tc_kernel<true> : dau_tc_kernel<false>, dim3(G), dim3(128), 81920, st, dp);
         HDLA_CHECK_LAUNCH("dau_tc_kernel");
         if (phase == HDLA_PHASE_PRE) return HDLA_OK;
     }
@@ -1884,7 +1942,7 @@ int tc_chunk_bwd(const HdlaDims& d, const void* q, const void* k, const void* v,
         sp.Hs = U4(pl.Hs); sp.HT = F(pl.HT); sp.dgl = dgl;
         sp.NT = pl.NT; sp.reverse = 1; sp.status = status; sp.add_stride = 1; sp.r1_stride = 1; sp.no_store = no_store;
         sp.nseg = 1; sp.seg_len = pl.NT; sp.zero_tile = U4(pl.zero);
-        sp.Kd = d.K; sp.Vd = d.V; sp.seq_tab = seq_tab; sp.H = d.H;
+        sp.Kd = d.K; sp.Vd = d.V; sp.KW = pl.KW; sp.VW = pl.VW; sp.seq_tab = seq_tab; sp.H = d.H;
         return sp;
     };
     if (phase == HDLA_PHASE_STATE) {
@@ -1893,15 +1951,15 @@ int tc_chunk_bwd(const HdlaDims& d, const void* q, const void* k, const void* v,
         if (pl.nseg > 1) {                    // per-segment gradients from zero, then composed with T^T
             ScanTcP s1 = rscan_params(nullptr, nullptr, nullptr, F(pl.Fseg), nullptr, 1);
             s1.nseg = pl.nseg; s1.seg_len = pl.seg_len; s1.fin_by_slot = 1;
-            launch(scan_tc_kernel, dim3(pl.BH * pl.nseg), dim3(256), 196608, st, s1);
+            launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(pl.BH * pl.nseg), dim3(256), 196608, st, s1);
             HDLA_CHECK_LAUNCH("scan_tc_kernel");
             launch(compose_segments_kernel, dim3(dim3(pl.BH, V / kComposeCols)), dim3(256), kComposeSmem, st, F(pl.Tseg), F(pl.Fseg), dht, nullptr, dh0,
-                                                                         pl.nseg, 1, 0, 0, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr);
+                                                                         pl.nseg, 1, 0, 0, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr, pl.KW);
             HDLA_CHECK_LAUNCH("compose_segments_kernel");
             return HDLA_OK;
         }
         ScanTcP sp = rscan_params(dht, nullptr, nullptr, dh0, nullptr, 1);
-        launch(scan_tc_kernel, dim3(pl.BH), dim3(256), 196608, st, sp);
+        launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(pl.BH), dim3(256), 196608, st, sp);
         HDLA_CHECK_LAUNCH("scan_tc_kernel");
         return HDLA_OK;
     }
@@ -1912,47 +1970,47 @@ int tc_chunk_bwd(const HdlaDims& d, const void* q, const void* k, const void* v,
         ScanTcP s1 = rscan_params(nullptr, U4(pl.DE), U4(pl.DV2), F(pl.Fseg), F(pl.dgl), 1);
         s1.nseg = pl.nseg; s1.seg_len = pl.seg_len; s1.fin_by_slot = 1;
         s1.seg_off = 1; s1.seg_cnt = pl.nseg - 1; s1.lead_real = 1; s1.lead_init = dht;
-        launch(scan_tc_kernel, dim3(pl.BH * (pl.nseg - 1)), dim3(256), 196608, st, s1);
+        launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(pl.BH * (pl.nseg - 1)), dim3(256), 196608, st, s1);
         HDLA_CHECK_LAUNCH("scan_tc_kernel");
         launch(compose_segments_kernel, dim3(dim3(pl.BH, V / kComposeCols)), dim3(256), kComposeSmem, st, F(pl.Tseg), F(pl.Fseg), nullptr, F(pl.Sin), nullptr,
-                                                                     pl.nseg, 1, 0, 1, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr);
+                                                                     pl.nseg, 1, 0, 1, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr, pl.KW);
         HDLA_CHECK_LAUNCH("compose_segments_kernel");
         ScanTcP s2 = rscan_params(F(pl.Sin), U4(pl.DE), U4(pl.DV2), dh0, F(pl.dgl), 0);
         s2.nseg = pl.nseg; s2.seg_len = pl.seg_len; s2.init_by_slot = 1; s2.fin_last_only = 1;
         s2.seg_off = 0; s2.seg_cnt = pl.nseg - 1;
-        launch(scan_tc_kernel, dim3(pl.BH * (pl.nseg - 1)), dim3(256), 196608, st, s2);
+        launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(pl.BH * (pl.nseg - 1)), dim3(256), 196608, st, s2);
         HDLA_CHECK_LAUNCH("scan_tc_kernel");
     } else     if (pl.nseg > 1) {
         // two-level reverse scan; the segment transitions were left in the workspace by the forward pass
         if (phase == HDLA_PHASE_ALL) {        // (a phased POST call finds the per-segment gradients in the workspace)
             ScanTcP s1 = rscan_params(nullptr, nullptr, nullptr, F(pl.Fseg), nullptr, 1);
             s1.nseg = pl.nseg; s1.seg_len = pl.seg_len; s1.fin_by_slot = 1;
-            launch(scan_tc_kernel, dim3(pl.BH * pl.nseg), dim3(256), 196608, st, s1);
+            launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(pl.BH * pl.nseg), dim3(256), 196608, st, s1);
             HDLA_CHECK_LAUNCH("scan_tc_kernel");
         }
-        launch(compose_segments_kernel, dim3(dim3(pl.BH, V / kComposeCols)), dim3(256), kComposeSmem, st, F(pl.Tseg), F(pl.Fseg), dht, F(pl.Sin), nullptr, pl.nseg, 1, 0, 0, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr);
+        launch(compose_segments_kernel, dim3(dim3(pl.BH, V / kComposeCols)), dim3(256), kComposeSmem, st, F(pl.Tseg), F(pl.Fseg), dht, F(pl.Sin), nullptr, pl.nseg, 1, 0, 0, pl.nseg, 1, pl.nseg, 1, nullptr, nullptr, pl.KW);
         HDLA_CHECK_LAUNCH("compose_segments_kernel");
         ScanTcP s2 = rscan_params(F(pl.Sin), U4(pl.DE), U4(pl.DV2), dh0, F(pl.dgl), 0);
         s2.nseg = pl.nseg; s2.seg_len = pl.seg_len; s2.init_by_slot = 1; s2.fin_last_only = 1;
-        launch(scan_tc_kernel, dim3(pl.BH * pl.nseg), dim3(256), 196608, st, s2);
+        launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(pl.BH * pl.nseg), dim3(256), 196608, st, s2);
         HDLA_CHECK_LAUNCH("scan_tc_kernel");
     } else {
         ScanTcP sp = rscan_params(dht, U4(pl.DE), U4(pl.DV2), dh0, F(pl.dgl), 0);
-        launch(scan_tc_kernel, dim3(pl.BH), dim3(256), 196608, st, sp);
+        launch(full ? scan_tc_kernel<true> : scan_tc_kernel<false>, dim3(pl.BH), dim3(256), 196608, st, sp);
         HDLA_CHECK_LAUNCH("scan_tc_kernel");
     }
     // --- wy: dP, dAak, dAab in one kernel
-    WyBwdP wyp{U4(pl.M), U4(pl.DV2), U4(pl.Vc), U4(pl.V2), U4(pl.dP), U4(pl.dAak), U4(pl.dAab), status};
-    launch(wy_bwd_tc_kernel, dim3(G), dim3(128), kWySmem, st, wyp);
+    WyBwdP wyp{U4(pl.M), U4(pl.DV2), U4(pl.Vc), U4(pl.V2), U4(pl.dP), U4(pl.dAak), U4(pl.dAab), status, pl.VW};
+    launch(full ? wy_bwd_tc_kernel<true> : wy_bwd_tc_kernel<false>, dim3(G), dim3(128), kWySmem, st, wyp);
     HDLA_CHECK_LAUNCH("wy_bwd_tc_kernel");
     // --- everything else: hat-operand gradients, dv, un-gating, dgk
     GradP gp{U4(pl.Hs), U4(pl.Bh), U4(pl.dOc), U4(pl.Kh), U4(pl.dAqb), U4(pl.dAqk), U4(pl.DE), U4(pl.dP), U4(pl.Aak),
              U4(pl.Aqk), U4(pl.dAab), U4(pl.dAak), U4(pl.V2), U4(pl.Ah), U4(pl.Qh), U4(pl.Vc),
              (bp)(ws + pl.ghat), F(pl.E), F(pl.dgl), (bp)dq, (bp)dk, (bp)dv, param_ab ? (bp)(ws + pl.dab) : (bp)da,
              param_ab ? (bp)(ws + pl.dab + pl.dab_half) : (bp)db, dgk, scale, d.T, d.H, pl.NT, d.gk_dtype,
-             status, (long long)G, d.K, d.V, chunk_tab};
+             status, (long long)G, d.K, d.V, pl.KW, pl.VW, chunk_tab};
     const unsigned grad_grid = G < (unsigned)sm_count() ? G : (unsigned)sm_count();    // one persistent CTA per SM
-    launch(grad_tc_kernel, dim3(grad_grid), dim3(544), kGradSmem, st, gp);
+    launch(full ? grad_tc_kernel<true> : grad_tc_kernel<false>, dim3(grad_grid), dim3(544), kGradSmem, st, gp);
     HDLA_CHECK_LAUNCH("grad_tc_kernel");
     if (param_ab)      // da, db -> dbeta (through the `da` argument), and their shares of dk and dgk = dlog_f added in place
         return param_ab_launch(true, a, k, gk, ws + pl.dab, ws + pl.dab + pl.dab_half, da, dk, dgk, d.B, d.T, d.H, d.K,
@@ -1963,23 +2021,23 @@ int tc_chunk_bwd(const HdlaDims& d, const void* q, const void* k, const void* v,
 // debugging aid: named bf16 tile buffer of the tensor-core workspace -> fp32 row-major [G][rows][cols]
 int tc_debug_buffer(const HdlaDims& d, const unsigned char* ws, const char* name, float* out, cudaStream_t st) {
     const TcPlan pl = make_tc_plan(d);
-    struct Ent { const char* n; size_t off; int rows, cols; };
-    const Ent tab[] = {{"Qh", pl.Qh, 64, 128}, {"Kh", pl.Kh, 64, 128}, {"Ah", pl.Ah, 128, 128}, {"Bh", pl.Bh, 128, 128},
-                       {"Vc", pl.Vc, 64, 128}, {"Aqk", pl.Aqk, 64, 64}, {"Aqb", pl.Aqb, 64, 128},
-                       {"Aak", pl.Aak, 128, 64}, {"M", pl.M, 128, 128},
-                       {"W", pl.W, 128, 128}, {"U", pl.U, 128, 128}, {"Hs", pl.Hs, 128, 128},
-                       {"V2", pl.V2, 128, 128},
-                       {"dOc", pl.dOc, 64, 128}, {"dAqk", pl.dAqk, 64, 64}, {"dAqb", pl.dAqb, 64, 128},
-                       {"DV2", pl.DV2, 128, 128}, {"DE", pl.DE, 128, 128},
-                       {"dP", pl.dP, 128, 128}, {"dAak", pl.dAak, 128, 64}, {"dAab", pl.dAab, 128, 128}};
+    struct Ent { const char* n; size_t off; int rows, cols, w_rows, w_cols; };
+    const Ent tab[] = {{"Qh", pl.Qh, 64, 128, 64, pl.KW}, {"Kh", pl.Kh, 64, 128, 64, pl.KW}, {"Ah", pl.Ah, 128, 128, 128, pl.KW}, {"Bh", pl.Bh, 128, 128, 128, pl.KW},
+                       {"Vc", pl.Vc, 64, 128, 64, pl.VW}, {"Aqk", pl.Aqk, 64, 64, 64, 64}, {"Aqb", pl.Aqb, 64, 128, 64, 128},
+                       {"Aak", pl.Aak, 128, 64, 128, 64}, {"M", pl.M, 128, 128, 128, 128},
+                       {"W", pl.W, 128, 128, 128, pl.KW}, {"U", pl.U, 128, 128, 128, pl.VW}, {"Hs", pl.Hs, 128, 128, pl.KW, pl.VW},
+                       {"V2", pl.V2, 128, 128, 128, pl.VW},
+                       {"dOc", pl.dOc, 64, 128, 64, pl.VW}, {"dAqk", pl.dAqk, 64, 64, 64, 64}, {"dAqb", pl.dAqb, 64, 128, 64, 128},
+                       {"DV2", pl.DV2, 128, 128, 128, pl.VW}, {"DE", pl.DE, 128, 128, pl.KW, pl.VW},
+                       {"dP", pl.dP, 128, 128, 128, pl.VW}, {"dAak", pl.dAak, 128, 64, 128, 64}, {"dAab", pl.dAab, 128, 128, 128, 128}};
     for (const Ent& e : tab)
         if (!strcmp(e.n, name)) {
             c8_to_rowmajor_kernel<<<(unsigned)pl.G, 128, 0, st>>>(reinterpret_cast<const uint4*>(ws + e.off), out,
-                                                                  e.rows, e.cols);
+                                                                  e.rows, e.cols, e.w_rows, e.w_cols);
             HDLA_CHECK_LAUNCH("c8_to_rowmajor_kernel");
             return HDLA_OK;
         }
-    if (!strcmp(name, "P") || !strcmp(name, "dW")) {         // P = Aak v,  dWh = dv2 St^T
+    if (pl.KW == K && pl.VW == V && (!strcmp(name, "P") || !strcmp(name, "dW"))) {         // P = Aak v,  dWh = dv2 St^T
         const bool fwd = name[0] == 'P';
         c8_product_kernel<<<(unsigned)pl.G, 128, 0, st>>>(reinterpret_cast<const uint4*>(ws + (fwd ? pl.Aak : pl.DV2)),
                                                           reinterpret_cast<const uint4*>(ws + (fwd ? pl.Vc : pl.Hs)), out,

@@ -17,6 +17,7 @@ constexpr int CH128 = 16 * 128;    // chunks of a [128 x 128] tile
 // workspace plan (byte offsets)
 // ------------------------------------------------------------------------------------------
 struct TcPlan {
+    int KW, VW;                        // widths of the tiles: head dims rounded up to 16 (the contraction step of one MMA)
     int B, T, H, NT, BH;               // NT: chunks per sequence (all chunks of the packed batch with cu_seqlens);
     long long G;                       // BH: (sequence, head) pairs = scans and states;  G = tiles = H * chunks
     size_t status, Qh, Kh, Ah, Bh, Vc, E, ghat, Aqk, Aqb, Aak, Aab, M, W, U, Hs, V2, HT, zero;
@@ -43,6 +44,7 @@ __device__ __forceinline__ void chunk_tokens(const int2* chunk_tab, int n, int T
 inline TcPlan make_tc_plan(const HdlaDims& d) {
     TcPlan p{};
     p.B = d.B; p.T = d.T; p.H = d.H;
+    p.KW = (d.K + 15) & ~15; p.VW = (d.V + 15) & ~15;
     p.NT = (d.T + C - 1) / C;
     p.BH = d.B * d.H;
     p.nseq = 0;

@@ -80,4 +80,13 @@ __device__ __forceinline__ void tmem_row64(uint32_t addr, float* f) {
     for (int j = 0; j < 32; ++j) { f[j] = __uint_as_float(a[j]); f[32 + j] = __uint_as_float(b[j]); }
 }
 
+// 32 accumulator columns of this thread's row -> registers
+__device__ __forceinline__ void tmem_row32(uint32_t addr, float* f) {
+    uint32_t a[32];
+    sm100::tmem_ld_x32(addr, a);
+    sm100::tmem_wait_ld();
+#pragma unroll
+    for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(a[j]);
+}
+
 }  // namespace hdla

@@ -32,7 +32,7 @@ def contiguous(fn):
 
 def _tc_shape(q, v, RANK_AB: int) -> bool:
     """Whether the bf16 tensor-core pipeline takes this problem (at its own chunk of 64): bf16, rank 2, head dims
-    that are multiples of 8 up to 128 (smaller ones run zero-padded on the same 128-wide tiles)."""
+    that are multiples of 8 up to 128 (smaller ones fill a prefix of the 128-wide tiles)."""
     T, K, V = q.shape[1], q.shape[-1], v.shape[-1]
     return (q.dtype == torch.bfloat16 and RANK_AB == 2 and K % 8 == 0 and V % 8 == 0 and 8 <= K <= 128
             and 8 <= V <= 128 and T > 32)

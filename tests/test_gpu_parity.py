@@ -363,6 +363,21 @@ def test_bf16_head_dims_below_128_run_on_tensor_cores(dev, B, T, H, K, V):
     assert torch.equal(o2, got["o"]) and torch.equal(ht2, got["ht"])
 
 
+@pytest.mark.parametrize("K,V", [(8, 8), (16, 128), (128, 24), (72, 40), (120, 104), (64, 64)])
+@pytest.mark.parametrize("B,T", [(1, 1100), (2, 65)])        # two-level scan with a ragged last chunk / one scan per pair
+def test_bf16_narrow_tiles_do_not_read_their_padding(dev, K, V, B, T):
+    """Tiles of narrow heads fill a prefix of their slots.  With NaN in all free device memory, anything read beyond the
+    prefix shows: widths at the edges of the 16-channel step, and of the 64-column halves of an accumulator."""
+    import hdla_impl_b200 as HD
+    x = make_inputs(B, T, 2, K, V, R, seed=K + V, dtype=torch.bfloat16, gk_div=4.0, h0_std=0.3, with_dht=True)
+    ref = oracle_chunk(x, K ** -0.5, True, True, torch.bfloat16)
+    junk = torch.full((1 << 26,), float("nan"), device=dev)     # the call's workspace is cut from this block
+    del junk
+    got = run_chunk(x, dev, K ** -0.5, 64, True, True, torch.bfloat16)
+    HD.check_status(dev, wait=True)
+    assert_close(got, ref, 2e-2, f"K={K} V={V}")               # bf16 results and operands, as for the other widths
+
+
 @pytest.mark.parametrize("seed", range(8))
 def test_bf16_random_shapes_against_oracle(dev, seed):
     """Seeded random problems of the tensor-core pipeline (batch, ragged length, heads, head dims that are multiples
