@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(128) gram_tc_kernel(GramP p) {
             p.Aak[g * CH64 + cg * 128 + r] = t8::pack8(f + cg * 8);   // [128 x 64] tile: 8 column groups of 128 rows
         }
 #pragma unroll 1
-        for (int hh = 0; hh < 2; ++hh) {                      // Aab: column token < row token
+        for (int hh = 0; hh < (warp < 2 ? 1 : 2); ++hh) {     // Aab: column token < row token (a lower tile)
             tmem_row64(t8::taddr(tmem, warp, 64 + hh * 64), f);
 #pragma unroll
             for (int cg = 0; cg < 8; ++cg) {
@@ -411,8 +411,8 @@ __global__ void __launch_bounds__(128) inverse_tc_kernel(InvP p) {
     // last time at the level that produces the block of M at the same place (later levels read it only into
     // accumulator rows that are never used).
     // The X blocks of a level (at most 64 x 64 in all) live in the tile's upper right quadrant (rows 0..63, columns
-    // 64..127), which is zero in L and in M and which the products read only into accumulator rows that are never
-    // used; it is cleared again before M is stored.  32 KB per CTA: seven CTAs per SM.
+    // 64..127), which is zero in L and in M, is not loaded or stored and which the products read only into accumulator
+    // rows that are never used.  32 KB per CTA: seven CTAs per SM.
     uint4* sD = reinterpret_cast<uint4*>(smem);      // 32 KB: L, overwritten by M
     __shared__ __align__(8) uint64_t ld_bar, mma_bar;
     __shared__ uint32_t tmem_s;
@@ -421,8 +421,8 @@ __global__ void __launch_bounds__(128) inverse_tc_kernel(InvP p) {
     if (warp == 0) { tmem_alloc(&tmem_s, 64); tmem_relinquish(); }
     if (tid == 0) {
         mbar_init(&ld_bar, 1); mbar_init(&mma_bar, 1); fence_mbar_init();
-        mbar_expect_tx(&ld_bar, 32768);
-        bulk_g2s(sD, p.Aab + g * CH128, 32768, &ld_bar);
+        mbar_expect_tx(&ld_bar, kLowerBytes);
+        lower_g2s(sD, p.Aab + g * CH128, &ld_bar);
     }
     tc_fence_before();
     __syncthreads();
@@ -513,11 +513,8 @@ __global__ void __launch_bounds__(128) inverse_tc_kernel(InvP p) {
         tc_fence_before();
         __syncthreads();
     }
-    for (int e = tid; e < 512; e += 128) sD[(8 + (e >> 6)) * 128 + (e & 63)] = make_uint4(0, 0, 0, 0);    // the quadrant
-    fence_proxy_async();
-    __syncthreads();
     if (tid == 0) {
-        bulk_s2g(p.M + g * CH128, sD, 32768);
+        lower_s2g(p.M + g * CH128, sD);
         bulk_commit();
         bulk_wait_read<0>();
     }
@@ -552,12 +549,14 @@ __global__ void __launch_bounds__(128) wu_tc_kernel(WuP p) {
     if (warp == 0) { tmem_alloc(&tmem_s, 256); tmem_relinquish(); }
     if (tid == 0) {
         mbar_init(&ld_bar, 1); mbar_init(&mma_bar, 1); fence_mbar_init();
-        mbar_expect_tx(&ld_bar, 16384 + 128 * VW + 32768 + 256 * KW);
+        mbar_expect_tx(&ld_bar, 16384 + 128 * VW + kLowerBytes + 256 * KW);
         bulk_g2s(sAak, p.Aak + g * CH64, 16384, &ld_bar);
         bulk_g2s(sV, p.Vc + g * CH64, 128 * VW, &ld_bar);
-        bulk_g2s(sM, p.M + g * CH128, 32768, &ld_bar);
+        lower_g2s(sM, p.M + g * CH128, &ld_bar);
         bulk_g2s(sA, p.Ah + g * CH128, 256 * KW, &ld_bar);
     }
+    lower_clear(sM, tid);
+    fence_proxy_async();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -904,7 +903,7 @@ __global__ void __launch_bounds__(256) scan_tc_kernel(ScanTcP p) {
 // Wh = M Ah and v2 = Wh St + u that is  M^T dv2 (P^T M^T + St^T Ah^T M^T) = dP (u + Wh St)^T = dP v2^T,  and the
 // share of dAh that went through dWh is  M^T dWh = dP St^T  (grad_tc_kernel): neither P, Ah and St are read here nor
 // dWh, dM and M^T dM formed.
-// Bound by memory: 112 KB in, 80 KB out per tile, against 176 + 112 KB of the longer form (which also left room for
+// Bound by memory: 104 KB in, 72 KB out per tile, against 176 + 112 KB of the longer form (which also left room for
 // one CTA per SM only).  dP takes M's place in shared memory, so 112 KB hold a tile and two CTAs per SM cover each
 // other's round trips.
 // ------------------------------------------------------------------------------------------
@@ -930,13 +929,15 @@ __global__ void __launch_bounds__(128) wy_bwd_tc_kernel(WyBwdP p) {
     if (warp == 0) { tmem_alloc(&tmem_s, 256); tmem_relinquish(); }
     if (tid == 0) {
         mbar_init(&ld1, 1); mbar_init(&ld2, 1); mbar_init(&mma_bar, 1); fence_mbar_init();
-        mbar_expect_tx(&ld1, 32768 + 256 * VW);
-        bulk_g2s(bM, p.M + g * CH128, 32768, &ld1);
+        mbar_expect_tx(&ld1, kLowerBytes + 256 * VW);
+        lower_g2s(bM, p.M + g * CH128, &ld1);
         bulk_g2s(bDV2, p.DV2 + g * CH128, 256 * VW, &ld1);
         mbar_expect_tx(&ld2, 128 * VW + 256 * VW);
         bulk_g2s(bVc, p.Vc + g * CH64, 128 * VW, &ld2);
         bulk_g2s(bV2, p.V2 + g * CH128, 256 * VW, &ld2);
     }
+    lower_clear(bM, tid);
+    fence_proxy_async();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -982,7 +983,7 @@ __global__ void __launch_bounds__(128) wy_bwd_tc_kernel(WyBwdP p) {
         p.dAak[g * CH64 + c8 * 128 + r] = t8::pack8(f + c8 * 8);
     }
 #pragma unroll 1
-    for (int hh = 0; hh < 2; ++hh) {
+    for (int hh = 0; hh < (warp < 2 ? 1 : 2); ++hh) {               // (a lower tile)
         tmem_row64(t8::taddr(tmem, warp, 64 + hh * 64), f);
 #pragma unroll
         for (int c8 = 0; c8 < 8; ++c8) {
@@ -1203,13 +1204,14 @@ __global__ void __launch_bounds__(128) out_tc_kernel(OutP p) {
 
 // debugging aid: C8 bf16 tile -> fp32 row-major
 // (tiles of narrow heads hold w_rows x w_cols elements of it, the rest is written as zero)
-__global__ void c8_to_rowmajor_kernel(const uint4* src, float* dst, int rows, int cols, int w_rows, int w_cols) {
+__global__ void c8_to_rowmajor_kernel(const uint4* src, float* dst, int rows, int cols, int w_rows, int w_cols,
+                                     int lower) {
     const long long g = blockIdx.x;
     const int nch = rows * cols / 8;
     for (int e = threadIdx.x; e < nch; e += blockDim.x) {
         const int cg = e / rows, r = e % rows;
         float f[8];
-        const bool kept = r < w_rows && cg * 8 < w_cols;
+        const bool kept = r < w_rows && cg * 8 < w_cols && !(lower && r < 64 && cg >= 8);
         t8::unpack8(kept ? src[g * nch + cg * w_rows + r] : make_uint4(0, 0, 0, 0), f);
         for (int j = 0; j < 8; ++j) dst[(size_t)g * rows * cols + (size_t)r * cols + cg * 8 + j] = f[j];
     }
@@ -1363,8 +1365,8 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
         mbar_expect_tx(&ld[T_dAakAh], 16384 + k128);          // (Ah follows when slot B is free)
         bulk_g2s(sa, p.dAak + g * CH64, 16384, &ld[T_dAakAh]);
         wait_or_flag(&mc6, ph, p.status, 76);
-        mbar_expect_tx(&ld[T_dAab], 32768);
-        bulk_g2s(sD, p.dAab + g * CH128, 32768, &ld[T_dAab]);
+        mbar_expect_tx(&ld[T_dAab], kLowerBytes);
+        lower_g2s(sD, p.dAab + g * CH128, &ld[T_dAab]);
         mbar_expect_tx(&ld[T_Qh], k64);
         bulk_g2s(sE, p.Qh + g * CH64, k64, &ld[T_Qh]);
         wait_or_flag(&ld[T_Kh], ph, p.status, 77);
@@ -1380,7 +1382,9 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
         wait_or_flag(&ld[T_Vc], ph, p.status, 81);
         chain0<false, false>(tmem + 384, t8::tile(sC, KW), t8::tile(sE + CH64, 64), 64, VW, false);    // P5: dSt v^T
         wait_or_flag(&ld[T_dAab], ph, p.status, 82);
-        chain0<true, false>(tmem + 128, t8::tile(sB, 128), t8::tile(sD, 128), 128, 128, true);    // P3: Bh^T dAab^T
+        // P3: Bh^T dAab^T, without the quadrant of dAab that is zero (and not in the slot)
+        t8::mma_chain<true, false>(tmem + 128, t8::tile(sB, 128), 0, 0, t8::tile(sD, 128), 0, 0, 128, 64, true);
+        t8::mma_chain<true, false>(tmem + 192, t8::tile(sB, 128), 64, 0, t8::tile(sD, 128), 64, 64, 64, 64, true);
         umma_commit(&mc9);                                                                        // slot B free
         wait_or_flag(&ld[T_V2], ph, p.status, 83);
         chain0<false, false>(tmem + 256, t8::tile(sC, KW), t8::tile(sA, 128), 128, VW, false);    // P4: dSt V2^T
@@ -1394,7 +1398,8 @@ __global__ void __launch_bounds__(544) grad_tc_kernel(GradP p) {
         chain0<true, false>(tmem + 128, t8::tile(sb, 64), t8::tile(sa, 128), 128, 64, true);      // P3: Kh^T dAak^T
         umma_commit(&m3);
         TL(7);
-        chain0<true, true>(tmem + 256, t8::tile(sB, 128), t8::tile(sD, 128), 128, 128, true);     // P4: Ah^T dAab
+        t8::mma_chain<true, true>(tmem + 256, t8::tile(sB, 128), 0, 0, t8::tile(sD, 128), 0, 0, 64, 64, true);      // P4: Ah^T dAab
+        t8::mma_chain<true, true>(tmem + 256, t8::tile(sB, 128), 64, 0, t8::tile(sD, 128), 64, 0, 128, 64, true);   //   (likewise)
         chain0<true, true>(tmem + 384, t8::tile(sB, 128), t8::tile(sa, 128), 64, 128, true);      // P5: Ah^T dAak
         umma_commit(&m4);
         wait_or_flag(&m4, ph, p.status, 88);
@@ -2033,7 +2038,7 @@ int tc_debug_buffer(const HdlaDims& d, const unsigned char* ws, const char* name
     for (const Ent& e : tab)
         if (!strcmp(e.n, name)) {
             c8_to_rowmajor_kernel<<<(unsigned)pl.G, 128, 0, st>>>(reinterpret_cast<const uint4*>(ws + e.off), out,
-                                                                  e.rows, e.cols, e.w_rows, e.w_cols);
+                                                                  e.rows, e.cols, e.w_rows, e.w_cols, !strcmp(name, "M") || !strcmp(name, "dAab"));
             HDLA_CHECK_LAUNCH("c8_to_rowmajor_kernel");
             return HDLA_OK;
         }

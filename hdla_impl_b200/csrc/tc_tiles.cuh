@@ -89,4 +89,24 @@ __device__ __forceinline__ void tmem_row32(uint32_t addr, float* f) {
     for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(a[j]);
 }
 
+// Aab, its gradient and M = (I - Aab)^-1 are [128 x 128] and lower triangular: the quadrant of rows 0..63, columns 64..127
+// is zero and neither stored nor loaded (24 of 32 KB move: the left half of the tile and eight 1 KB pieces; the kernels
+// between which these tiles pass are bound by the bytes they move).
+constexpr uint32_t kLowerBytes = 24576;
+__device__ __forceinline__ void lower_g2s(uint4* dst, const uint4* src, uint64_t* bar) {
+    sm100::bulk_g2s(dst, src, 16384, bar);
+#pragma unroll 1
+    for (int c = 8 * 128 + 64; c < 16 * 128; c += 128) sm100::bulk_g2s(dst + c, src + c, 1024, bar);
+}
+__device__ __forceinline__ void lower_s2g(uint4* dst, const uint4* src) {
+    sm100::bulk_s2g(dst, src, 16384);
+#pragma unroll 1
+    for (int c = 8 * 128 + 64; c < 16 * 128; c += 128) sm100::bulk_s2g(dst + c, src + c, 1024);
+}
+// zeros in the quadrant, for products that read the whole tile (128 threads; a proxy fence and a barrier follow)
+__device__ __forceinline__ void lower_clear(uint4* tile, int tid) {
+#pragma unroll
+    for (int e = tid; e < 512; e += 128) tile[(8 + (e >> 6)) * 128 + (e & 63)] = make_uint4(0, 0, 0, 0);
+}
+
 }  // namespace hdla
