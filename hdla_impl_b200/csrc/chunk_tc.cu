@@ -42,6 +42,7 @@ struct PrepP {
     uint4 *Qh, *Kh, *Ah, *Bh, *Vc;
     float* E;
     __nv_bfloat16* ghat;                  // e^{gi - half} per (token, channel), bf16 row-major [64][128]
+                                          // (null in a forward-only call: only the backward pass reads it)
     float scale;
     int T, H, NT, gdt;
     int* status;
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(128, 4) prep_hat_kernel(PrepP p) {
             c0 = t8::pack8(y);
             c1 = t8::pack8(z);
             if (k_in) sm100::st_global_32B(p.Bh + (size_t)g * CH128 + kc * 128 + r * R, c0, c1);
-            if (k_in) *reinterpret_cast<uint4*>(p.ghat + (size_t)g * C * K + (size_t)r * K + kc * 8) = t8::pack8(ep);
+            if (k_in && p.ghat) *reinterpret_cast<uint4*>(p.ghat + (size_t)g * C * K + (size_t)r * K + kc * 8) = t8::pack8(ep);
         } else {   // rows 2r, 2r+1 of Ah / Bh are adjacent chunks: one 32-byte store each
             uint4 c0, c1;
             t8::unpack8(cur.a0, x);
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(128, 4) prep_hat_kernel(PrepP p) {
             if (k_in) sm100::st_global_32B(p.Bh + (size_t)g * CH128 + kc * 128 + r * R, c0, c1);
             // the un-gating factors of the backward pass, e^{gi - half}, in bf16 (their error, 2^-9, is below the
             // rounding of the bf16 gradients they scale)
-            if (k_in) *reinterpret_cast<uint4*>(p.ghat + (size_t)g * C * K + (size_t)r * K + kc * 8) = t8::pack8(ep);
+            if (k_in && p.ghat) *reinterpret_cast<uint4*>(p.ghat + (size_t)g * C * K + (size_t)r * K + kc * 8) = t8::pack8(ep);
         }
         cur = nxt;
         if (tid == 0) TL(2 + it);
@@ -1801,7 +1802,7 @@ int tc_chunk_fwd(const HdlaDims& d, const void* q, const void* k, const void* v,
             TRY(tc_launch_chunk_prep(pl, d, q, k, v, a, b, gk, scale, ws, save_bwd, st));
         } else {
             PrepP pp{(bp)q, (bp)k, (bp)v, (bp)a, (bp)b, gk, U4(pl.Qh), U4(pl.Kh), U4(pl.Ah), U4(pl.Bh), U4(pl.Vc),
-                     F(pl.E), (__nv_bfloat16*)(ws + pl.ghat), scale, d.T, d.H, pl.NT, d.gk_dtype, status, d.K, d.V, chunk_tab, pl.KW, pl.VW,
+                     F(pl.E), save_bwd ? (__nv_bfloat16*)(ws + pl.ghat) : nullptr, scale, d.T, d.H, pl.NT, d.gk_dtype, status, d.K, d.V, chunk_tab, pl.KW, pl.VW,
                      param_ab ? (bp)a : nullptr, (d.flags & HDLA_FLAG_NORM_K) ? 1 : 0};
             if (param_ab) launch(full ? prep_hat_kernel<true, true> : prep_hat_kernel<true, false>, dim3(G), dim3(128), 0, st, pp);
             else launch(full ? prep_hat_kernel<false, true> : prep_hat_kernel<false, false>, dim3(G), dim3(128), 0, st, pp);
