@@ -93,16 +93,16 @@ def bytes_per_token_head(C: int, D: int, elt: int) -> float:
 # scan_tc_kernel is launched twice per step (forward 192.5, reverse 225).
 KERNEL_KIB = {
     "chunk_prep_tc_kernel": 424.5,
-    "prep_hat_kernel": 256.5, "gram_tc_kernel": 168.0, "inverse_tc_kernel": 64.0, "wu_tc_kernel": 192.0,
+    "prep_hat_kernel": 256.5, "gram_tc_kernel": 160.0, "inverse_tc_kernel": 48.0, "wu_tc_kernel": 152.0,
     "scan_tc_kernel": (192.5 + 225.0) / 2, "out_tc_kernel": 136.0, "dau_tc_kernel": 152.0,
-    "wy_bwd_tc_kernel": 288.0, "grad_tc_kernel": 560.5,
+    "wy_bwd_tc_kernel": 176.0, "grad_tc_kernel": 488.5,
 }
 # dram__bytes_read.sum + dram__bytes_write.sum per launch (GB) at cfg 1: one ncu capture at B=2 (a quarter of
 # cfg 1; traffic is proportional to the number of chunks), scaled by 4 -- see profiles/
 KERNEL_NCU_TRAFFIC_GB = {
-    "prep_hat_kernel": 2.09, "gram_tc_kernel": 1.20, "inverse_tc_kernel": 0.33, "wu_tc_kernel": 1.39,
-    "scan_tc_kernel": (1.51 + 1.79) / 2, "out_tc_kernel": 1.08, "dau_tc_kernel": 1.06, "wy_bwd_tc_kernel": 2.25,
-    "grad_tc_kernel": 4.62,
+    "prep_hat_kernel": 1.97, "gram_tc_kernel": 1.15, "inverse_tc_kernel": 0.21, "wu_tc_kernel": 1.08,
+    "scan_tc_kernel": (1.51 + 1.79) / 2, "out_tc_kernel": 1.08, "dau_tc_kernel": 1.06, "wy_bwd_tc_kernel": 1.26,
+    "grad_tc_kernel": 3.98,
 }
 
 

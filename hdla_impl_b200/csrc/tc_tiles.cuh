@@ -91,7 +91,7 @@ __device__ __forceinline__ void tmem_row32(uint32_t addr, float* f) {
 
 // Aab, its gradient and M = (I - Aab)^-1 are [128 x 128] and lower triangular: the quadrant of rows 0..63, columns 64..127
 // is zero and neither stored nor loaded (24 of 32 KB move: the left half of the tile and eight 1 KB pieces; the kernels
-// between which these tiles pass are bound by the bytes they move).
+// between which these tiles pass are bound by the bytes they move: B8 T4096 H16 fwd+bwd 3099 -> 3040 us).
 constexpr uint32_t kLowerBytes = 24576;
 __device__ __forceinline__ void lower_g2s(uint4* dst, const uint4* src, uint64_t* bar) {
     sm100::bulk_g2s(dst, src, 16384, bar);
