@@ -14,7 +14,7 @@
 // Head dims below 128: a [rows x channels] tile keeps its 128-wide slot but only its first KW (VW) = head dim rounded
 // up to 16 columns are written, moved and multiplied -- column groups are contiguous in C8, so that is a prefix -- and a
 // state tile is [KW x VW] with a row pitch of KW.  The kernels exist twice: FULL (128 x 128, extents are constants) and
-// with the extents as arguments.  B4 T2001 H16 K=V=64 fwd+bwd: 866 us with zero-padded 128-wide tiles, 749 us so.
+// with the extents as arguments.  B4 T2001 H16 K=V=64 fwd+bwd: 856 us with zero-padded 128-wide tiles, 739 us so.
 //
 // All matrices between kernels are bf16 in the C8 blocked layout (tc_tiles.cuh) and move with
 // bulk asynchronous copies; all products run on tcgen05.mma with fp32 accumulation in TMEM.
