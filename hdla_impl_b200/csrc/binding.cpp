@@ -14,6 +14,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime.h>
 #include <dlfcn.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/grad_mode.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -466,23 +467,24 @@ Tensor norm_gate_op(const Tensor& x_, const Tensor& gate_, const Tensor& w_, dou
 }
 
 // ------------------------------------------------------------------------------------------ Python functions
-// Runs f without the GIL and turns C++ exceptions into Python ones; false if one is set.
+// Runs f without the GIL and turns C++ exceptions into Python ones as PyTorch's own bindings do: a Python exception
+// that travelled through C++ (raised by a saved-tensor hook, say: non-reentrant checkpointing ends its recomputation
+// with one) arrives as itself, an allocator's as torch.OutOfMemoryError.  False if an exception is set.
 template <typename F>
 bool guarded(F f) {
-    std::string what;
-    bool python = false, bad = false;
+    std::exception_ptr err;
+    bool python = false;
     PyThreadState* ts = PyEval_SaveThread();
     try {
         f();
     } catch (const PythonError&) {
-        bad = python = true;
-    } catch (const std::exception& e) {
-        bad = true;
-        what = e.what();
+        python = true;
+    } catch (...) {
+        err = std::current_exception();
     }
     PyEval_RestoreThread(ts);
-    if (bad && !python) PyErr_SetString(PyExc_RuntimeError, what.c_str());
-    return !bad;
+    if (err) torch::translate_exception_to_python(err);
+    return !err && !python;
 }
 
 // A tensor argument of the ordinary case, or null; None is an undefined tensor where `optional`.

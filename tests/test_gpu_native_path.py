@@ -1,0 +1,93 @@
+"""GPU: the compiled host path of the entry points (csrc/binding.cpp) -- what happens around the kernels."""
+import pytest
+import torch
+from torch.utils.checkpoint import checkpoint
+
+from hdla_impl_b200.synthetic import make_inputs
+
+pytestmark = pytest.mark.gpu
+R = 2
+NAMES = ("q", "k", "v", "a", "b", "gk")
+
+
+@pytest.fixture(scope="module")
+def dev():
+    assert torch.cuda.is_available(), "these tests need a CUDA device"
+    return torch.device("cuda:0")
+
+
+def leaves(dev, dtype, B=1, T=100, H=2, D=64, seed=0):
+    x = make_inputs(B, T, H, D, D, R, seed=seed, dtype=dtype, gk_div=4.0)
+    return [x[n].to(dev).requires_grad_(True) for n in NAMES], x["do"].to(dev)
+
+
+def layer_leaves(dev, B=1, T=100, H=2, D=64):
+    g = torch.Generator().manual_seed(3)
+    rn = lambda *s: torch.randn(*s, generator=g)
+    x = [rn(B, T, H, D), rn(B, T, H, D), rn(B, T, H, D), torch.sigmoid(rn(B, T, H, 1)),
+         torch.nn.functional.logsigmoid(rn(B, T, H, D)) / 8, rn(B, T, H * D), 1 + 0.1 * rn(H * D)]
+    return [t.to(torch.bfloat16).to(dev).requires_grad_(True) for t in x], rn(B, T, H * D).to(torch.bfloat16).to(dev)
+
+
+def layer(q, k, v, beta, log_f, gate, weight):
+    from hdla_impl_b200.layer_ops import chunk_hdla_delta_rule, rms_norm_fused_gate
+    o, _ = chunk_hdla_delta_rule(q, k, v, beta, log_f, normalize_k=True)
+    return rms_norm_fused_gate(o.flatten(2), gate, weight)
+
+
+def chunk(*t):
+    import hdla_impl_b200 as HD
+    return HD.chunk_hrdplr_delta_rule(*t, R, output_final_state=True)[0]
+
+
+@pytest.mark.parametrize("what", ["fp32", "bf16", "layer", "operator of the layer"])
+def test_non_reentrant_checkpoint_of_the_operator(dev, what):
+    """The recomputation ends with an exception from the pack hook of the region's last saved tensor, here one of the
+    operator's (or the norm's); the same kernels run on the same inputs, so the gradients are equal bit for bit."""
+    if what.startswith("layer"):
+        x, do = layer_leaves(dev)
+        f = layer
+    elif what.startswith("operator"):
+        x, do = layer_leaves(dev)
+        x, do = x[:5], do.view(x[0].shape)
+        from hdla_impl_b200.layer_ops import chunk_hdla_delta_rule
+        f = lambda *t: chunk_hdla_delta_rule(*t, normalize_k=True)[0]
+    else:
+        x, do = leaves(dev, torch.float32 if what == "fp32" else torch.bfloat16)
+        f = chunk
+    plain = torch.autograd.grad(f(*x), x, do)
+    kept = torch.autograd.grad(checkpoint(f, *x, use_reentrant=False), x, do)
+    for a, b in zip(plain, kept):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("f", ["chunk", "norm"])
+def test_a_pack_hooks_exception_arrives_as_itself(dev, f):
+    class Mine(Exception):
+        pass
+
+    def pack(t):
+        raise Mine("from the hook")
+
+    x, _ = layer_leaves(dev) if f == "norm" else leaves(dev, torch.bfloat16)
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+        with pytest.raises(Mine, match="from the hook"):
+            if f == "norm":
+                from hdla_impl_b200.layer_ops import rms_norm_fused_gate
+                rms_norm_fused_gate(x[5], x[5], x[6])
+            else:
+                chunk(*x)
+
+
+def test_out_of_memory_arrives_as_such(dev):
+    x, _ = leaves(dev, torch.bfloat16, T=4096, H=8, D=128)
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(dev).total_memory
+    # the inputs are in place; the workspace (hundreds of megabytes here) does not fit into 32 more
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved(dev) + (32 << 20)) / total, dev)
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            chunk(*x)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0, dev)
+    chunk(*x)
