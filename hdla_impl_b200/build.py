@@ -47,7 +47,7 @@ def _stale() -> bool:
 
 
 def _binding_stale() -> bool:
-    deps = [BINDING_SRC, os.path.join(ROOT, "include", "hdla.h")]
+    deps = [BINDING_SRC, os.path.join(CSRC, "status_board.h"), os.path.join(ROOT, "include", "hdla.h")]
     return not os.path.exists(BINDING) or any(os.path.getmtime(f) > os.path.getmtime(BINDING) for f in deps)
 
 

@@ -24,7 +24,6 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <deque>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -34,6 +33,7 @@
 #include <vector>
 
 #include "../../include/hdla.h"
+#include "status_board.h"
 
 namespace {
 
@@ -115,117 +115,80 @@ PyObject* wrap(const Tensor& t) {
 // while the largest chunk decay seen on that device is above half the limit.  HDLA_STRICT=1 always waits;
 // HDLA_ASYNC_STATUS=1 never does (an overflow then raises at the next entry).
 //
-// Backward runs on autograd's own threads without the GIL, so the state has a lock of its own, which is not held
-// while an event is waited for or Python code runs.
-constexpr int kRing = 64;
+// A call that is captured into a graph posts nothing: its copy would land at every replay, when no caller waits for it
+// and the slot may be another call's.
+//
+// Backward runs on autograd's own threads without the GIL: the boards have locks of their own, which are not held while
+// an event is waited for or Python code runs.
 constexpr double kDecayLimit = 150.0;
-struct DevStatus {
-    int32_t (*host)[4] = nullptr;
-    cudaEvent_t ev[kRing];
-    int next = 0;
-    std::deque<int> pending;
-    double decay = NAN;                     // largest chunk decay seen; NAN: nothing seen yet
+struct Gpu {                                  // what status_board.h asks for
+    typedef cudaEvent_t Event;
+    typedef cudaStream_t Stream;
+    static int32_t* alloc_words(int slots) {
+        void* p = nullptr;
+        check_cuda(cudaHostAlloc(&p, static_cast<size_t>(slots) * 16, cudaHostAllocPortable), "status words");
+        return static_cast<int32_t*>(p);
+    }
+    static Event make_event(int dev) {
+        c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(dev));
+        cudaEvent_t e;
+        check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "status event");
+        return e;
+    }
+    static void copy(int32_t* dst, const void* src, Stream st) {
+        check_cuda(cudaMemcpyAsync(dst, src, 16, cudaMemcpyDeviceToHost, st), "status words");
+    }
+    static void record(Event e, Stream st) { check_cuda(cudaEventRecord(e, st), "status words"); }
+    static bool done(Event e) {
+        const cudaError_t r = cudaEventQuery(e);
+        if (r == cudaErrorNotReady) { cudaGetLastError(); return false; }
+        check_cuda(r, "status words");
+        return true;
+    }
+    static void wait(Event e) {
+        cudaError_t r;
+        if (PyGILState_Check()) {
+            Py_BEGIN_ALLOW_THREADS
+            r = cudaEventSynchronize(e);
+            Py_END_ALLOW_THREADS
+        } else {
+            r = cudaEventSynchronize(e);
+        }
+        check_cuda(r, "status words");
+    }
 };
-std::map<int, DevStatus> g_status;
+typedef hdla_host::StatusBoard<Gpu> Board;
+
+[[noreturn]] void status_fail(const int32_t* w) {
+    if (w[0])
+        throw std::runtime_error("libhdla: a device-side wait ran out (code " + std::to_string(w[0]) +
+                                 "); the results of that call are invalid");
+    throw std::runtime_error(
+        "libhdla: the total log decay of some chunk exceeds 150 in some channel, beyond what the bf16 tensor-core "
+        "pipeline represents; the results of that call are invalid. Set HDLA_FORCE_SIMT=1 to use the fp32 pipeline, "
+        "which has no such limit.");
+}
+std::map<int, Board> g_boards;                // by device; an entry stays where it is
 std::mutex g_mu;
 typedef std::unique_lock<std::mutex> Lock;
 
-DevStatus& status_of(int dev) {                               // (with g_mu held)
-    DevStatus& st = g_status[dev];
-    if (!st.host) {
-        void* p = nullptr;
-        check_cuda(cudaHostAlloc(&p, kRing * 16, cudaHostAllocPortable), "status words");
-        memset(p, 0, kRing * 16);
-        c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(dev));
-        for (auto& e : st.ev) check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "status event");
-        st.host = static_cast<int32_t(*)[4]>(p);
-    }
-    return st;
-}
-void note_decay(DevStatus& st, const int32_t* w) {
-    float seen;
-    memcpy(&seen, &w[2], 4);
-    if (seen == seen && !(st.decay > seen)) st.decay = seen;
-}
-std::string status_error(const int32_t* w) {
-    if (w[0])
-        return "libhdla: a device-side wait ran out (code " + std::to_string(w[0]) + "); the results of that call are invalid";
-    return "libhdla: the total log decay of some chunk exceeds 150 in some channel, beyond what the bf16 tensor-core "
-           "pipeline represents; the results of that call are invalid. Set HDLA_FORCE_SIMT=1 to use the fp32 pipeline, "
-           "which has no such limit.";
-}
-void wait_event(cudaEvent_t e) {                              // (without g_mu)
-    cudaError_t r;
-    if (PyGILState_Check()) {
-        Py_BEGIN_ALLOW_THREADS
-        r = cudaEventSynchronize(e);
-        Py_END_ALLOW_THREADS
-    } else {
-        r = cudaEventSynchronize(e);
-    }
-    check_cuda(r, "status words");
-}
-// Look at the posts that have landed (with `wait`, at all of them); throws if one reports a problem.
-void status_check(int dev, bool wait) {
+Board& board_of(int dev) {
     Lock lk(g_mu);
-    auto it = g_status.find(dev);
-    if (it == g_status.end()) return;
-    DevStatus& st = it->second;
-    if (wait) {
-        const std::deque<int> todo = st.pending;
-        lk.unlock();
-        for (int slot : todo) wait_event(st.ev[slot]);
-        lk.lock();
-    }
-    while (!st.pending.empty()) {
-        const int slot = st.pending.front();
-        const cudaError_t e = cudaEventQuery(st.ev[slot]);
-        if (e == cudaErrorNotReady) { cudaGetLastError(); break; }
-        check_cuda(e, "status words");
-        int32_t w[4];
-        memcpy(w, st.host[slot], 16);
-        st.pending.pop_front();
-        note_decay(st, w);
-        if (w[0] || w[1]) throw std::runtime_error(status_error(w));
-    }
+    return g_boards.try_emplace(dev, dev, status_fail).first->second;
 }
-int status_post(const void* ws, int dev, cudaStream_t stream, bool is_capturing) {
-    Lock lk(g_mu);
-    DevStatus& st = status_of(dev);
-    const int slot = st.next;
-    st.next = (slot + 1) % kRing;
-    while (!is_capturing && st.pending.size() >= kRing) {     // ring wrapped: the oldest copy finished long ago
-        cudaEvent_t oldest = st.ev[st.pending.front()];
-        lk.unlock();
-        wait_event(oldest);
-        status_check(dev, false);
-        lk.lock();
-    }
-    check_cuda(cudaMemcpyAsync(st.host[slot], ws, 16, cudaMemcpyDeviceToHost, stream), "status words");
-    if (is_capturing) return slot;                            // a captured copy lands at replay: there is nothing to query
-    check_cuda(cudaEventRecord(st.ev[slot], stream), "status words");
-    st.pending.push_back(slot);
-    lk.unlock();
-    if (env_is_1("HDLA_STRICT")) status_check(dev, true);
-    return slot;
+// Look at the words that have landed (with `wait`, at all of them); throws if one reports a problem.
+void status_check(int dev, bool wait) { board_of(dev).check(wait); }
+void status_post(const void* ws, int dev, cudaStream_t stream, bool is_capturing) {
+    if (is_capturing) return;
+    Board& board = board_of(dev);
+    board.publish(board.post(ws, stream));
+    if (env_is_1("HDLA_STRICT")) board.check(true);
 }
-bool overflow_plausible(int dev, bool is_capturing) {
-    if (env_is_1("HDLA_ASYNC_STATUS") || is_capturing) return false;
+bool overflow_plausible(Board& board) {
+    if (env_is_1("HDLA_ASYNC_STATUS")) return false;
     if (env_is_1("HDLA_STRICT")) return true;
-    Lock lk(g_mu);
-    const double decay = status_of(dev).decay;
+    const double decay = board.decay();
     return decay != decay || decay > 0.5 * kDecayLimit;
-}
-void wait_words(int dev, int slot, int32_t* w) {
-    Lock lk(g_mu);
-    DevStatus& st = status_of(dev);
-    lk.unlock();
-    wait_event(st.ev[slot]);
-    lk.lock();
-    memcpy(w, st.host[slot], 16);
-    for (auto it = st.pending.begin(); it != st.pending.end(); ++it)
-        if (*it == slot) { st.pending.erase(it); break; }
-    note_decay(st, w);
 }
 
 // ------------------------------------------------------------------------------------------ chunked operator
@@ -269,14 +232,16 @@ ChunkOut chunk_forward(const ChunkArgs& c, const Tensor& q, const Tensor& k, con
     if (want_ht) r.ht = dense({c.n_states, d.H, d.K, d.V}, at::kFloat, q.device());
     check(abi.chunk_fwd(&d, ptr(q), ptr(k), ptr(v), ptr(a), ptr(b), ptr(gk), static_cast<float>(c.scale), fptr(h0),
                         mptr(r.o), fptr(r.ht), mptr(r.ws), n, st), "hdla_chunk_fwd");
-    if (abi.uses_tensor_cores(&d)) {
-        const int slot = status_post(ptr(r.ws), dev, st, cap);
-        if (overflow_plausible(dev, cap)) {
+    if (abi.uses_tensor_cores(&d) && !cap) {
+        Board& board = board_of(dev);
+        if (overflow_plausible(board)) {
             int32_t w[4];
-            wait_words(dev, slot, w);
+            board.take(board.post(ptr(r.ws), st), w);
             // (the fp32 pipeline takes no packed batches: the caller's per-sequence path has to be used for such decays)
             if (w[1] && !w[0] && (c.cu.empty() || (d.flags & HDLA_FLAG_PARAM_AB))) throw DecayOverflow();
-            if (w[0] || w[1]) throw std::runtime_error(status_error(w));
+            if (w[0] || w[1]) status_fail(w);
+        } else {
+            status_post(ptr(r.ws), dev, st, cap);
         }
     }
     if (!keep_ws) r.ws = Tensor();
@@ -697,7 +662,7 @@ PyObject* py_norm_gate(PyObject*, PyObject* const* av, Py_ssize_t n) {
     return wrap(o);
 }
 
-// status functions: check(dev index, wait), post(workspace tensor) -> slot, decay(dev), set_decay(dev, x or None)
+// status functions: check(dev index or -1, wait), post(workspace tensor), decay(dev), set_decay(dev, x or None)
 PyObject* py_status_check(PyObject*, PyObject* const* av, Py_ssize_t n) {
     if (n != 2) { PyErr_SetString(PyExc_TypeError, "status_check(device index or -1, wait)"); return nullptr; }
     const long dev = PyLong_AsLong(av[0]);
@@ -707,7 +672,7 @@ PyObject* py_status_check(PyObject*, PyObject* const* av, Py_ssize_t n) {
             std::vector<int> devs;
             {
                 Lock lk(g_mu);
-                for (auto& e : g_status)
+                for (auto& e : g_boards)
                     if (dev < 0 || e.first == dev) devs.push_back(e.first);
             }
             for (int i : devs) status_check(i, wait != 0);
@@ -718,20 +683,19 @@ PyObject* py_status_check(PyObject*, PyObject* const* av, Py_ssize_t n) {
 PyObject* py_status_post(PyObject*, PyObject* ws) {
     const Tensor* t = arg(ws);
     if (!t || t->nbytes() < 16) { PyErr_SetString(PyExc_TypeError, "status_post takes a CUDA workspace"); return nullptr; }
-    int slot = -1;
     if (!guarded([&] {
             c10::cuda::CUDAGuard guard(t->device());
             const cudaStream_t st = c10::cuda::getCurrentCUDAStream(t->get_device()).stream();
-            slot = status_post(ptr(*t), t->get_device(), st, capturing(st));
+            status_post(ptr(*t), t->get_device(), st, capturing(st));
         }))
         return nullptr;
-    return PyLong_FromLong(slot);
+    Py_RETURN_NONE;
 }
 PyObject* py_decay(PyObject*, PyObject* dev) {
     const long i = PyLong_AsLong(dev);
     if (PyErr_Occurred()) return nullptr;
     double x = NAN;
-    if (!guarded([&] { Lock lk(g_mu); x = status_of((int)i).decay; })) return nullptr;
+    if (!guarded([&] { x = board_of((int)i).decay(); })) return nullptr;
     if (x != x) Py_RETURN_NONE;
     return PyFloat_FromDouble(x);
 }
@@ -740,7 +704,7 @@ PyObject* py_set_decay(PyObject*, PyObject* const* av, Py_ssize_t n) {
     const long i = PyLong_AsLong(av[0]);
     const double x = av[1] == Py_None ? NAN : PyFloat_AsDouble(av[1]);
     if (PyErr_Occurred()) return nullptr;
-    if (!guarded([&] { Lock lk(g_mu); status_of((int)i).decay = x; })) return nullptr;
+    if (!guarded([&] { board_of((int)i).set_decay(x); })) return nullptr;
     Py_RETURN_NONE;
 }
 

@@ -143,9 +143,9 @@ def check_status(dev=None, wait: bool = False) -> None:
     _lib.native().status_check(index, bool(wait))
 
 
-def _post_status(ws: torch.Tensor, dev) -> int:
-    """Enqueue the copy of the status words of the call that just used ``ws``; returns the ring slot."""
-    return _lib.native().status_post(ws)
+def _post_status(ws: torch.Tensor, dev) -> None:
+    """Enqueue the copy of the status words of the call that just used ``ws``."""
+    _lib.native().status_post(ws)
 
 
 def _alloc_ws(nbytes: int, device) -> torch.Tensor:
