@@ -25,8 +25,8 @@ PHASE_ALL, PHASE_PRE, PHASE_TRANSITION, PHASE_STATE, PHASE_POST = 0x00, 0x10, 0x
 
 EXPORTS = (
     "hdla_version", "hdla_last_error", "hdla_chunk_workspace_bytes", "hdla_chunk_fwd", "hdla_chunk_bwd",
-    "hdla_recurrent_fwd", "hdla_chunk_uses_tensor_cores", "hdla_chunk_fwd_noalloc", "hdla_noalloc_read_status",
-    "hdla_recurrent_read_status", "hdla_compose_states", "hdla_param_ab_fwd", "hdla_param_ab_bwd",
+    "hdla_recurrent_fwd", "hdla_chunk_uses_tensor_cores", "hdla_fp32_status_words", "hdla_chunk_fwd_noalloc",
+    "hdla_noalloc_read_status", "hdla_recurrent_read_status", "hdla_compose_states", "hdla_param_ab_fwd", "hdla_param_ab_bwd",
     "hdla_norm_gate_fwd", "hdla_norm_gate_bwd",
     # include/hdla_debug.h
     "hdla_kernel_launches", "hdla_timing_enable", "hdla_timing_report", "hdla_debug_tc_buffer",
@@ -92,6 +92,8 @@ def load() -> C.CDLL:
         lib.hdla_timing_report.argtypes = [C.c_char_p, C.c_size_t]
         lib.hdla_chunk_uses_tensor_cores.restype = C.c_int
         lib.hdla_chunk_uses_tensor_cores.argtypes = [dp]
+        lib.hdla_fp32_status_words.restype = C.c_int
+        lib.hdla_fp32_status_words.argtypes = [C.POINTER(vp)]
         lib.hdla_debug_tc_buffer.restype = C.c_int
         lib.hdla_debug_tc_buffer.argtypes = [dp, vp, C.c_char_p, vp, vp]
         lib.hdla_chunk_workspace_bytes.restype = C.c_size_t

@@ -93,6 +93,11 @@ int hdla_chunk_uses_tensor_cores(const HdlaDims* dims) {
     return tc_supported(*dims) ? 1 : 0;
 }
 
+int hdla_fp32_status_words(void** words) {
+    if (!words) return fail(HDLA_ERR_INVALID, "fp32_status_words: words is null");
+    return f32_status_words(words);
+}
+
 int hdla_chunk_fwd(const HdlaDims* dims, const void* q, const void* k, const void* v, const void* a, const void* b,
                    const void* gk, float scale, const float* h0, void* o, float* ht, void* workspace,
                    size_t workspace_bytes, void* cuda_stream) {

@@ -21,6 +21,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -43,6 +44,7 @@ using at::Tensor;
 struct Abi {
     decltype(&hdla_chunk_workspace_bytes) workspace_bytes;
     decltype(&hdla_chunk_uses_tensor_cores) uses_tensor_cores;
+    decltype(&hdla_fp32_status_words) fp32_status_words;
     decltype(&hdla_chunk_fwd) chunk_fwd;
     decltype(&hdla_chunk_bwd) chunk_bwd;
     decltype(&hdla_recurrent_fwd) recurrent_fwd;
@@ -168,16 +170,46 @@ typedef hdla_host::StatusBoard<Gpu> Board;
         "pipeline represents; the results of that call are invalid. Set HDLA_FORCE_SIMT=1 to use the fp32 pipeline, "
         "which has no such limit.");
 }
-std::map<int, Board> g_boards;                // by device; an entry stays where it is
+struct DeviceState {
+    Board board;
+    std::atomic<unsigned> fp32_calls{0};
+    explicit DeviceState(int dev) : board(dev, status_fail) {}
+};
+std::map<int, DeviceState> g_devices;         // by device; an entry stays where it is
 std::mutex g_mu;
 typedef std::unique_lock<std::mutex> Lock;
 
-Board& board_of(int dev) {
+DeviceState& state_of(int dev) {
     Lock lk(g_mu);
-    return g_boards.try_emplace(dev, dev, status_fail).first->second;
+    return g_devices.try_emplace(dev, dev).first->second;
+}
+Board& board_of(int dev) { return state_of(dev).board; }
+
+// The fp32 pipeline's kernels have one set of words per device, written only when a wait has run out.  A training step there
+// can take less time than copying words after every call would: every kFp32Every-th call posts them, and so does a check
+// that waits.
+constexpr unsigned kFp32Every = 64;
+void fp32_post(int dev, cudaStream_t stream) {
+    void* words = nullptr;
+    check(abi.fp32_status_words(&words), "hdla_fp32_status_words");
+    Board& board = board_of(dev);
+    board.publish(board.post(words, stream));
 }
 // Look at the words that have landed (with `wait`, at all of them); throws if one reports a problem.
-void status_check(int dev, bool wait) { board_of(dev).check(wait); }
+void status_check(int dev, bool wait) {
+    if (wait && state_of(dev).fp32_calls != 0) {
+        c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(dev));
+        check_cuda(cudaDeviceSynchronize(), "status words");
+        fp32_post(dev, c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(dev)).stream());
+    }
+    board_of(dev).check(wait);
+}
+void fp32_called(int dev, cudaStream_t stream, bool is_capturing) {
+    if (is_capturing) return;
+    const unsigned calls = ++state_of(dev).fp32_calls;
+    if (env_is_1("HDLA_STRICT")) status_check(dev, true);
+    else if (calls % kFp32Every == 0) fp32_post(dev, stream);
+}
 void status_post(const void* ws, int dev, cudaStream_t stream, bool is_capturing) {
     if (is_capturing) return;
     Board& board = board_of(dev);
@@ -232,9 +264,9 @@ ChunkOut chunk_forward(const ChunkArgs& c, const Tensor& q, const Tensor& k, con
     if (want_ht) r.ht = dense({c.n_states, d.H, d.K, d.V}, at::kFloat, q.device());
     check(abi.chunk_fwd(&d, ptr(q), ptr(k), ptr(v), ptr(a), ptr(b), ptr(gk), static_cast<float>(c.scale), fptr(h0),
                         mptr(r.o), fptr(r.ht), mptr(r.ws), n, st), "hdla_chunk_fwd");
-    if (abi.uses_tensor_cores(&d) && !cap) {
+    if (abi.uses_tensor_cores(&d)) {
         Board& board = board_of(dev);
-        if (overflow_plausible(board)) {
+        if (!cap && overflow_plausible(board)) {
             int32_t w[4];
             board.take(board.post(ptr(r.ws), st), w);
             // (the fp32 pipeline takes no packed batches: the caller's per-sequence path has to be used for such decays)
@@ -243,6 +275,8 @@ ChunkOut chunk_forward(const ChunkArgs& c, const Tensor& q, const Tensor& k, con
         } else {
             status_post(ptr(r.ws), dev, st, cap);
         }
+    } else {
+        fp32_called(dev, st, cap);
     }
     if (!keep_ws) r.ws = Tensor();
     return r;
@@ -274,6 +308,7 @@ ChunkGrads chunk_backward(const ChunkArgs& c, const Tensor& q, const Tensor& k, 
                         ptr(d_o), fptr(dht), mptr(g.dq), mptr(g.dk), mptr(g.dv), mptr(g.da), mptr(g.db), mptr(g.dgk),
                         fptr(g.dh0), mptr(ws), static_cast<size_t>(ws.numel()), st), "hdla_chunk_bwd");
     if (abi.uses_tensor_cores(&d)) status_post(ptr(ws), dev, st, cap);
+    else fp32_called(dev, st, cap);
     return g;
 }
 
@@ -672,7 +707,7 @@ PyObject* py_status_check(PyObject*, PyObject* const* av, Py_ssize_t n) {
             std::vector<int> devs;
             {
                 Lock lk(g_mu);
-                for (auto& e : g_boards)
+                for (auto& e : g_devices)
                     if (dev < 0 || e.first == dev) devs.push_back(e.first);
             }
             for (int i : devs) status_check(i, wait != 0);
@@ -716,6 +751,7 @@ PyObject* py_bind(PyObject*, PyObject* const* av, Py_ssize_t n) {
     if (!guarded([&] {
             look_up(h, "hdla_chunk_workspace_bytes", abi.workspace_bytes);
             look_up(h, "hdla_chunk_uses_tensor_cores", abi.uses_tensor_cores);
+            look_up(h, "hdla_fp32_status_words", abi.fp32_status_words);
             look_up(h, "hdla_chunk_bwd", abi.chunk_bwd);
             look_up(h, "hdla_norm_gate_fwd", abi.norm_gate_fwd);
             look_up(h, "hdla_norm_gate_bwd", abi.norm_gate_bwd);

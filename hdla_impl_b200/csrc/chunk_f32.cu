@@ -33,6 +33,26 @@ namespace {
 constexpr int CT = 16, M2 = 32, RR = 48;     // tokens of a tile, low-rank rows, stacked rows ([q|k|v] 16 + [a|b|v2] 32)
 constexpr int VS = 16;                       // state columns of a scan CTA
 
+// Status words of these kernels (include/hdla.h, hdla_fp32_status_words), one set per device: they are only written when a
+// time-limited wait has run out.  (Words in the workspace, copied out after every call, cost 13 us of a training step of
+// 107.)
+__device__ int g_f32_status[4] = {0, 0, 0x7fc00000, 0};
+
+// Waits with a limit and records `code` if it runs out; the waits after one that ran out have a shorter limit, so that a
+// kernel whose copies never arrive ends.  (Out of line: with the flag carried through the kernels B2 T1000 H8 K=V=128 took
+// 652 us instead of 639.)
+__device__ __noinline__ void wait_or_record(uint64_t* bar, uint32_t parity, int code) {
+    const bool lost = *reinterpret_cast<volatile int*>(&g_f32_status[0]) != 0;
+    if (!sm100::mbar_wait(bar, parity, lost ? 200000 : sm100::kWaitBudgetNs)) atomicExch(&g_f32_status[0], code);
+}
+__device__ __forceinline__ void wait_copy(uint64_t* bar, uint32_t parity, int code) {
+    if (!sm100::mbar_try_wait(bar, parity)) wait_or_record(bar, parity, code);
+}
+// before a CTA leaves: copies that were late when they were waited for have arrived, or are waited for once more
+__device__ __forceinline__ void wait_late(uint64_t* bar, uint32_t parity) {
+    if (*reinterpret_cast<volatile int*>(&g_f32_status[0]) != 0) wait_or_record(bar, parity, g_f32_status[0]);
+}
+
 // ------------------------------------------------------------------------------------------ workspace
 // Per tile, padded to KP x VP channels: a record [WQ | KB | decay | A2 | M | Aak] with WQ = [w; qg], KB = [kg; bg] (48 x KP),
 // A2 = [Aqk | Aqb] (16 x 48); UV = [v; u, replaced by v2] (48 x VP); state checkpoints; backward: dv2, dS, shares of dgl.
@@ -322,7 +342,6 @@ struct ScanP {
     void* o;                     // fwd, may be null
     int T, H, K, V, VP, NT, dt, nslice, save;
     long long rec_floats;
-    int* status;
 };
 
 template <int KP>
@@ -415,7 +434,7 @@ __global__ void __launch_bounds__(128) f32_scan_kernel(ScanP p) {
             if (REV) st4(p.dE + (size_t)g * KP * p.VP + at, S[0][c], S[1][c], S[2][c], S[3][c]);
             else if (p.save) st4(p.h + ((size_t)bh * (p.NT + 1) + n) * KP * p.VP + at, S[0][c], S[1][c], S[2][c], S[3][c]);
         }
-        if (!sm100::mbar_wait(&s.bar[it & 1], (it >> 1) & 1) && p.status) atomicExch(p.status, 1);
+        wait_copy(&s.bar[it & 1], (it >> 1) & 1, 90 + REV);
         // row product over the state's rows: fwd [w; qg] S, rev bg dS
         f2 acc[NA][4];
 #pragma unroll
@@ -539,6 +558,8 @@ __global__ void __launch_bounds__(128) f32_scan_kernel(ScanP p) {
         __syncthreads();                         // state, vv and this record buffer are free / complete
         if (tid == 0 && it + 2 < p.NT) request(it + 2);
     }
+    if (tid == 0)
+        for (int it = max(p.NT - 2, 0); it < p.NT; ++it) wait_late(&s.bar[it & 1], (it >> 1) & 1);
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -604,7 +625,7 @@ __global__ void __launch_bounds__(256, KP == 128 ? 1 : 2) f32_tile_bwd_kernel(Ti
         st4(&s.Y[i][c], x[0], x[1], x[2], x[3]);
     }
     for (int e = tid; e < M2 * M2; e += 256) s.M[e / M2][e % M2] = rM[e];
-    sm100::mbar_wait(&s.bar, 0);
+    wait_copy(&s.bar, 0, 92);
     __syncthreads();
     {   // dP = M^T dv2, in place
         constexpr int VG = VP / 4, NR = M2 * VG / 256;
@@ -829,6 +850,7 @@ __global__ void __launch_bounds__(256, KP == 128 ? 1 : 2) f32_tile_bwd_kernel(Ti
         for (int c = 0; c < CPT; ++c) x[c] = D[i][ch + c] - dge[t][c];
         if (i < valid) st_row<CPT>(x, p.dgk, (((size_t)b * p.T + t0 + i) * p.H + h) * p.K, ch, p.K, p.gdt, p.vec_k);
     }
+    if (tid == 0) wait_late(&s.bar, 0);
 }
 
 // ------------------------------------------------------------------------------------------ host side
@@ -896,6 +918,12 @@ int bwd(const HdlaDims& d, const F32Plan& pl, const TileP& tp, ScanP sp, cudaStr
 }
 
 }  // namespace
+
+int f32_status_words(void** words) {
+    const cudaError_t e = cudaGetSymbolAddress(words, g_f32_status);
+    if (e != cudaSuccess) return fail(HDLA_ERR_CUDA, "fp32 status words: %s", cudaGetErrorString(e));
+    return HDLA_OK;
+}
 
 // Rank 2, head dims up to 128; other problems stay on the general kernels of chunk_simt.cu.
 bool f32_supported(const HdlaDims& d) {

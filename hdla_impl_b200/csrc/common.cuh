@@ -107,6 +107,7 @@ int simt_chunk_bwd(const HdlaDims& d, const void* q, const void* k, const void* 
 // fp32 pipeline for rank 2 and head dims up to 128, chunk_f32.cu
 bool f32_supported(const HdlaDims& d);
 size_t f32_workspace_floats(const HdlaDims& d, int with_backward);
+int f32_status_words(void** words);
 int f32_chunk_fwd(const HdlaDims& d, const void* q, const void* k, const void* v, const void* a, const void* b,
                   const void* gk, float scale, const float* h0, void* o, float* ht, float* ws, size_t ws_floats,
                   bool need_o, cudaStream_t st);

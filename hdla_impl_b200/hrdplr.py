@@ -138,7 +138,7 @@ def _status_state(dev) -> _DecayHistory:
 
 
 def check_status(dev=None, wait: bool = False) -> None:
-    """Raise if an earlier bf16 call on ``dev`` reported a problem. ``wait`` synchronises first."""
+    """Raise if an earlier call on ``dev`` reported a problem. ``wait`` synchronises first."""
     index = -1 if dev is None else (dev.index if isinstance(dev, torch.device) else int(dev))
     _lib.native().status_check(index, bool(wait))
 

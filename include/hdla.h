@@ -27,7 +27,7 @@
 extern "C" {
 #endif
 
-#define HDLA_VERSION 102
+#define HDLA_VERSION 103
 
 #if defined(__GNUC__)
 #define HDLA_API __attribute__((visibility("default")))
@@ -149,6 +149,12 @@ HDLA_API int hdla_chunk_uses_tensor_cores(const HdlaDims* dims);
  * Callers read them after the stream has finished the call (hdla_chunk_fwd_noalloc, which has no caller
  * workspace: hdla_noalloc_read_status).  Every device-side wait is bounded in time (2 s on the GPU's
  * nanosecond timer), so a kernel always returns. */
+
+/* The fp32 pipeline of rank-2 problems (K, V <= 128) has time-limited waits too, but no status words in its workspace: its
+ * kernels write to words of their own, one set per device, and only when a wait has run out.  Stores their address on the
+ * current device (device memory, the three words above; word 0 stays non-zero once some call's wait ran out in this
+ * process, word 1 is 0 and word 2 a NaN).  No counterpart in the reference. */
+HDLA_API int hdla_fp32_status_words(void** words);
 
 /* Chunked forward.  Replaces chunk_hrdplr_fwd (HRDPLR/hrdplr.py:25-99), i.e. the stage
  * sequence cumsum -> intra-chunk A matrices -> (I-Aab)^-1 and w/u -> state scan -> output.

@@ -91,3 +91,51 @@ def test_out_of_memory_arrives_as_such(dev):
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0, dev)
     chunk(*x)
+
+
+_FP32_WAIT = """
+import ctypes as C, sys, torch
+sys.path.insert(0, {root!r})
+import hdla_impl_b200 as HD
+from hdla_impl_b200 import _lib
+from hdla_impl_b200.synthetic import make_inputs
+dev = torch.device("cuda:0")
+x = make_inputs(1, 40, 2, 64, 64, 2, seed=0)
+args = [x[n].to(dev).requires_grad_(True) for n in ("q", "k", "v", "a", "b", "gk")]
+step = lambda: torch.autograd.grad(HD.chunk_hrdplr_delta_rule(*args, 2)[0], args, x["do"].to(dev))
+for _ in range(100):
+    step()
+HD.check_status(dev, wait=True)
+words = C.c_void_p()
+_lib.check(_lib.load().hdla_fp32_status_words(C.byref(words)), "hdla_fp32_status_words")
+_lib.check(_lib.load().hdla_debug_wait_timeout(words, C.c_uint64(1000000), _lib.stream_ptr(dev)), "hdla_debug_wait_timeout")
+def raised(f):
+    try:
+        f()
+    except RuntimeError as e:
+        assert "device-side wait ran out (code 99)" in str(e), e
+        return True
+    return False
+if {how!r} == "check":
+    assert raised(lambda: HD.check_status(dev, wait=True))
+else:
+    def calls():
+        for _ in range(64):
+            step()
+            torch.cuda.synchronize()
+    assert raised(calls)
+print("reported")
+"""
+
+
+@pytest.mark.parametrize("how", ["check", "calls"])
+def test_fp32_pipeline_reports_a_wait_that_ran_out(dev, how):
+    """With the fp32 pipeline's words as a kernel's run-out wait leaves them, a check that waits raises, and so does one of
+    the next 64 steps.  (The words keep the report for as long as the process lives: a process of its own.)"""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _FP32_WAIT.format(root=root, how=how)], stdout=subprocess.PIPE,
+                       stderr=subprocess.STDOUT, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("reported"), r.stdout

@@ -124,6 +124,16 @@ def test_tensor_core_pipeline_selection():
     assert uses(2, 256, 2, 64, 64, 2, 64, 1, 0, _lib.PHASE_PRE) == 0      # phased calls need the full 128 x 128
 
 
+def test_no_device_side_wait_is_dropped():
+    """The result of a time-limited wait is used wherever a kernel waits (before a CTA leaves, a second wait for what is late
+    has nothing left to report)."""
+    csrc = os.path.join(ROOT, "hdla_impl_b200", "csrc")
+    for name in sorted(os.listdir(csrc)):
+        for line in open(os.path.join(csrc, name)):
+            if re.match(r"\s*(sm100::)?mbar_wait(_backoff)?\(", line):
+                raise AssertionError(f"{name}: {line.strip()}")
+
+
 def test_in_operator_parametrisation_flag_is_sized_and_gated_on_the_host():
     """HDLA_FLAG_PARAM_AB: the backward workspace grows by the two gradient tensors [B, 2T, H, K] bf16 that stay inside
     the library, the forward workspace does not change, and problems outside the tensor-core pipeline are refused."""
