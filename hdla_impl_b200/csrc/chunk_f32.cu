@@ -925,10 +925,20 @@ int f32_status_words(void** words) {
     return HDLA_OK;
 }
 
-// Rank 2, head dims up to 128; other problems stay on the general kernels of chunk_simt.cu.
+// Rank 2, head dims up to 128; other problems stay on the general kernels of chunk_simt.cu.  So do large ones that would
+// need more memory here than there: heads of a few channels, padded to 64, with a requested chunk of 16 (5.5 KB per token
+// and head against 2.1 to 4.9 for K = V = 1 to 16; from 24 channels on, or with larger chunks, this pipeline needs less).
+// They would fit a device there and not here, which no gain in time makes up for; up to kAlwaysBytes, a small part of any
+// device that runs these kernels, the faster pipeline takes them (B4 T1024 H8 K = V = 16, chunk 16, fwd+bwd: 533 us in
+// 173 MB against 2324 us in 152 MB).
+constexpr size_t kAlwaysBytes = (size_t)4 << 30;
 bool f32_supported(const HdlaDims& d) {
     const F32Plan pl = make_f32_plan(d);
-    return d.R == 2 && d.K <= 128 && d.V <= 128 && pl.G < 0x7fffffffLL && (long long)pl.BH * pl.nslice < 0x7fffffffLL;
+    if (d.flags & kFlagGeneralKernels) return false;
+    if (!(d.R == 2 && d.K <= 128 && d.V <= 128 && pl.G < 0x7fffffffLL && (long long)pl.BH * pl.nslice < 0x7fffffffLL))
+        return false;
+    return (size_t)pl.total * sizeof(float) <= kAlwaysBytes ||
+           ((size_t)pl.total <= simt_workspace_floats(d, 1) && (size_t)pl.total_fwd <= simt_workspace_floats(d, 0));
 }
 size_t f32_workspace_floats(const HdlaDims& d, int with_backward) {
     const F32Plan pl = make_f32_plan(d);

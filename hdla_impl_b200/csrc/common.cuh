@@ -104,6 +104,9 @@ int simt_chunk_bwd(const HdlaDims& d, const void* q, const void* k, const void* 
                    const void* gk, float scale, const float* h0, const void* d_o, const float* dht, void* dq,
                    void* dk, void* dv, void* da, void* db, void* dgk, float* dh0, float* ws, cudaStream_t st);
 
+// internal bit of HdlaDims.flags: not the pipeline for rank 2 below, whatever the problem (noalloc.cu)
+constexpr int kFlagGeneralKernels = 1 << 30;
+
 // fp32 pipeline for rank 2 and head dims up to 128, chunk_f32.cu
 bool f32_supported(const HdlaDims& d);
 size_t f32_workspace_floats(const HdlaDims& d, int with_backward);

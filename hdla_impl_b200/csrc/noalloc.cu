@@ -48,8 +48,15 @@ extern "C" int hdla_chunk_fwd_noalloc(const HdlaDims* dims, const void* q, const
                                       void* o, float* ht, void* cuda_stream) {
     int rc = hdla::check_common(dims, true);                    // null or malformed dims: HDLA_ERR_INVALID / _UNSUPPORTED
     if (rc != HDLA_OK) return rc;
-    const size_t need = hdla_chunk_workspace_bytes(dims, 0);
+    HdlaDims d = *dims;
+    size_t need = hdla_chunk_workspace_bytes(&d, 0);
     if (need == 0) return HDLA_ERR_UNSUPPORTED;                 // hdla_last_error() already says why
+    if (need > (size_t)HDLA_NOALLOC_SCRATCH_BYTES) {            // heads of a few channels need less on the general kernels
+        HdlaDims general = d;
+        general.flags |= hdla::kFlagGeneralKernels;
+        const size_t n = hdla_chunk_workspace_bytes(&general, 0);
+        if (n != 0 && n <= (size_t)HDLA_NOALLOC_SCRATCH_BYTES) { d = general; need = n; }
+    }
     if (need > (size_t)HDLA_NOALLOC_SCRATCH_BYTES)
         return hdla::fail(HDLA_ERR_WORKSPACE,
                           "hdla_chunk_fwd_noalloc: this problem needs %zu bytes of scratch but the built-in scratch "
@@ -62,7 +69,7 @@ extern "C" int hdla_chunk_fwd_noalloc(const HdlaDims* dims, const void* q, const
     // except the leading status block, which must start at zero.
     cudaError_t e = cudaMemsetAsync(scratch, 0, 256, static_cast<cudaStream_t>(cuda_stream));
     if (e != cudaSuccess) return hdla::fail(HDLA_ERR_CUDA, "noalloc: clearing the status block: %s", cudaGetErrorString(e));
-    return hdla_chunk_fwd(dims, q, k, v, a, b, gk, scale, h0, o, ht, scratch, (size_t)HDLA_NOALLOC_SCRATCH_BYTES,
+    return hdla_chunk_fwd(&d, q, k, v, a, b, gk, scale, h0, o, ht, scratch, (size_t)HDLA_NOALLOC_SCRATCH_BYTES,
                           cuda_stream);
 }
 

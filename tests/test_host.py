@@ -124,6 +124,27 @@ def test_tensor_core_pipeline_selection():
     assert uses(2, 256, 2, 64, 64, 2, 64, 1, 0, _lib.PHASE_PRE) == 0      # phased calls need the full 128 x 128
 
 
+@pytest.mark.parametrize("K,V,chunk,fwd_mb,both_mb", [
+    (1, 1, 16, 58, 131), (8, 8, 16, 101, 210), (16, 16, 16, 152, 304), (24, 24, 16, 205, 402), (8, 8, 64, 256, 568),
+    (65, 65, 16, 509, 969), (128, 128, 64, 1041, 2019)])
+def test_large_fp32_problems_do_not_need_more_memory_than_on_the_general_kernels(K, V, chunk, fwd_mb, both_mb):
+    """The general kernels' plan for 65536 (token, head) pairs takes the given megabytes (rounded down).  Heads of a few
+    channels are padded to 64 in the rank-2 pipeline: what that makes larger must stay small (4 GB), and what fits the
+    built-in scratch with the general kernels must go on to be taken there."""
+    lib = _lib.load()
+    dims = lambda B, T: C.byref(_lib.HdlaDims(B, T, 8, K, V, 2, chunk, 0, 0, 0))
+    for B in (2, 16, 32, 64, 512):
+        for wb, mb in ((0, fwd_mb), (1, both_mb)):
+            n = lib.hdla_chunk_workspace_bytes(dims(B, 4096), wb)
+            assert 0 < n <= max(4 << 30, (mb + 1) * (B << 19))
+    fits = int(4096 * min(1.0, 2 * 63 / (fwd_mb + 1))) // 64 * 64       # tokens whose plan just fits 64 MB there
+    # (the size is looked at before the device: without one the call fails there, not for want of scratch)
+    any_ptr = C.c_void_p(256)
+    if not torch.cuda.is_available():
+        rc = lib.hdla_chunk_fwd_noalloc(dims(1, fits), *[any_ptr] * 6, 1.0, None, any_ptr, None, None)
+        assert rc != -3, _lib.last_error()
+
+
 def test_no_device_side_wait_is_dropped():
     """The result of a time-limited wait is used wherever a kernel waits (before a CTA leaves, a second wait for what is late
     has nothing left to report)."""
