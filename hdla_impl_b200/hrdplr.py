@@ -173,7 +173,8 @@ def _chunk_fwd(q, k, v, a, b, gk, scale, initial_state, output_final_state, RANK
     _lib.require_cuda(q, k, v, a, b, gk, initial_state)
     N = None if cu_seqlens is None else len(cu_seqlens) - 1
     _check_shapes(q, k, v, a, b, gk, RANK_AB, initial_state, N)
-    rest = (RANK_AB, float(scale), _plain(initial_state), output_final_state, chunk_size, cu_seqlens, bool(_keep_ws))
+    rest = (RANK_AB, float(scale), _state(initial_state), output_final_state,
+            _internal_chunk(q, v, RANK_AB, chunk_size), cu_seqlens, bool(_keep_ws))
     r = _lib.native().chunk(*[_plain(t) for t in (q, k, v, a, b, gk)], *rest)
     if r is NotImplemented:
         workspace_bytes(_dims(q, v, a, gk, RANK_AB, chunk_size, 0, cu_seqlens), bool(_keep_ws))      # says why
@@ -184,6 +185,11 @@ def _chunk_fwd(q, k, v, a, b, gk, scale, initial_state, output_final_state, RANK
 def _plain(t):
     """The tensor itself, detached and without its subclass."""
     return t if t is None else t.detach().as_subclass(torch.Tensor)
+
+
+def _state(t):
+    """An initial state as the native path takes it: of a floating-point type (an integer one is converted)."""
+    return _plain(t) if t is None or t.is_floating_point() else _plain(t).to(torch.float32)
 
 
 class ChunkDPLRDeltaRuleFunction(torch.autograd.Function):
@@ -217,8 +223,9 @@ class ChunkDPLRDeltaRuleFunction(torch.autograd.Function):
         q, k, v, a, b, gk, initial_state = ctx.saved_tensors
         ws, ctx.ws = ctx.ws, None
         grads = _lib.native().chunk_backward(*[_plain(t) for t in (q, k, v, a, b, gk)], ctx.RANK_AB, float(ctx.scale),
-                                             _plain(initial_state), _plain(do), _plain(dht), ws, ctx.chunk_size,
-                                             ctx.cu_seqlens, ctx.force_simt)
+                                             _state(initial_state), _plain(do), _plain(dht), ws,
+                                             _internal_chunk(q, v, ctx.RANK_AB, ctx.chunk_size), ctx.cu_seqlens,
+                                             ctx.force_simt)
         dq, dk, dv, da, db, dgk, dh0 = grads
         if dh0 is not None and initial_state.dtype != torch.float32:
             dh0 = dh0.to(initial_state.dtype)

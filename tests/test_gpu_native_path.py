@@ -93,6 +93,27 @@ def test_out_of_memory_arrives_as_such(dev):
     chunk(*x)
 
 
+def test_integer_initial_state_and_any_chunk_size(dev):
+    """What the entry point took when Python checked its arguments: a state of an integer type is converted, and the
+    tensor-core pipeline, which runs at its own chunk, does not look at the chunk size asked for."""
+    import hdla_impl_b200 as HD
+    x, do = leaves(dev, torch.bfloat16)
+    h0 = torch.randint(-1, 2, (1, 2, 64, 64), generator=torch.Generator().manual_seed(1)).to(dev)
+
+    def run(h, c):
+        o, ht = HD.chunk_hrdplr_delta_rule(*x, R, initial_state=h, output_final_state=True, chunk_size=c)
+        return [o, ht, *torch.autograd.grad(o, x, do)]
+
+    want = run(h0.float(), 64)
+    for h, c in ((h0, 64), (h0.to(torch.int32), 64), (h0.float(), None), (h0, 0)):
+        for a, b in zip(run(h, c), want):
+            assert torch.equal(a, b), (h.dtype, c)
+    f32, _ = leaves(dev, torch.float32)
+    a = HD.chunk_hrdplr_delta_rule(*f32, R, initial_state=h0, output_final_state=True)
+    b = HD.chunk_hrdplr_delta_rule(*f32, R, initial_state=h0.float(), output_final_state=True)
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+
+
 _FP32_WAIT = """
 import ctypes as C, sys, torch
 sys.path.insert(0, {root!r})
