@@ -20,6 +20,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <atomic>
 #include <cmath>
@@ -96,6 +97,9 @@ Tensor f32_contiguous(const Tensor& t) { return t.defined() ? t.to(at::kFloat).c
 bool transforms_active() {        // functorch transforms wrap tensors; the Python route says that they are not supported
     return c10::impl::tls_local_dispatch_key_set().included_.has(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
 }
+// A tracer records the Python autograd functions as calls (inside which it may go on tracing); of what happens here it
+// would see nothing but tensors out of nowhere.
+bool tracing() { return torch::jit::tracer::isTracing(); }
 bool capturing(cudaStream_t st) {
     cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(st, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
@@ -587,7 +591,7 @@ PyObject* py_chunk(PyObject*, PyObject* const* av, Py_ssize_t n) {
     const bool bare = av[12] != Py_None, keep = av[12] == Py_True;
     const int want_ht = PyObject_IsTrue(av[9]);
     if (want_ht < 0) { PyErr_Clear(); NOT_MINE(); }
-    if (!chunk_call(av, av[10], av[11], x)) NOT_MINE();
+    if ((!bare && tracing()) || !chunk_call(av, av[10], av[11], x)) NOT_MINE();
     ChunkOut r;
     bool overflow = false;
     if (!guarded([&] {
@@ -642,7 +646,7 @@ PyObject* py_recurrent(PyObject*, PyObject* const* av, Py_ssize_t n) {
     if (n != 12) { PyErr_SetString(PyExc_TypeError, "recurrent takes 12 arguments"); return nullptr; }
     const Tensor *q = arg(av[0]), *k = arg(av[1]), *v = arg(av[2]), *a = arg(av[3]), *b = arg(av[4]), *gk = arg(av[5]),
                  *h0 = arg(av[8], true), *cu = arg(av[11], true);
-    if (!abi.recurrent_fwd || !q || !k || !v || !a || !b || !gk || !h0 || !cu || transforms_active()) NOT_MINE();
+    if (!abi.recurrent_fwd || !q || !k || !v || !a || !b || !gk || !h0 || !cu || transforms_active() || tracing()) NOT_MINE();
     if (needs_grad({q, k, v, a, b, gk, h0}) || q->dim() != 4 || v->dim() != 4) NOT_MINE();
     const int64_t B = q->size(0), T = q->size(1), H = q->size(2), K = q->size(3), V = v->size(3);
     const int64_t R = PyLong_AsLongLong(av[6]);
@@ -686,7 +690,7 @@ PyObject* py_recurrent(PyObject*, PyObject* const* av, Py_ssize_t n) {
 PyObject* py_norm_gate(PyObject*, PyObject* const* av, Py_ssize_t n) {
     if (n != 4) { PyErr_SetString(PyExc_TypeError, "norm_gate takes 4 arguments"); return nullptr; }
     const Tensor *x = arg(av[0]), *gate = arg(av[1]), *w = arg(av[2]);
-    if (!abi.norm_gate_fwd || !x || !gate || !w || transforms_active()) NOT_MINE();
+    if (!abi.norm_gate_fwd || !x || !gate || !w || transforms_active() || tracing()) NOT_MINE();
     const double eps = PyFloat_AsDouble(av[3]);
     if (PyErr_Occurred()) { PyErr_Clear(); NOT_MINE(); }
     if (dtype_code(*x) < 0 || x->dim() < 1 || x->numel() == 0 || gate->sizes() != x->sizes() || w->dim() != 1 ||

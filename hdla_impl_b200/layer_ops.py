@@ -66,6 +66,47 @@ def parameterize_a_b(beta: torch.Tensor, k: torch.Tensor, log_f: torch.Tensor) -
     return _ParamAB.apply(beta, k, log_f)
 
 
+class _DecayOverflow(Exception):
+    """A chunk's total log decay is beyond the bf16 tensor-core pipeline: the caller takes the two-call route."""
+
+
+class _ChunkHdla(torch.autograd.Function):
+    """Operator call with the in-operator a/b parametrisation, for arguments that need a Python autograd function (tensor
+    subclasses, tracing); gradients for q, k, v, beta, log_f and the state."""
+
+    @staticmethod
+    @_op.contiguous
+    @_op.autocast_custom_fwd
+    def forward(ctx, q, k, v, beta, log_f, scale, initial_state, output_final_state, cu_seqlens, normalize_k):
+        _lib.require_cuda(q, k, v, beta, log_f, initial_state)
+        keep = _op.save_workspace_default() and any(
+            isinstance(t, torch.Tensor) and t.requires_grad for t in (q, k, v, beta, log_f, initial_state))
+        ctx.flags, ctx.scale, ctx.cu_seqlens = (_lib.FLAG_NORM_K if normalize_k else 0), float(scale), cu_seqlens
+        ctx.beta_like = beta.shape, beta.dtype
+        beta = beta.to(q.dtype).contiguous()
+        r = _lib.native().chunk(*[_op._plain(t) for t in (q, k, v, beta)], None, _op._plain(log_f), ctx.flags, ctx.scale,
+                                _op._state(initial_state), output_final_state, 64, cu_seqlens, keep)
+        if r is None:
+            raise _DecayOverflow()
+        o, ht, ctx.ws, _ = r
+        ctx.save_for_backward(q, k, v, beta, log_f, initial_state)
+        return o, ht
+
+    @staticmethod
+    @_op.contiguous
+    @_op.autocast_custom_bwd
+    def backward(ctx, do, dht):
+        q, k, v, beta, log_f, initial_state = ctx.saved_tensors
+        ws, ctx.ws = ctx.ws, None
+        dq, dk, dv, dbeta, _, dlog_f, dh0 = _lib.native().chunk_backward(
+            *[_op._plain(t) for t in (q, k, v, beta)], None, _op._plain(log_f), ctx.flags, ctx.scale,
+            _op._state(initial_state), _op._plain(do), _op._plain(dht), ws, 64, ctx.cu_seqlens, False)
+        if dh0 is not None and initial_state.dtype != torch.float32:
+            dh0 = dh0.to(initial_state.dtype)
+        shape, dtype = ctx.beta_like
+        return dq, dk, dv, dbeta.view(shape).to(dtype), dlog_f, None, dh0, None, None, None
+
+
 _warned_two_call = False
 L2_NORM_EPS = 1e-5      # of the reference's l2_norm (HRDPLR/normalizations/l2_norm.py:4)
 
@@ -113,6 +154,12 @@ def chunk_hdla_delta_rule(
     if offsets is not None and (q.shape[0] != 1 or offsets[0] != 0 or offsets[-1] != T
                                 or any(y < x for x, y in zip(offsets, offsets[1:]))):
         raise ValueError(f"cu_seqlens {offsets} must rise from 0 to T={T} in a batch of one")
+    if r is not None and (_op._packed_supported(q, v, 2) and q.dtype == k.dtype == v.dtype
+                          and log_f.dtype in (torch.bfloat16, torch.float32)):
+        try:
+            return _ChunkHdla.apply(q, k, v, beta, log_f, scale, initial_state, output_final_state, offsets, normalize_k)
+        except _DecayOverflow:
+            r = None
     if r is None and not _warned_two_call:
         _warned_two_call = True
         warnings.warn("hdla_impl_b200: a chunk's total log decay exceeds what the bf16 tensor-core pipeline "

@@ -114,6 +114,59 @@ def test_integer_initial_state_and_any_chunk_size(dev):
     assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
 
 
+def recurrent(*t):
+    import hdla_impl_b200 as HD
+    return HD.fused_recurrent_dplr_delta_rule(*t, R, output_final_state=True)
+
+
+@pytest.mark.parametrize("what", ["chunk fp32", "chunk bf16", "recurrent", "layer"])
+def test_a_traced_call_runs_on_its_own_inputs(dev, what):
+    """torch.jit.trace records the operators as calls: the traced function computes on what it is given, not what it was
+    traced with (equal bit for bit to the direct call: the same kernels)."""
+    if what == "layer":
+        f, (x, _) = layer, layer_leaves(dev)
+    else:
+        f = recurrent if what == "recurrent" else chunk
+        x, _ = leaves(dev, torch.float32 if what == "chunk fp32" else torch.bfloat16)
+    x = [t.detach() for t in x]
+    y = [t.flip(1) if t.dim() > 1 else t for t in x]
+    traced = torch.jit.trace(f, tuple(x), check_trace=False)
+    for inputs in (y, x):
+        got, want = traced(*inputs), f(*inputs)
+        for a, b in zip(got if isinstance(got, tuple) else (got,), want if isinstance(want, tuple) else (want,)):
+            assert torch.equal(a, b)
+
+
+class Sub(torch.Tensor):
+    """A tensor subclass without behaviour of its own: such tensors take the Python autograd functions."""
+
+
+@pytest.mark.parametrize("what", ["chunk fp32", "chunk bf16", "recurrent", "layer"])
+def test_tensor_subclasses_take_the_same_kernels(dev, what):
+    from hdla_impl_b200 import _lib
+    if what == "layer":
+        f, (x, do) = layer, layer_leaves(dev)
+    else:
+        f = recurrent if what == "recurrent" else chunk
+        x, do = leaves(dev, torch.float32 if what == "chunk fp32" else torch.bfloat16)
+    x = [t.detach() for t in x]
+
+    def run(ts):
+        n0 = _lib.kernel_launches()
+        if what == "recurrent":
+            out = list(f(*ts))
+        else:
+            ts = [t.requires_grad_(True) for t in ts]
+            o = f(*ts)
+            out = [o, *torch.autograd.grad(o, ts, do)]
+        return out, _lib.kernel_launches() - n0
+
+    (want, n_want), (got, n_got) = run([t.clone() for t in x]), run([t.clone().as_subclass(Sub) for t in x])
+    assert n_got == n_want
+    for a, b in zip(got, want):
+        assert torch.equal(a.as_subclass(torch.Tensor), b)
+
+
 _FP32_WAIT = """
 import ctypes as C, sys, torch
 sys.path.insert(0, {root!r})
