@@ -351,6 +351,30 @@ bool needs_grad(std::initializer_list<const Tensor*> ts) {
     return false;
 }
 
+// A saved contiguous tensor.  What a saved-tensor hook hands back is looked at before a kernel gets its pointer.
+struct Saved {
+    SavedVariable var;
+    std::vector<int64_t> size;
+    at::ScalarType type = at::kFloat;
+    at::Device device = at::kCPU;
+    bool defined = false;
+
+    void save(const Tensor& t) {
+        var = SavedVariable(t, false);
+        defined = t.defined();
+        if (defined) { size = t.sizes().vec(); type = t.scalar_type(); device = t.device(); }
+    }
+    Tensor get(const char* node) const {
+        const Tensor t = var.unpack();
+        if (!defined) return t;
+        if (!t.defined() || t.device() != device || t.scalar_type() != type || t.sizes() != at::IntArrayRef(size) ||
+            t.layout() != at::kStrided)
+            throw std::runtime_error(std::string(node) + ": a saved-tensor hook returned a tensor of another shape, type or "
+                                     "device than the saved one's");
+        return t.contiguous();
+    }
+};
+
 template <typename NodeT>
 std::shared_ptr<NodeT> make_node() { return std::shared_ptr<NodeT>(new NodeT(), torch::autograd::deleteNode); }
 
@@ -358,7 +382,7 @@ std::shared_ptr<NodeT> make_node() { return std::shared_ptr<NodeT>(new NodeT(), 
 // the workspace gone -- the backward kernels write into it -- and recomputes what it held.
 struct ChunkNode : torch::autograd::Node {
     ChunkArgs args;
-    SavedVariable q, k, v, a, b, gk, h0;
+    Saved q, k, v, a, b, gk, h0;
     Tensor ws;
     bool force_simt = false;
     at::ScalarType a_type, h0_type;
@@ -366,7 +390,7 @@ struct ChunkNode : torch::autograd::Node {
     std::string name() const override { return "HdlaChunkBackward"; }
     void release_variables() override {
         std::lock_guard<std::mutex> lock(mutex_);
-        for (SavedVariable* s : {&q, &k, &v, &a, &b, &gk, &h0}) s->reset_data();
+        for (Saved* s : {&q, &k, &v, &a, &b, &gk, &h0}) s->var.reset_data();
         ws = Tensor();
     }
     variable_list apply(variable_list&& grads) override {
@@ -375,9 +399,9 @@ struct ChunkNode : torch::autograd::Node {
         if (!grads[0].defined() && (grads.size() < 2 || !grads[1].defined())) return variable_list(7);
         Tensor w = std::move(ws);
         ws = Tensor();
-        ChunkGrads g = chunk_backward(args, q.unpack(), k.unpack(), v.unpack(), a.unpack(), b.unpack(), gk.unpack(),
-                                      h0.unpack(), grads[0], grads.size() > 1 ? grads[1] : Tensor(), std::move(w),
-                                      force_simt);
+        const char* me = "HdlaChunkBackward";
+        ChunkGrads g = chunk_backward(args, q.get(me), k.get(me), v.get(me), a.get(me), b.get(me), gk.get(me), h0.get(me),
+                                      grads[0], grads.size() > 1 ? grads[1] : Tensor(), std::move(w), force_simt);
         if (g.da.scalar_type() != a_type) g.da = g.da.to(a_type);
         if (g.dh0.defined() && g.dh0.scalar_type() != h0_type) g.dh0 = g.dh0.to(h0_type);
         return {g.dq, g.dk, g.dv, g.da, g.db, g.dgk, g.dh0};
@@ -399,9 +423,8 @@ std::pair<Tensor, Tensor> chunk_op(const ChunkArgs& args, const Tensor& q_, cons
         if (grad) {
             node = make_node<ChunkNode>();
             node->args = args;
-            node->q = SavedVariable(q, false); node->k = SavedVariable(k, false); node->v = SavedVariable(v, false);
-            node->a = SavedVariable(a, false); node->b = SavedVariable(b, false); node->gk = SavedVariable(gk, false);
-            node->h0 = SavedVariable(h0, false);
+            node->q.save(q); node->k.save(k); node->v.save(v); node->a.save(a); node->b.save(b); node->gk.save(gk);
+            node->h0.save(h0);
             node->ws = r.ws;
             node->force_simt = r.forced_simt;
             node->a_type = a_.scalar_type();
@@ -417,20 +440,21 @@ std::pair<Tensor, Tensor> chunk_op(const ChunkArgs& args, const Tensor& q_, cons
 }
 
 struct NormGateNode : torch::autograd::Node {
-    SavedVariable x, gate, w;
+    Saved x, gate, w;
     double eps = 0;
     at::ScalarType gate_type, w_type;
 
     std::string name() const override { return "HdlaNormGateBackward"; }
     void release_variables() override {
         std::lock_guard<std::mutex> lock(mutex_);
-        x.reset_data(); gate.reset_data(); w.reset_data();
+        x.var.reset_data(); gate.var.reset_data(); w.var.reset_data();
     }
     variable_list apply(variable_list&& grads) override {
         std::lock_guard<std::mutex> lock(mutex_);
         at::NoGradGuard no_grad;
         if (!grads[0].defined()) return variable_list(3);
-        const Tensor xs = x.unpack(), gs = gate.unpack(), ws = w.unpack();
+        const char* me = "HdlaNormGateBackward";
+        const Tensor xs = x.get(me), gs = gate.get(me), ws = w.get(me);
         c10::cuda::CUDAGuard guard(xs.device());
         const Tensor d_o = grads[0].to(xs.scalar_type()).contiguous();
         Tensor dx = dense_like(xs), dg = dense_like(gs);
@@ -459,7 +483,7 @@ Tensor norm_gate_op(const Tensor& x_, const Tensor& gate_, const Tensor& w_, dou
                                 c10::cuda::getCurrentCUDAStream(x.get_device()).stream()), "hdla_norm_gate_fwd");
         if (grad) {
             node = make_node<NormGateNode>();
-            node->x = SavedVariable(x, false); node->gate = SavedVariable(gate, false); node->w = SavedVariable(w, false);
+            node->x.save(x); node->gate.save(gate); node->w.save(w);
             node->eps = eps; node->gate_type = gate_.scalar_type(); node->w_type = w_.scalar_type();
         }
     }

@@ -167,6 +167,34 @@ def test_tensor_subclasses_take_the_same_kernels(dev, what):
         assert torch.equal(a.as_subclass(torch.Tensor), b)
 
 
+@pytest.mark.parametrize("f", ["chunk", "norm"])
+def test_what_an_unpack_hook_returns_is_looked_at(dev, f):
+    """A copy in another layout is as good as the saved tensor; a tensor of another shape, type or device is an error, not
+    a pointer for a kernel."""
+    if f == "norm":
+        from hdla_impl_b200.layer_ops import rms_norm_fused_gate
+        x, do = layer_leaves(dev)
+        x, op = [x[5], x[5].detach().clone().requires_grad_(True), x[6]], rms_norm_fused_gate
+    else:
+        x, do = leaves(dev, torch.bfloat16)
+        op = chunk
+
+    def grads(unpack):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach().clone(), unpack):
+            o = op(*x)
+        return torch.autograd.grad(o, x, do)
+
+    want = torch.autograd.grad(op(*x), x, do)
+    strided = lambda t: t.transpose(0, -1).contiguous().transpose(0, -1)
+    for a, b in zip(grads(strided), want):
+        assert torch.equal(a, b)
+    for bad in (lambda t: t.cpu(), lambda t: t.double(), lambda t: t[..., :-1], lambda t: t[:0]):
+        with pytest.raises(RuntimeError, match="saved-tensor hook"):
+            grads(bad)
+    for a, b in zip(grads(lambda t: t), want):
+        assert torch.equal(a, b)
+
+
 _FP32_WAIT = """
 import ctypes as C, sys, torch
 sys.path.insert(0, {root!r})
