@@ -136,9 +136,7 @@ def native():
         with _lock:
             if _native is None:
                 from . import build as _build
-                path = _build.BINDING
-                if not os.path.exists(path):
-                    _build.build_binding()
+                path = _build.build_binding()               # (built only if missing, older than its source, or for another PyTorch)
                 spec = importlib.util.spec_from_file_location("hdla_impl_b200._binding", path)
                 mod = importlib.util.module_from_spec(spec)
                 spec.loader.exec_module(mod)

@@ -777,6 +777,11 @@ PyObject* py_bind(PyObject*, PyObject* const* av, Py_ssize_t n) {
     void* h = PyLong_AsVoidPtr(av[0]);
     if (PyErr_Occurred()) return nullptr;
     if (!guarded([&] {
+            decltype(&hdla_version) version;
+            look_up(h, "hdla_version", version);
+            if (version() != HDLA_VERSION)
+                throw std::runtime_error("_binding.so is built for version " + std::to_string(HDLA_VERSION) +
+                                         " of libhdla, this is version " + std::to_string(version()));
             look_up(h, "hdla_chunk_workspace_bytes", abi.workspace_bytes);
             look_up(h, "hdla_chunk_uses_tensor_cores", abi.uses_tensor_cores);
             look_up(h, "hdla_fp32_status_words", abi.fp32_status_words);
@@ -793,6 +798,9 @@ PyObject* py_bind(PyObject*, PyObject* const* av, Py_ssize_t n) {
     g_on_overflow = av[1];
     Py_RETURN_NONE;
 }
+
+// read from the file before it is loaded (build.py)
+__attribute__((used)) const char kBuiltFor[] = HDLA_BUILT_FOR;
 
 #define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL
 PyMethodDef methods[] = {{"bind", FAST(py_bind), nullptr},
