@@ -1,11 +1,11 @@
-// fp32 CUDA-core pipeline of the chunked HDLA operator (forward and backward).
+// General fp32 CUDA-core kernels of the chunked HDLA operator (forward and backward).
 //
-// This is the full-precision path: it serves fp32 inputs (tensor-core operand rounding cannot
-// meet a 1e-4 tolerance) and is the on-device reference every tensor-core stage is compared
-// with.  It mirrors the reference's stage sequence one to one
+// They serve what neither the bf16 tensor-core pipeline (chunk_tc.cu) nor the fp32 pipeline of rank-2
+// problems (chunk_f32.cu) takes: ranks other than 2, head dims above 128, large problems of a few
+// channels.  They mirror the reference's stage sequence one to one
 //   forward  (HRDPLR/hrdplr.py:25-99):   cumsum+gating -> A matrices -> (I-Aab)^-1 -> w,u -> state scan -> o
 //   backward (HRDPLR/hrdplr.py:146-284): dAu -> dhu (reverse scan) -> dv -> bwd_o -> wy -> intra -> dgk
-// but keeps every intermediate in fp32, chunk-major and zero padded to whole chunks:
+// but keep every intermediate in fp32, chunk-major and zero padded to whole chunks:
 // buffer[(bh*NT + n)][rows][cols] with bh = b*H + h.  Decay-weighted products are evaluated
 // with the exponent difference taken per element (exp(g_i - g_j) with g_i <= g_j on the causal
 // mask), so no operand is ever scaled by exp(-g) and nothing can overflow however strong the

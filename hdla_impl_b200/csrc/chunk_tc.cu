@@ -1,5 +1,5 @@
 // Tensor-core (tcgen05 / TMEM / bulk-copy) pipeline of the chunked HDLA operator for bf16 inputs,
-// chunk 64, rank 2, K = V = 128.
+// chunk 64, rank 2, K and V multiples of 8 up to 128.
 //
 // Scaled ("hat") operands.  With gi / ge the inclusive / exclusive chunk-local cumulative log
 // decay and half = gi[last]/2 (per chunk and channel), E = exp(half):
@@ -46,7 +46,7 @@ struct PrepP {
     float scale;
     int T, H, NT, gdt;
     int* status;
-    int Kd, Vd;                           // head dims of the public tensors (multiples of 8, <= 128); the tiles are padded with zeros
+    int Kd, Vd;                           // head dims of the public tensors (multiples of 8, <= 128); columns from there to KW / VW are zero
     const int2* chunk_tab;                // variable-length batches: (first token, tokens) per chunk, else null
     int KW, VW;                           // widths of the tiles (head dims rounded up to 16), <= 128
     const __nv_bfloat16* beta;            // in-operator a/b parametrisation: [B,T,H]; a and b are not read, gk is log_f
@@ -1683,6 +1683,8 @@ int set_smem(Kern kern, int bytes) {
     return HDLA_OK;
 }
 
+}  // namespace
+
 // number of SMs of the current device (grid size of the persistent kernels), cached per host thread and device
 int sm_count() {
     static thread_local int cached_dev = -1, cached = 0;
@@ -1696,8 +1698,6 @@ int sm_count() {
     }
     return cached;
 }
-
-}  // namespace
 
 int tc_compose_states(const float* T, const float* F, const float* S0, const float* pre, const float* post,
                       float* out, int BH, int count, long long f_stride, long long t_stride, int reverse,
@@ -1723,7 +1723,7 @@ int tc_wait_timeout_probe(int* status, unsigned long long budget_ns, cudaStream_
 }
 
 bool tc_supported(const HdlaDims& d) {
-    // head dims below 128 run on the same 128-wide tiles, padded with zeros (multiples of 8: whole 16-byte chunks);
+    // head dims below 128 fill a prefix of the 128-wide tiles (multiples of 8: whole 16-byte chunks);
     // phased calls (context parallelism) exchange K x V states between devices and need the full 128 x 128
     const bool dims_ok = d.K % 8 == 0 && d.V % 8 == 0 && d.K >= 8 && d.V >= 8 && d.K <= K && d.V <= V;
     const bool full = d.K == K && d.V == V;

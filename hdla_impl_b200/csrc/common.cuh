@@ -16,6 +16,7 @@ int fail(int code, const char* fmt, ...);
 void count_launch(const char* what);
 // Tells the instrumentation which stream the calling thread's current entry point launches on.
 void begin_call(cudaStream_t stream);
+int sm_count();          // SMs of the current device
 // Validation shared by all entry points (api.cu).
 int check_common(const HdlaDims* d, bool chunked);
 

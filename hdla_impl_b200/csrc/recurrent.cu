@@ -349,9 +349,9 @@ __global__ void __launch_bounds__(128, KR * CPT <= 32 ? 4 : KR * CPT <= 64 ? 3 :
 //   * one CTA per (sequence, head): ONE cp.async.bulk brings the whole contiguous fp32 [K,V] tile
 //     (64 KB at K=V=128) into shared memory and one brings it back, so the bytes in flight per SM
 //     are set by how many tiles fit in shared memory (three), not by the register file;
-//   * the update runs in place in shared memory with the same ownership as above (lane owns rows
-//     lane/8 + 4s of 4 adjacent columns: 128-bit, conflict-free accesses; reductions by register
-//     sums and two shuffles);
+//   * the update runs in place in shared memory: lane l of a warp owns rows l/8 + 4s of 4 adjacent
+//     columns, a warp 32 columns (128-bit, conflict-free accesses; reductions by register sums and
+//     two shuffles);
 //   * the CTA leaves as soon as the outgoing copy has read the tile (wait_group.read), the global
 //     write itself drains asynchronously while the next CTA's load is already running.
 // ------------------------------------------------------------------------------------------
@@ -571,10 +571,10 @@ int recurrent_fwd_launch(const HdlaDims& d, const void* q, const void* k, const 
     }
     int rc;
     const int NH = N * d.H;
-    // Two columns per lane instead of four while that leaves no more than two warps to a scheduler (148 SMs x 4): the pass
+    // Two columns per lane instead of four while that leaves no more than two warps to a scheduler (four per SM): the pass
     // over the state is then what a token waits for, and it is half as long.  (With more warps the wider tile wins,
     // since a shared load feeds twice the arithmetic.)
-    const bool narrow = d.R == 2 && (long long)NH * ((d.V + 15) / 16) <= 148 * 4;
+    const bool narrow = d.R == 2 && (long long)NH * ((d.V + 15) / 16) <= sm_count() * 4;
     if (narrow && d.K <= 64)       rc = launch_reg<8, 2, 2>(p, NH, st);
     else if (narrow && d.K <= 128) rc = launch_reg<16, 2, 2>(p, NH, st);
     else if (d.K <= 32)  rc = launch_rank<4, 4>(p, NH, d.R, st);
