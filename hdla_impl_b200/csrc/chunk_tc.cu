@@ -1220,24 +1220,6 @@ __global__ void c8_to_rowmajor_kernel(const uint4* src, float* dst, int rows, in
     }
 }
 
-// debugging aid: product of two C8 tiles, X [128 x n] times Y [n x 128] (or Y^T, Y [128 x n]) -> fp32 row-major, for
-// the intermediates that the pipeline itself no longer forms
-__global__ void c8_product_kernel(const uint4* x, const uint4* y, float* dst, int n, int y_transposed) {
-    const long long g = blockIdx.x;
-    const int yr = y_transposed ? 128 : n;
-    const __nv_bfloat16* xt = reinterpret_cast<const __nv_bfloat16*>(x + g * (n * 16));
-    const __nv_bfloat16* yt = reinterpret_cast<const __nv_bfloat16*>(y + g * (n * 16));
-    auto at = [](const __nv_bfloat16* t, int rows, int r, int c) {
-        return __bfloat162float(t[(((c >> 3) * rows + r) << 3) + (c & 7)]);
-    };
-    for (int e = threadIdx.x; e < 128 * 128; e += blockDim.x) {
-        const int r = e >> 7, c = e & 127;
-        float s = 0.f;
-        for (int j = 0; j < n; ++j) s = fmaf(at(xt, 128, r, j), y_transposed ? at(yt, yr, c, j) : at(yt, yr, j, c), s);
-        dst[(size_t)g * 128 * 128 + e] = s;
-    }
-}
-
 // ------------------------------------------------------------------------------------------
 // backward, last stage: gradients of the hat operands, dv, un-gating and dgk in one kernel
 //   (HRDPLR/bwd_triton.py: dv 227-290, bwd_o 295-487, score-gradient applications of intra 761-827,
@@ -2045,14 +2027,6 @@ int tc_debug_buffer(const HdlaDims& d, const unsigned char* ws, const char* name
             HDLA_CHECK_LAUNCH("c8_to_rowmajor_kernel");
             return HDLA_OK;
         }
-    if (pl.KW == K && pl.VW == V && (!strcmp(name, "P") || !strcmp(name, "dW"))) {         // P = Aak v,  dWh = dv2 St^T
-        const bool fwd = name[0] == 'P';
-        c8_product_kernel<<<(unsigned)pl.G, 128, 0, st>>>(reinterpret_cast<const uint4*>(ws + (fwd ? pl.Aak : pl.DV2)),
-                                                          reinterpret_cast<const uint4*>(ws + (fwd ? pl.Vc : pl.Hs)), out,
-                                                          fwd ? 64 : 128, fwd ? 0 : 1);
-        HDLA_CHECK_LAUNCH("c8_product_kernel");
-        return HDLA_OK;
-    }
     if (!strcmp(name, "E")) {
         cudaMemcpyAsync(out, ws + pl.E, (size_t)pl.G * K * 4, cudaMemcpyDeviceToDevice, st);
         return HDLA_OK;

@@ -24,7 +24,7 @@ HDLA_API void hdla_timing_enable(int on);
 HDLA_API size_t hdla_timing_report(char* buf, size_t size);
 
 /* Converts one named bf16 tile buffer of the tensor-core workspace ("Qh","Kh","Ah","Bh","Vc","Aqk","Aqb","Aak",
- * "M","W","P","U","Hs","V2","dOc","dAqk","dAqb","DV2","DE","dW","dP","dAak","dAab") to fp32 row-major
+ * "M","W","U","Hs","V2","dOc","dAqk","dAqb","DV2","DE","dP","dAak","dAab") to fp32 row-major
  * [B*H*NT][rows][cols] in `out` (device memory), or copies "E" / "dgl" / the "status" words. */
 HDLA_API int hdla_debug_tc_buffer(const HdlaDims* dims, const void* workspace, const char* name, float* out,
                                   void* cuda_stream);

@@ -195,6 +195,70 @@ def test_what_an_unpack_hook_returns_is_looked_at(dev, f):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_second_backward_recomputes(dev, dtype):
+    """The first backward uses up the kept workspace; a second one through the same graph computes it again (the same
+    kernels on the same inputs: equal bit for bit), a third after the graph is gone is an error."""
+    x, do = leaves(dev, dtype)
+    o = chunk(*x)
+    first = torch.autograd.grad(o, x, do, retain_graph=True)
+    second = torch.autograd.grad(o, x, do)
+    for a, b in zip(first, second):
+        assert torch.equal(a, b)
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(o, x, do)
+
+
+def test_threads_on_streams_of_their_own(dev):
+    """Four threads, each with its stream and inputs, forward and backward, with a decay history that makes forwards wait
+    for their own status words: results as alone."""
+    import threading
+    import hdla_impl_b200 as HD
+    from hdla_impl_b200 import hrdplr
+    n, rounds = 4, 40
+    inputs = [leaves(dev, torch.bfloat16 if i % 2 else torch.float32, T=100 + 30 * i, seed=i) for i in range(n)]
+    want = [torch.autograd.grad(chunk(*x), x, do) for x, do in inputs]
+    torch.cuda.synchronize(dev)
+    before = hrdplr._status_state(dev)["decay"]
+    hrdplr._status_state(dev)["decay"] = 100.0
+    wrong = []
+
+    def work(i):
+        try:
+            x, do = inputs[i]
+            with torch.cuda.stream(torch.cuda.Stream(dev)):
+                for _ in range(rounds):
+                    got = torch.autograd.grad(chunk(*x), x, do)
+                torch.cuda.current_stream(dev).synchronize()
+            if not all(torch.equal(a, b) for a, b in zip(got, want[i])):
+                wrong.append(i)
+        except Exception as e:          # noqa: BLE001 -- reported by the main thread
+            wrong.append(e)
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(n)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    hrdplr._status_state(dev)["decay"] = before
+    assert not wrong, wrong
+    HD.check_status(dev, wait=True)
+
+
+@pytest.mark.parametrize("what", ["chunk", "layer"])
+def test_transforms_that_the_operator_does_not_support_are_refused(dev, what):
+    """Forward-mode gradients and vmap raise; they do not run without the tangent or on a wrapper's memory."""
+    import torch.autograd.forward_ad as fwad
+    x, _ = layer_leaves(dev) if what == "layer" else leaves(dev, torch.bfloat16)
+    f = layer if what == "layer" else chunk
+    x = [t.detach() for t in x]
+    with fwad.dual_level():
+        with pytest.raises(RuntimeError):
+            f(fwad.make_dual(x[0], torch.ones_like(x[0])), *x[1:])
+    with pytest.raises(RuntimeError):
+        torch.vmap(lambda q: f(q, *x[1:]))(torch.stack([x[0], x[0]]))
+
+
 _FP32_WAIT = """
 import ctypes as C, sys, torch
 sys.path.insert(0, {root!r})

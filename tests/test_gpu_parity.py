@@ -64,7 +64,7 @@ def assert_close(got, ref, tol, label=""):
 
 @pytest.mark.parametrize("chunk", [64, 16])
 def test_chunk_cfg0_fp32(dev, chunk):
-    """B2 T256 H4 K=V=64 fp32 seed 0, zero initial state: o, final state and all gradients."""
+    """B2 T256 H4 K=V=64 fp32 seed 0, zero initial state: o, final state and all gradients, whatever chunk is asked for."""
     x = make_inputs(2, 256, 4, 64, 64, R, seed=0, with_dht=True)
     got = run_chunk(x, dev, 1.0, chunk, False, False, torch.float32)
     ref = oracle_chunk(x, 1.0, False, False, torch.float32)
@@ -82,7 +82,7 @@ def test_chunk_cfg0_against_reference_golden(dev, golden_dir):
 
 @pytest.mark.parametrize("chunk", [16, 32, 64])
 def test_chunk_small_golden_strong_decay(dev, golden_dir, chunk):
-    """Reference golden case: undivided logsigmoid decay, random h0 and dht, K=32, V=48."""
+    """Reference golden case: undivided logsigmoid decay, random h0 and dht, K=32, V=48, whatever chunk is asked for."""
     z = np.load(os.path.join(golden_dir, "naive_small.npz"))
     x = {n[3:]: torch.from_numpy(z[n]) for n in z.files if n.startswith("in_")}
     ref = {n[4:]: torch.from_numpy(z[n]) for n in z.files if n.startswith("out_")}
@@ -403,8 +403,9 @@ def test_bf16_random_shapes_against_oracle(dev, seed):
 
 @pytest.mark.parametrize("seed", range(6))
 def test_fp32_random_shapes_against_oracle(dev, seed):
-    """Seeded random problems of the fp32 pipeline: any head dims (odd ones included, as the reference takes any
-    K <= 256 and any V), ragged lengths, chunk 16 / 32 / 64, strong and weak decay: forward + backward, 1e-4."""
+    """Seeded random fp32 problems: any head dims (odd ones included, as the reference takes any K <= 256 and any V),
+    ragged lengths, strong and weak decay: forward + backward, 1e-4.  (Up to 128 channels they run on the pipeline of
+    16-token tiles whatever chunk is asked for; the general kernels have a test of their own below.)"""
     import random
     rng = random.Random(3000 + seed)
     B, H = rng.choice([1, 2]), rng.choice([1, 2, 3])
@@ -418,6 +419,36 @@ def test_fp32_random_shapes_against_oracle(dev, seed):
     got = run_chunk(x, dev, scale, chunk, use_h0, use_dht, torch.float32)
     ref = oracle_chunk(x, scale, use_h0, use_dht, torch.float32)
     assert_close(got, ref, 1e-4, f"B{B} T{T} H{H} K{K} V{V} chunk {chunk} h0={use_h0} dht={use_dht} gk/{gk_div}")
+
+
+@pytest.mark.parametrize("rank,K,V,chunk,T,dtype", [
+    (1, 64, 64, 16, 83, torch.float32), (3, 40, 24, 32, 70, torch.float32), (4, 32, 48, 32, 130, torch.float32),
+    (1, 128, 128, 64, 64, torch.float32), (4, 16, 20, 16, 33, torch.float32), (2, 136, 64, 16, 65, torch.float32),
+    (2, 64, 256, 32, 100, torch.float32), (2, 200, 130, 64, 129, torch.float32), (2, 256, 256, 64, 40, torch.float32),
+    (1, 64, 64, 64, 100, torch.bfloat16), (3, 33, 17, 32, 45, torch.bfloat16), (2, 160, 96, 16, 50, torch.bfloat16)])
+def test_general_fp32_kernels_against_oracle(dev, rank, K, V, chunk, T, dtype):
+    """What no pipeline takes -- ranks other than 2, head dims above 128 -- at chunks of 16, 32 and 64 with ragged ends, an
+    initial state and the final state's gradient: forward + backward.  fp32 arithmetic throughout, as the other fp32
+    tests; bf16 tensors only round the results."""
+    import hdla_impl_b200 as HD
+    from hdla_impl_b200 import _lib
+    B, H = 2, 2
+    x = make_inputs(B, T, H, K, V, rank, seed=T + K, dtype=dtype, gk_div=2.0, h0_std=0.4, with_dht=True)
+    names = ("q", "k", "v", "a", "b", "gk")
+    lv = [x[n].to(dev).requires_grad_(True) for n in names] + [x["h0"].to(dev).requires_grad_(True)]
+    _lib.timing_report()
+    _lib.timing_enable(True)
+    o, ht = HD.chunk_hrdplr_delta_rule(*lv[:6], rank, scale=0.3, initial_state=lv[6], output_final_state=True,
+                                       chunk_size=chunk)
+    grads = torch.autograd.grad([o, ht], lv, [x["do"].to(dev), x["dht"].to(dev)])
+    _lib.timing_enable(False)
+    launched = set(_lib.timing_report())
+    assert launched and not any(n.startswith("f32_") or "_tc_" in n for n in launched), launched
+    got = dict(zip(["o", "ht"] + GRADS + ["dh0"], [o, ht, *grads]))
+    st = orc.staged_forward(*[x[n].double() for n in names], rank, 0.3, x["h0"], 64)
+    g = orc.staged_backward(st, x["do"].double(), x["dht"])
+    ref = dict(o=st["o_bthv"], ht=st["ht"], **{n: g[n] for n in GRADS + ["dh0"]})
+    assert_close(got, ref, 1e-4 if dtype == torch.float32 else 1e-2, f"rank {rank} K{K} V{V} chunk {chunk} T{T}")
 
 
 @pytest.mark.parametrize("seed", range(4))
@@ -882,7 +913,7 @@ def test_fp32_pipeline_edges(dev, B, T, H, K, V, gk_div, h0, dtype, monkeypatch)
 def test_bf16_requested_chunk_16_runs_on_tensor_cores(dev, monkeypatch):
     """The reference layer passes chunk_size=16; the result is chunk-size independent, so supported bf16
     problems still take the tensor-core pipeline (10 launches for forward+backward, 7 with the one-kernel chunk
-    preparation, not the 43 of the fp32 one)."""
+    preparation)."""
     import hdla_impl_b200 as H
     from hdla_impl_b200 import _lib
     x = make_inputs(1, 256, 2, 128, 128, R, seed=17, dtype=torch.bfloat16, with_dht=True)
@@ -898,7 +929,7 @@ def test_bf16_requested_chunk_16_runs_on_tensor_cores(dev, monkeypatch):
     for n in a:
         assert torch.equal(a[n], b[n]), n
     monkeypatch.setenv("HDLA_HONOR_CHUNK", "1")
-    c = run_chunk(x, dev, 1.0, 16, False, True, torch.bfloat16)      # fp32 pipeline at chunk 16
+    c = run_chunk(x, dev, 1.0, 16, False, True, torch.bfloat16)      # a chunk of 16 is the fp32 pipeline's
     ref = oracle_chunk(x, 1.0, False, True, torch.bfloat16)
     assert_close(c, ref, 2e-2, "chunk 16 honoured")
     assert_close(a, ref, 2e-2, "chunk 16 requested")
