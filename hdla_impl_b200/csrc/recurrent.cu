@@ -5,8 +5,8 @@
 //     S_t   = exp(g_t) (.) S_{t-1} + sum_r b_r sa_r^T + k_t v_t^T
 //     o_t   = (scale q_t)^T S_t
 //
-// Two kernels: up to kBulkTokens tokens per call the state tile passes through shared memory by bulk copies
-// (recurrent_bulk_kernel: bound by HBM, the fp32 state is read and written once); longer sequences keep it in
+// Two kernels: up to kTileTokens tokens per call the state tile passes through shared memory
+// (recurrent_tile_kernel: bound by HBM, the fp32 state is read and written once); longer sequences keep it in
 // registers (recurrent_reg_kernel: bound by fp32 arithmetic or by the dependent steps of the recurrence).
 #include "common.cuh"
 #include "f32x2.cuh"
@@ -15,8 +15,8 @@
 namespace hdla {
 namespace {
 
-// Set to 1 by the decode kernel when its (time-bounded) wait for the state tile ran out: the call's
-// outputs are invalid and the final state was not written.  Read with hdla_recurrent_read_status().
+// Read with hdla_recurrent_read_status(): non-zero once a time-limited wait of a kernel here ran out.  None of them has
+// such waits, so it stays zero.
 __device__ int g_recurrent_status;
 
 struct RecParams {
@@ -28,12 +28,6 @@ struct RecParams {
     float scale;
     int T, H, K, V, dt, gdt, reverse;
 };
-
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sm100::smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // Sum N values over the eight row lanes of a warp (lane bits 2..4), N = 1, 2, 4 or 8: each step halves the values a lane
 // still carries, so N = 8 costs 7 shuffles instead of 24.  Lane r ends with the sums of N/8 (at least one) values,
@@ -106,7 +100,7 @@ __device__ __forceinline__ void st_cols(const float* x, float* base, int nh, int
     }
 }
 
-// Register-state kernel: more than kBulkTokens tokens per call.
+// Register-state kernel: more than kTileTokens tokens per call.
 //   * A column of the state depends on the other columns through nothing, so the columns are spread over warps (and,
 //     while there are fewer warps than the chip runs, over CTAs): a warp owns 4 CPT columns, lane (r, c) of it the
 //     rows 4 r + 32 j + {0..3} of CPT adjacent columns, in registers, as packed row pairs.
@@ -123,7 +117,7 @@ __device__ __forceinline__ void st_cols(const float* x, float* base, int nh, int
 constexpr int kRecBlock = 8;
 // Up to two tokens the bulk-copied tile is the faster form (256 x 32 heads: 176 / 267 us for 1 / 2 tokens against 328 /
 // 284), from three on the registers are (4 tokens: 366 against 456 us; 8 heads, 4 tokens: 7.4 against 15.5).
-constexpr int kBulkTokens = 2;
+constexpr int kTileTokens = 2;
 
 template <int KR, int CPT, int R>
 __global__ void __launch_bounds__(128, KR * CPT <= 32 ? 4 : KR * CPT <= 64 ? 3 : 2) recurrent_reg_kernel(RecParams p, int col_blocks, int async_ok) {
@@ -173,9 +167,9 @@ __global__ void __launch_bounds__(128, KR * CPT <= 32 ? 4 : KR * CPT <= 64 ? 3 :
             }
             unsigned char* dst = raw + (size_t)w * 16;
             if (p.reverse) step = (size_t)0 - step;
-            for (int tk = 0; tk < cnt; ++tk, src += step, dst += tok_raw) cp_async16(dst, src);
+            for (int tk = 0; tk < cnt; ++tk, src += step, dst += tok_raw) sm100::cp_async16(dst, src);
         }
-        cp_async_commit();
+        sm100::cp_async_commit();
     };
     // Turn them into fp32, four elements at a time: a thread keeps its place for all tokens of the block, so the
     // eight tokens' loads are in flight together.
@@ -244,7 +238,7 @@ __global__ void __launch_bounds__(128, KR * CPT <= 32 ? 4 : KR * CPT <= 64 ? 3 :
 
     for (long long s0 = 0; s0 < len; s0 += kRecBlock) {
         const int cnt = (int)min((long long)kRecBlock, len - s0);
-        if (async_ok) cp_async_wait_all();
+        if (async_ok) sm100::cp_async_wait<0>();
         __syncthreads();                                     // the raw block is here and the fp32 block has been read
         convert(s0);
         __syncthreads();
@@ -343,26 +337,34 @@ __global__ void __launch_bounds__(128, KR * CPT <= 32 ? 4 : KR * CPT <= 64 ? 3 :
     }
 }
 
+// an element as it is stored, and its value
+__device__ __forceinline__ uint32_t ld_raw(const void* p, size_t i, int dt) {
+    return dt == HDLA_F32 ? static_cast<const uint32_t*>(p)[i] : static_cast<const unsigned short*>(p)[i];
+}
+__device__ __forceinline__ float raw_float(uint32_t x, int dt) { return __uint_as_float(dt == HDLA_F32 ? x : x << 16); }
+
 // ------------------------------------------------------------------------------------------
-// Decode variant (a few tokens per call): the state tile is staged in shared memory by the bulk
-// asynchronous copy engine instead of through registers.
-//   * one CTA per (sequence, head): ONE cp.async.bulk brings the whole contiguous fp32 [K,V] tile
-//     (64 KB at K=V=128) into shared memory and one brings it back, so the bytes in flight per SM
-//     are set by how many tiles fit in shared memory (three), not by the register file;
-//   * the update runs in place in shared memory: lane l of a warp owns rows l/8 + 4s of 4 adjacent
-//     columns, a warp 32 columns (128-bit, conflict-free accesses; reductions by register sums and
-//     two shuffles);
-//   * the CTA leaves as soon as the outgoing copy has read the tile (wait_group.read), the global
-//     write itself drains asynchronously while the next CTA's load is already running.
+// Decode variant (one or two tokens per call): the state tile is staged in shared memory.
+//   * one CTA per (sequence, head) brings the whole contiguous fp32 [K,V] tile (64 KB at K=V=128) into shared memory by
+//     16-byte asynchronous copies, so the bytes in flight per SM are set by how many tiles fit in shared memory (three),
+//     not by the register file;
+//   * a token's vectors are asked for a step ahead, the first one's before the tile, and stay as they came until they are
+//     needed: behind the tile's copies, or converted at once, they cost 25 to 50 us of 165 (256 sequences x 32 heads);
+//   * lane l of a warp owns rows l/8 + 4s of 4 adjacent columns, a warp 32 columns (128-bit, conflict-free accesses;
+//     reductions by register sums and two shuffles); a token updates the tile in place, the last one writes it to global
+//     memory from the registers (whole 128-byte lines), which drains while the next CTA's tile is on its way.
+// Bound by HBM, the fp32 state being read and written once: 256 sequences x 32 heads of 128 take 165 us for one token,
+// 6.6 TB/s; two tokens 226.
+// (Before, one bulk copy brought the tile in, counted on an mbarrier, and one took it back: 184 and 267 us.  That form ended
+// in a launch failure with 28 CTAs of 256-byte tiles on an SM -- K = V = 8, 4096 heads, two tokens -- with every address,
+// size and alignment in order; larger tiles, which leave room for fewer CTAs, never showed it.)
 // ------------------------------------------------------------------------------------------
 template <int R>
-__global__ void __launch_bounds__(256) recurrent_bulk_kernel(RecParams p) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t bar;
+__global__ void __launch_bounds__(256) recurrent_tile_kernel(RecParams p) {
+    extern __shared__ __align__(16) float sS[];                 // [K][V], then the token's vectors
     const int nh = blockIdx.x;
     const int n = nh / p.H, h = nh % p.H;
     const int K = p.K, V = p.V, H = p.H;
-    float* sS = reinterpret_cast<float*>(smem_raw);             // [K][V]
     float* s_q = sS + (size_t)K * V;
     float* s_k = s_q + K;
     float* s_e = s_k + K;
@@ -373,29 +375,52 @@ __global__ void __launch_bounds__(256) recurrent_bulk_kernel(RecParams p) {
     const int r = lane >> 3;
     const int c4 = (warp * 8 + (lane & 7)) * 4;
     const bool col_ok = c4 < V;
-    const uint32_t tile_bytes = (uint32_t)K * V * 4u;
 
     long long bos, len;
     if (p.cu) { bos = p.cu[n]; len = p.cu[n + 1] - bos; }
     else      { bos = (long long)n * p.T; len = p.T; }
-    bool state_ok = true;                                        // false once the wait for the state tile ran out
 
-    if (threadIdx.x == 0) {
-        sm100::mbar_init(&bar, 1);
-        sm100::fence_mbar_init();
-        if (p.h0) {
-            sm100::mbar_expect_tx(&bar, tile_bytes);
-            sm100::bulk_g2s(sS, p.h0 + (size_t)nh * K * V, tile_bytes, &bar);
+    const int tid = threadIdx.x;
+    uint32_t raw[4 + 2 * R];                                     // element tid of q k gk v and of every a, b
+    auto ask = [&](long long step) {
+        const long long t = p.reverse ? (bos + len - 1 - step) : (bos + step);
+        const size_t tk = ((size_t)t * H + h) * K + tid;
+        if (tid < K) {
+            raw[0] = ld_raw(p.q, tk, p.dt); raw[1] = ld_raw(p.k, tk, p.dt); raw[2] = ld_raw(p.gk, tk, p.gdt);
+#pragma unroll
+            for (int rr = 0; rr < R; ++rr) {
+                const size_t ta = (((size_t)t * R + rr) * H + h) * K + tid;
+                raw[4 + 2 * rr] = ld_raw(p.a, ta, p.dt); raw[5 + 2 * rr] = ld_raw(p.b, ta, p.dt);
+            }
         }
+        if (tid < V) raw[3] = ld_raw(p.v, ((size_t)t * H + h) * V + tid, p.dt);
+    };
+    if (len > 0) ask(0);
+    const size_t tile = (size_t)nh * K * V;
+    if (p.h0) {
+        const float* src = p.h0 + tile;
+#pragma unroll 8
+        for (int i = tid * 4; i < K * V; i += blockDim.x * 4) sm100::cp_async16(sS + i, src + i);
+    } else {
+        for (int i = tid * 4; i < K * V; i += blockDim.x * 4)
+            *reinterpret_cast<float4*>(sS + i) = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    if (!p.h0)
-        for (int i = threadIdx.x; i < K * V / 4; i += blockDim.x)
-            reinterpret_cast<float4*>(sS)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    sm100::cp_async_commit();
 
     for (long long step = 0; step < len; ++step) {
+        const bool last = step + 1 == len;
         const long long t = p.reverse ? (bos + len - 1 - step) : (bos + step);
         const size_t tk = ((size_t)t * H + h) * K;
-        for (int i = threadIdx.x; i < K; i += blockDim.x) {
+        if (tid < K) {
+            s_q[tid] = raw_float(raw[0], p.dt) * p.scale; s_k[tid] = raw_float(raw[1], p.dt);
+            s_e[tid] = __expf(raw_float(raw[2], p.gdt));
+#pragma unroll
+            for (int rr = 0; rr < R; ++rr) {
+                s_a[rr * K + tid] = raw_float(raw[4 + 2 * rr], p.dt); s_b[rr * K + tid] = raw_float(raw[5 + 2 * rr], p.dt);
+            }
+        }
+        if (tid < V) s_v[tid] = raw_float(raw[3], p.dt);
+        for (int i = tid + blockDim.x; i < K; i += blockDim.x) { // (heads with more rows than the CTA has threads)
             s_q[i] = ld_elem(p.q, tk + i, p.dt) * p.scale;
             s_k[i] = ld_elem(p.k, tk + i, p.dt);
             s_e[i] = __expf(ld_elem(p.gk, tk + i, p.gdt));
@@ -406,13 +431,9 @@ __global__ void __launch_bounds__(256) recurrent_bulk_kernel(RecParams p) {
                 s_b[rr * K + i] = ld_elem(p.b, ta + i, p.dt);
             }
         }
-        for (int i = threadIdx.x; i < V; i += blockDim.x)
-            s_v[i] = ld_elem(p.v, ((size_t)t * H + h) * V + i, p.dt);
+        sm100::cp_async_wait<0>();                               // the tile (first step)
         __syncthreads();
-        if (step == 0 && p.h0) {                                 // bounded; the tile is in shared memory after it
-            state_ok = __syncthreads_and(sm100::mbar_wait(&bar, 0) ? 1 : 0) != 0;
-            if (!state_ok && threadIdx.x == 0) atomicExch(&g_recurrent_status, 1);
-        }
+        if (!last) ask(step + 1);
 
         float sa[R][4];
 #pragma unroll
@@ -438,6 +459,7 @@ __global__ void __launch_bounds__(256) recurrent_bulk_kernel(RecParams p) {
         float oa[4] = {0.f, 0.f, 0.f, 0.f};
         if (col_ok) {
             const float vv[4] = {s_v[c4], s_v[c4 + 1], s_v[c4 + 2], s_v[c4 + 3]};
+            float* out = last && p.ht ? p.ht + tile + c4 : nullptr;
             for (int kk = r; kk < K; kk += 4) {
                 float4* ps = reinterpret_cast<float4*>(sS + (size_t)kk * V + c4);
                 const float4 x = *ps;
@@ -450,7 +472,9 @@ __global__ void __launch_bounds__(256) recurrent_bulk_kernel(RecParams p) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) y[j] = fmaf(bv, sa[rr][j], y[j]);
                 }
-                *ps = make_float4(y[0], y[1], y[2], y[3]);
+                const float4 z = make_float4(y[0], y[1], y[2], y[3]);
+                if (!last) *ps = z;
+                else if (out) *reinterpret_cast<float4*>(out + (size_t)kk * V) = z;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) oa[j] = fmaf(qv, y[j], oa[j]);
             }
@@ -471,20 +495,13 @@ __global__ void __launch_bounds__(256) recurrent_bulk_kernel(RecParams p) {
                 *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.o) + to) = pk;
             }
         }
-        __syncthreads();                                         // vectors are single buffered
+        if (!last) __syncthreads();                              // vectors are single buffered
     }
-    if (len == 0 && p.h0) {
-        state_ok = __syncthreads_and(sm100::mbar_wait(&bar, 0) ? 1 : 0) != 0;
-        if (!state_ok && threadIdx.x == 0) atomicExch(&g_recurrent_status, 1);
-    }
-    if (p.ht && state_ok) {                                      // a state that never arrived is not written back
-        sm100::fence_proxy_async();
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            sm100::bulk_s2g(p.ht + (size_t)nh * K * V, sS, tile_bytes);
-            sm100::bulk_commit();
-            sm100::bulk_wait_read<0>();
-        }
+    if (len == 0) {                                              // a sequence without tokens: its state passes through
+        sm100::cp_async_wait<0>();
+        if (p.ht)                                                // (each thread the pieces it brought in itself)
+            for (int i = tid * 4; i < K * V; i += blockDim.x * 4)
+                *reinterpret_cast<float4*>(p.ht + tile + i) = *reinterpret_cast<const float4*>(sS + i);
     }
 }
 
@@ -545,28 +562,28 @@ int recurrent_fwd_launch(const HdlaDims& d, const void* q, const void* k, const 
     RecParams p{q, k, v, a, b, gk, h0, o, ht, cu_seqlens, scale, d.T, d.H, d.K, d.V, d.dtype, d.gk_dtype, reverse};
     const int blocks = N * d.H;
     const int threads = 32 * ((d.V + 31) / 32);
-    // few tokens per call: the bulk-copy staged kernel (state tile must fit in shared memory)
+    // few tokens per call: the kernel with the tile in shared memory (which it must fit)
     const size_t tile = (size_t)d.K * d.V * 4;
-    if (d.T <= kBulkTokens && tile <= 65536 && tile % 16 == 0 && d.R <= 4) {
-        const size_t smem_b = tile + sizeof(float) * ((3 + 2 * d.R) * (size_t)d.K + d.V);
+    if (d.T <= kTileTokens && tile <= 65536 && tile % 16 == 0 && d.R <= 4) {
+        const size_t smem_t = tile + sizeof(float) * ((3 + 2 * d.R) * (size_t)d.K + d.V);
         static thread_local int attr_dev = -1;
         int dev = 0;
         cudaGetDevice(&dev);
         if (attr_dev != dev) {
-            cudaError_t e = cudaFuncSetAttribute(recurrent_bulk_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536 + 16384);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(recurrent_bulk_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536 + 16384);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(recurrent_bulk_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536 + 16384);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(recurrent_bulk_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536 + 16384);
+            cudaError_t e = cudaFuncSetAttribute(recurrent_tile_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536 + 16384);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(recurrent_tile_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536 + 16384);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(recurrent_tile_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536 + 16384);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(recurrent_tile_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536 + 16384);
             if (e != cudaSuccess) return fail(HDLA_ERR_CUDA, "recurrent: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
             attr_dev = dev;
         }
         switch (d.R) {
-            case 1: recurrent_bulk_kernel<1><<<blocks, threads, smem_b, st>>>(p); break;
-            case 2: recurrent_bulk_kernel<2><<<blocks, threads, smem_b, st>>>(p); break;
-            case 3: recurrent_bulk_kernel<3><<<blocks, threads, smem_b, st>>>(p); break;
-            default: recurrent_bulk_kernel<4><<<blocks, threads, smem_b, st>>>(p); break;
+            case 1: recurrent_tile_kernel<1><<<blocks, threads, smem_t, st>>>(p); break;
+            case 2: recurrent_tile_kernel<2><<<blocks, threads, smem_t, st>>>(p); break;
+            case 3: recurrent_tile_kernel<3><<<blocks, threads, smem_t, st>>>(p); break;
+            default: recurrent_tile_kernel<4><<<blocks, threads, smem_t, st>>>(p); break;
         }
-        HDLA_CHECK_LAUNCH("recurrent_bulk_kernel");
+        HDLA_CHECK_LAUNCH("recurrent_tile_kernel");
         return HDLA_OK;
     }
     int rc;

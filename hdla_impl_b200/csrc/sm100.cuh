@@ -100,6 +100,18 @@ __device__ __forceinline__ void bulk_wait() {          // writes are complete
     asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// ------------------------------------------------------------------------------ per-thread async copy
+// 16 bytes, global -> shared, past the L1.  A thread waits for its own copies as it would for a load (no time limit and
+// nothing to report); a barrier makes them visible to the others.
+__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src_gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src_gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {      // at most N of this thread's groups are still under way
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // ------------------------------------------------------------------------------ tensor memory
 // Warp-collective. Writes the TMEM base address (lane 0, first column) to *dst_smem.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {

@@ -51,7 +51,6 @@ def fused_recurrent_dplr_delta_rule_fwd(q, k, v, a, b, gk, rank_ab, scale=1.0, i
                                     _lib.ptr(gk), float(scale), _lib.ptr(h0), _lib.ptr(o), _lib.ptr(ht),
                                     _lib.ptr(cu), N, int(bool(reverse)), _lib.stream_ptr(dev))
         _lib.check(rc, "hdla_recurrent_fwd")
-        _poll_status(_lib.load, dev)
     return o, ht
 
 
@@ -61,55 +60,19 @@ def _tokens_of_merged(TR: int, rank_ab: int) -> int:
     return T
 
 
-# The decode kernel stages the state tile with an asynchronous copy and waits for it with a time limit; if
-# that wait ever ran out it says so in a device word (hdla_recurrent_read_status).  Decode steps are short,
-# so the word is fetched (without blocking) only every _POLL_EVERY calls and looked at when the copy has
-# landed; check_recurrent_status(wait=True) fetches and inspects it at once.
-_POLL_EVERY = 256
-_poll = {}        # device index -> dict(calls=int, host=pinned int32[1], event=Event|None)
-
-
-def _poll_state(dev):
-    st = _poll.get(dev.index)
-    if st is None:
-        st = dict(calls=0, host=torch.zeros(1, dtype=torch.int32).pin_memory(), event=None)
-        _poll[dev.index] = st
-    return st
-
-
-def _poll_status(load, dev) -> None:
-    st = _poll.get(dev.index) or _poll_state(dev)
-    event = st["event"]
-    if event is not None and not torch.cuda.is_current_stream_capturing() and event.query():
-        st["event"] = None
-        if int(st["host"][0]):
-            raise RuntimeError("libhdla: a device-side wait ran out in the decode kernel; the results of that call "
-                               "are invalid and its final state was not written")
-    st["calls"] += 1
-    if st["calls"] % _POLL_EVERY == 0 and st["event"] is None and not torch.cuda.is_current_stream_capturing():
-        with torch.cuda.device(dev):
-            _lib.check(load().hdla_recurrent_read_status(_lib.ptr(st["host"]), _lib.stream_ptr(dev)),
-                       "hdla_recurrent_read_status")
-            st["event"] = torch.cuda.Event()
-            st["event"].record(torch.cuda.current_stream(dev))
-
-
 def check_recurrent_status(dev, wait: bool = True) -> None:
-    """Fetch the decode kernel's status word for ``dev`` now and raise if a wait ever ran out there."""
+    """Fetch the status word of the recurrent kernels for ``dev`` and, with ``wait``, raise if a time-limited wait ever ran
+    out there (the present kernels have none)."""
     dev = torch.device(dev)
-    lib = _lib.load()
-    st = _poll_state(dev)
+    host = torch.zeros(1, dtype=torch.int32).pin_memory()
     with torch.cuda.device(dev):
-        _lib.check(lib.hdla_recurrent_read_status(_lib.ptr(st["host"]), _lib.stream_ptr(dev)),
+        _lib.check(_lib.load().hdla_recurrent_read_status(_lib.ptr(host), _lib.stream_ptr(dev)),
                    "hdla_recurrent_read_status")
-        ev = torch.cuda.Event()
-        ev.record(torch.cuda.current_stream(dev))
-    st["event"] = ev
-    if wait:
-        ev.synchronize()
-        st["event"] = None
-        if int(st["host"][0]):
-            raise RuntimeError("libhdla: a device-side wait ran out in the decode kernel")
+        if not wait:
+            return
+        torch.cuda.current_stream(dev).synchronize()
+    if int(host[0]):
+        raise RuntimeError("libhdla: a device-side wait ran out in a recurrent kernel")
 
 
 class FusedRecurrentDPLRDeltaRuleFunction(torch.autograd.Function):
@@ -155,7 +118,6 @@ def fused_recurrent_dplr_delta_rule(
     r = (_lib._native or _lib.native()).recurrent(q, k, v, a, b, gk, rank_ab, scale, initial_state, output_final_state,
                                                   reverse, cu_seqlens)
     if r is not NotImplemented:
-        _poll_status(_lib.load, q.device)
         return r
     # what the native path does not take: inputs that require gradients, tensor subclasses, invalid arguments
     if cu_seqlens is not None:

@@ -229,10 +229,9 @@ HDLA_API int hdla_recurrent_fwd(const HdlaDims* dims,
                        const int64_t* cu_seqlens, int32_t n_seqs, int32_t reverse,
                        void* cuda_stream);
 
-/* Enqueues a copy of the decode kernel's status word to dst (1 x int32; device or pinned host memory): non-zero
- * once a bounded wait for a state tile ran out in some hdla_recurrent_fwd call of this process on the current
- * device (that call's outputs are invalid and its final state was not written).  No counterpart in the
- * reference, whose kernel has no asynchronous copies to wait for. */
+/* Enqueues a copy of the recurrent kernels' status word to dst (1 x int32; device or pinned host memory): non-zero once
+ * a time-limited wait ran out in some hdla_recurrent_fwd call of this process on the current device.  The present
+ * kernels have no such waits, so it reads zero.  No counterpart in the reference. */
 HDLA_API int hdla_recurrent_read_status(int32_t* dst, void* cuda_stream);
 
 /* Composition of affine state maps, for callers that cut a sequence over devices (context parallelism; the

@@ -227,6 +227,41 @@ def test_recurrent_register_kernel_edges(dev, B, T, H, K, V, rank, cu, dtype, re
     assert orc.rel_err(o, ro) < (2e-5 if dtype == torch.float32 else 4e-3)
 
 
+@pytest.mark.parametrize("K,V,rank", [(8, 8, 1), (16, 16, 2), (33, 20, 2), (128, 128, 2)])
+@pytest.mark.parametrize("T", [1, 2])
+def test_recurrent_many_heads(dev, K, V, rank, T):
+    """One and two tokens for more heads than the device runs at once, with tiles of a quarter to 64 KB (two dozen small ones
+    share an SM), and a packed batch with sequences of no token, whose state passes through."""
+    import hdla_impl_b200 as Hm
+    B, H = 1536, 4
+    g = torch.Generator(device=dev).manual_seed(K)
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev)
+    nrm = torch.nn.functional.normalize
+    x = [nrm(rn(B, T, H, K), dim=-1), nrm(rn(B, T, H, K), dim=-1), rn(B, T, H, V), -nrm(rn(B, T * rank, H, K), dim=-1),
+         0.5 * nrm(rn(B, T * rank, H, K), dim=-1), torch.nn.functional.logsigmoid(rn(B, T, H, K)) / 4]
+    h0 = rn(B, H, K, V)
+    o, ht = Hm.fused_recurrent_dplr_delta_rule(*x, rank, initial_state=h0, output_final_state=True)
+    q, k, v, a, b, gk = [t.double() for t in x]
+    S = h0.double()
+    for t in range(T):
+        at, bt = (y[:, t * rank:(t + 1) * rank] for y in (a, b))
+        S = (gk[:, t].exp().unsqueeze(-1) * S + torch.einsum("brhk,brhv->bhkv", bt, torch.einsum("brhk,bhkv->brhv", at, S))
+             + torch.einsum("bhk,bhv->bhkv", k[:, t], v[:, t]))
+        # fp32: sums of up to 128 products, sqrt(128) 2^-24 < 1e-6 of the largest value, carried over two steps
+        assert orc.rel_err(o[:, t], torch.einsum("bhk,bhkv->bhv", q[:, t], S) * K ** -0.5) < 5e-6
+    assert orc.rel_err(ht, S) < 5e-6
+    # the first element's tokens as a packed batch between two empty sequences: the same kernel on the same numbers
+    h1 = torch.cat([h0[1:2], h0[:1], h0[2:3]])
+    o1, ht1 = Hm.fused_recurrent_dplr_delta_rule(*[t[:1] for t in x], rank, initial_state=h1, output_final_state=True,
+                                                 cu_seqlens=torch.tensor([0, 0, T, T], device=dev))
+    assert torch.equal(o1, o[:1]) and torch.equal(ht1, torch.cat([h0[1:2], ht[:1], h0[2:3]]))
+    # the state in place
+    from hdla_impl_b200.recurrent import fused_recurrent_dplr_delta_rule_fwd
+    hi = h0.clone()
+    oi, hti = fused_recurrent_dplr_delta_rule_fwd(*x, rank, K ** -0.5, hi, True, inplace_state=True)
+    assert hti.data_ptr() == hi.data_ptr() and torch.equal(hi, ht) and torch.equal(oi, o)
+
+
 def test_recurrent_inplace_state(dev):
     import hdla_impl_b200 as H
     x = make_inputs(4, 1, 2, 64, 64, R, seed=10, h0_std=0.5)
