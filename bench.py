@@ -634,7 +634,7 @@ def bench_decode_small(dev, steps=128):
     torch.cuda.empty_cache()
     return {"workload": "cfg2: B256 H32 K=V=128 decode, one token per step, fp32 state in place", "steps": steps,
             "us_per_step": sec * 1e6, "value": B / sec, "unit": "tokens/s",
-            "roofline": {"bound": "hbm", "kernel": "recurrent_bulk_kernel", "achieved": gbs, "peak": peaks["hbm_gbs"],
+            "roofline": {"bound": "hbm", "kernel": "recurrent_tile_kernel", "achieved": gbs, "peak": peaks["hbm_gbs"],
                          "unit": "GB/s", "frac": gbs / peaks["hbm_gbs"], "algorithmic_bytes_per_step": byts,
                          "peak_source": f"{how} (copy)", "l2": "state (537 MB) is larger than the 126 MB L2"}}
 
@@ -876,7 +876,7 @@ def run_decode(args, rank, world, local_rank):
             "e2e": {"value": B * world / (ms_e2e / steps / 1e3), "unit": "tokens/s", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h},
             "gpu_launches": int(launches),
-            "roofline": {"bound": "hbm", "kernel": "recurrent_bulk_kernel", "achieved": gbs, "peak": peaks["hbm_gbs"],
+            "roofline": {"bound": "hbm", "kernel": "recurrent_tile_kernel", "achieved": gbs, "peak": peaks["hbm_gbs"],
                          "unit": "GB/s", "frac": gbs / peaks["hbm_gbs"], "traffic": None,
                          "peak_source": f"{how} (copy)", "algorithmic_bytes": byts},
             "cpu_baseline": None, "clocks": clocks,

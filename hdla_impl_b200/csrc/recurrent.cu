@@ -100,7 +100,7 @@ __device__ __forceinline__ void st_cols(const float* x, float* base, int nh, int
     }
 }
 
-// Register-state kernel: more than kTileTokens tokens per call.
+// Register-state kernel: more than a few tokens per call (kTileTokens).
 //   * A column of the state depends on the other columns through nothing, so the columns are spread over warps (and,
 //     while there are fewer warps than the chip runs, over CTAs): a warp owns 4 CPT columns, lane (r, c) of it the
 //     rows 4 r + 32 j + {0..3} of CPT adjacent columns, in registers, as packed row pairs.
@@ -115,9 +115,12 @@ __device__ __forceinline__ void st_cols(const float* x, float* base, int nh, int
 // global memory between two CTA barriers: 413 tokens in 16 sequences x 16 heads of 128 took 262 us, now 66; one
 // sequence of 128 tokens x 4 heads 540 us, now 85.
 constexpr int kRecBlock = 8;
-// Up to two tokens the bulk-copied tile is the faster form (256 x 32 heads: 176 / 267 us for 1 / 2 tokens against 328 /
-// 284), from three on the registers are (4 tokens: 366 against 456 us; 8 heads, 4 tokens: 7.4 against 15.5).
-constexpr int kTileTokens = 2;
+// Up to two tokens the tile in shared memory is the faster form (4096 heads of 128: 0.71 / 0.83 of the registers' time for 1 /
+// 2 tokens), from three on the registers are (0.98 for 3, 1.25 for 6; with 64 heads 1.6 and 2.2; with so few heads they
+// already are for two tokens, 1.33).  But the register kernel pads K to 32, 64, 128 or 256 rows: where a fifth or more of
+// them is padding and there are two heads or more to an SM, the tile is faster up to eight tokens -- 0.66 of the time over
+// 352 measured cases (K x V of 16 x 64 to 100 x 132, ranks 1 to 4, 1024 and 4096 heads, 3 to 8 tokens), up to 1.1 in four.
+constexpr int kTileTokens = 2, kTileTokensPadded = 8;
 
 template <int KR, int CPT, int R>
 __global__ void __launch_bounds__(128, KR * CPT <= 32 ? 4 : KR * CPT <= 64 ? 3 : 2) recurrent_reg_kernel(RecParams p, int col_blocks, int async_ok) {
@@ -344,7 +347,7 @@ __device__ __forceinline__ uint32_t ld_raw(const void* p, size_t i, int dt) {
 __device__ __forceinline__ float raw_float(uint32_t x, int dt) { return __uint_as_float(dt == HDLA_F32 ? x : x << 16); }
 
 // ------------------------------------------------------------------------------------------
-// Decode variant (one or two tokens per call): the state tile is staged in shared memory.
+// Decode variant (a few tokens per call): the state tile is staged in shared memory.
 //   * one CTA per (sequence, head) brings the whole contiguous fp32 [K,V] tile (64 KB at K=V=128) into shared memory by
 //     16-byte asynchronous copies, so the bytes in flight per SM are set by how many tiles fit in shared memory (three),
 //     not by the register file;
@@ -564,7 +567,9 @@ int recurrent_fwd_launch(const HdlaDims& d, const void* q, const void* k, const 
     const int threads = 32 * ((d.V + 31) / 32);
     // few tokens per call: the kernel with the tile in shared memory (which it must fit)
     const size_t tile = (size_t)d.K * d.V * 4;
-    if (d.T <= kTileTokens && tile <= 65536 && tile % 16 == 0 && d.R <= 4) {
+    const int rows = d.K <= 32 ? 32 : d.K <= 64 ? 64 : d.K <= 128 ? 128 : 256;        // of the register kernel
+    const bool padded = 5 * d.K <= 4 * rows && tile > 2048 && blocks >= 2 * sm_count();
+    if (d.T <= (padded ? kTileTokensPadded : kTileTokens) && tile <= 65536 && tile % 16 == 0 && d.R <= 4) {
         const size_t smem_t = tile + sizeof(float) * ((3 + 2 * d.R) * (size_t)d.K + d.V);
         static thread_local int attr_dev = -1;
         int dev = 0;

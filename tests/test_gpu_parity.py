@@ -227,11 +227,11 @@ def test_recurrent_register_kernel_edges(dev, B, T, H, K, V, rank, cu, dtype, re
     assert orc.rel_err(o, ro) < (2e-5 if dtype == torch.float32 else 4e-3)
 
 
-@pytest.mark.parametrize("K,V,rank", [(8, 8, 1), (16, 16, 2), (33, 20, 2), (128, 128, 2)])
-@pytest.mark.parametrize("T", [1, 2])
+@pytest.mark.parametrize("K,V,rank,T", [(8, 8, 1, 1), (8, 8, 1, 2), (16, 16, 2, 1), (33, 20, 2, 2), (128, 128, 2, 1),
+                                        (128, 128, 2, 2), (16, 64, 2, 3), (33, 20, 4, 8), (100, 100, 3, 5), (100, 132, 2, 8)])
 def test_recurrent_many_heads(dev, K, V, rank, T):
-    """One and two tokens for more heads than the device runs at once, with tiles of a quarter to 64 KB (two dozen small ones
-    share an SM), and a packed batch with sequences of no token, whose state passes through."""
+    """A few tokens for more heads than the device runs at once, with tiles of a quarter to 64 KB (two dozen small ones share
+    an SM), and a packed batch with sequences of no token, whose state passes through."""
     import hdla_impl_b200 as Hm
     B, H = 1536, 4
     g = torch.Generator(device=dev).manual_seed(K)
@@ -247,14 +247,17 @@ def test_recurrent_many_heads(dev, K, V, rank, T):
         at, bt = (y[:, t * rank:(t + 1) * rank] for y in (a, b))
         S = (gk[:, t].exp().unsqueeze(-1) * S + torch.einsum("brhk,brhv->bhkv", bt, torch.einsum("brhk,bhkv->brhv", at, S))
              + torch.einsum("bhk,bhv->bhkv", k[:, t], v[:, t]))
-        # fp32: sums of up to 128 products, sqrt(128) 2^-24 < 1e-6 of the largest value, carried over two steps
+        # fp32: sums of up to 128 products, sqrt(128) 2^-24 < 1e-6 of the largest value, carried over up to eight steps
         assert orc.rel_err(o[:, t], torch.einsum("bhk,bhkv->bhv", q[:, t], S) * K ** -0.5) < 5e-6
     assert orc.rel_err(ht, S) < 5e-6
-    # the first element's tokens as a packed batch between two empty sequences: the same kernel on the same numbers
+    # the first element's tokens as a packed batch between two empty sequences (few heads: with more than two tokens the
+    # other kernel, whose sums are in another order)
     h1 = torch.cat([h0[1:2], h0[:1], h0[2:3]])
     o1, ht1 = Hm.fused_recurrent_dplr_delta_rule(*[t[:1] for t in x], rank, initial_state=h1, output_final_state=True,
                                                  cu_seqlens=torch.tensor([0, 0, T, T], device=dev))
-    assert torch.equal(o1, o[:1]) and torch.equal(ht1, torch.cat([h0[1:2], ht[:1], h0[2:3]]))
+    same = torch.equal if T <= 2 else lambda x, y: orc.rel_err(x, y) < 5e-6
+    assert same(o1, o[:1]) and same(ht1[1:2], ht[:1])
+    assert torch.equal(ht1[0], h0[1]) and torch.equal(ht1[2], h0[2])
     # the state in place
     from hdla_impl_b200.recurrent import fused_recurrent_dplr_delta_rule_fwd
     hi = h0.clone()
