@@ -63,14 +63,14 @@ def _tokens_of_merged(TR: int, rank_ab: int) -> int:
 def check_recurrent_status(dev, wait: bool = True) -> None:
     """Fetch the status word of the recurrent kernels for ``dev`` and, with ``wait``, raise if a time-limited wait ever ran
     out there (the present kernels have none)."""
+    if not wait:
+        return
     dev = torch.device(dev)
     host = torch.zeros(1, dtype=torch.int32).pin_memory()
     with torch.cuda.device(dev):
         _lib.check(_lib.load().hdla_recurrent_read_status(_lib.ptr(host), _lib.stream_ptr(dev)),
                    "hdla_recurrent_read_status")
-        if not wait:
-            return
-        torch.cuda.current_stream(dev).synchronize()
+        torch.cuda.current_stream(dev).synchronize()             # (before the word's memory goes)
     if int(host[0]):
         raise RuntimeError("libhdla: a device-side wait ran out in a recurrent kernel")
 
