@@ -39,8 +39,8 @@ constexpr int VS = 16;                       // state columns of a scan CTA
 __device__ int g_f32_status[4] = {0, 0, 0x7fc00000, 0};
 
 // Waits with a limit and records `code` if it runs out; the waits after one that ran out have a shorter limit, so that a
-// kernel whose copies never arrive ends.  (Out of line: with the flag carried through the kernels B2 T1000 H8 K=V=128 took
-// 652 us instead of 639.)
+// kernel whose copies never arrive ends.  (Out of line: inline, the scans' code gets worse, and B2 T1000 H8 K=V=128 forward
+// and backward takes 683 us instead of 630.)
 __device__ __noinline__ void wait_or_record(uint64_t* bar, uint32_t parity, int code) {
     const bool lost = *reinterpret_cast<volatile int*>(&g_f32_status[0]) != 0;
     if (!sm100::mbar_wait(bar, parity, lost ? 200000 : sm100::kWaitBudgetNs)) atomicExch(&g_f32_status[0], code);
@@ -355,8 +355,10 @@ struct ScanSmem {
     uint64_t bar[2];
 };
 
+// (three CTAs to an SM are what shared memory leaves room for with KP = 64; without the bound the compiler aims at four and
+// spills, which cost 91 instead of 85 us for B2 T256 H4 K=V=64 forward and backward)
 template <int KP, bool REV>
-__global__ void __launch_bounds__(128) f32_scan_kernel(ScanP p) {
+__global__ void __launch_bounds__(128, 3) f32_scan_kernel(ScanP p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     typedef ScanSmem<KP> Sm;
     Sm& s = *reinterpret_cast<Sm*>(smem_raw);
