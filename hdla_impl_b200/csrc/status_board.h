@@ -110,8 +110,9 @@ private:
                 free_.push_back(&all_.back());
             }
         }
-        Slot* s = free_.back();
-        free_.pop_back();
+        Slot* s = free_.front();                 // the one free for longest: a line of pinned memory that the host has just
+                                                 // read takes a copy later (B4 T2001 H16 K=V=64 fwd+bwd 734 -> 737 us)
+        free_.pop_front();
         return s;
     }
     void release(Slot* s) {
@@ -128,8 +129,7 @@ private:
     const Fail fail_;
     std::mutex mu_;
     std::deque<Slot> all_;                       // (a deque: slots keep their addresses)
-    std::vector<Slot*> free_;
-    std::deque<Slot*> posted_;
+    std::deque<Slot*> free_, posted_;
     double decay_ = NAN;
 };
 
