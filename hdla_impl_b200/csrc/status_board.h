@@ -110,9 +110,8 @@ private:
                 free_.push_back(&all_.back());
             }
         }
-        Slot* s = free_.front();                 // the one free for longest: a line of pinned memory that the host has just
-                                                 // read takes a copy later (B4 T2001 H16 K=V=64 fwd+bwd 734 -> 737 us)
-        free_.pop_front();
+        Slot* s = free_.back();
+        free_.pop_back();
         return s;
     }
     void release(Slot* s) {
@@ -129,7 +128,8 @@ private:
     const Fail fail_;
     std::mutex mu_;
     std::deque<Slot> all_;                       // (a deque: slots keep their addresses)
-    std::deque<Slot*> free_, posted_;
+    std::vector<Slot*> free_;
+    std::deque<Slot*> posted_;
     double decay_ = NAN;
 };
 
